@@ -32,42 +32,23 @@
 // backprojection, to ~1e-7 voxels (cone_bp_kernel).  When every view is
 // separable the same way (detector perpendicular to the main axis, u and v
 // along the two lateral axes: tomosynthesis) cone_bp_sep_kernel runs
-// instead, on projections pre-multiplied by seg (cone_prj_seg_kernel).
+// instead, on projections pre-multiplied by seg (cone_prj_seg_kernel).  Plans
+// of upright detectors (v along z, u in the x-y plane) run the kernels of
+// cone_col.cu, which trace each detector column's in-plane path once.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
+#include "cone_internal.h"
 #include "rn_internal.h"
 
 namespace rn {
-
-struct ConeView {
-    double S[3];              // source, voxel coordinates
-    double C[3];              // end point of ray (iu, iv) = (0, 0), voxel coordinates
-    double Eu[3], Ev[3];      // end-point step per detector index along u / v
-    float Sh[3], Sl[3];       // source as hi / lo floats
-    float au[4], av[4], ad[4];   // shadow: iu = (au . P + au[3]) / (ad . P + ad[3]), iv likewise
-    float ulo, uhi, vlo, vhi, dlo, dhi;   // sums of min(0, a_k) / max(0, a_k) over the three axes
-    // separable views (affine = 1 or 2): every ray advances by the same Dm0
-    // along m, and r_a = rho[0] + iu rho[1] + iv rho[2], r_b = rho[3] +
-    // iu rho[4] + iv rho[5] with rho[2] = rho[4] = 0 (affine = 1: a follows
-    // iu, b follows iv) or rho[1] = rho[5] = 0 (affine = 2)
-    double rho[6];
-    double Dm0;
-    int m, a, b, affine;
-};
-
-struct ConeDims {
-    int n[3];
-    float d[3];
-    long long st[3];          // image strides (elements) along x, y, z
-    int nc, nu, nv, nview, nb;
-    long long img_b, prj_b;   // batch strides
-};
 
 // Per ray (view, iv, iu) geometry for the backprojection:
 // {r_a hi, r_a lo, r_b hi, r_b lo}, {1 / r_a, 1 / r_b, seg, E_m}.
@@ -90,14 +71,6 @@ __global__ void cone_ray_kernel(float4* __restrict__ rays, const ConeView* __res
     rays[2 * i + 1] = make_float4(fabs(ra) > 1e-30 ? (float)(1.0 / ra) : 1e30f,
                                   fabs(rb) > 1e-30 ? (float)(1.0 / rb) : 1e30f, (float)seg,
                                   (float)(V.S[V.m] + Dm));
-}
-
-__device__ __forceinline__ long long to_fixed(double v) { return llrint(v * 4294967296.0); }
-
-// Fractional part of a fixed-point position as a float in [0, 1) (its top 23
-// bits: exact to 1.2e-7).
-__device__ __forceinline__ float fixed_frac(long long p) {
-    return __uint_as_float(0x3f800000u | ((unsigned)p >> 9)) - 1.0f;
 }
 
 // Per-ray stepping state: lateral positions at the start of slab k0 and
@@ -801,11 +774,36 @@ struct rn_cone_plan {
     bool bp_sep = false;       // every view separable the same way (cone_bp_sep_kernel)
     ConeView h_view0;          // host copy of view 0 (axes of a separable plan)
     bool unit = true;          // every ray's lateral slopes are at most 1
+    bool col = false;          // upright detectors: the kernels of cone_col.cu
+    ColView* d_col = nullptr;
+    // scratch of one call: taken from and given back to the plan's own pool in
+    // stream order, so calls on several streams or threads each have theirs;
+    // the pool keeps the memory for the next call until the plan goes
+    std::mutex pool_mu;
+    cudaMemPool_t pool = nullptr;
     float* d_prjw = nullptr;   // separable backprojection: projections times segment lengths (lazily allocated)
     long long launches = 0;
 };
 
 namespace {
+
+int scratch_get(rn_cone_plan* p, size_t bytes, cudaStream_t st, void** out) {
+    {
+        std::lock_guard<std::mutex> lk(p->pool_mu);
+        if (!p->pool) {
+            cudaMemPoolProps props;
+            memset(&props, 0, sizeof(props));
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = p->device;
+            RN_CUDA_TRY(cudaMemPoolCreate(&p->pool, &props));
+            uint64_t keep = UINT64_MAX;
+            RN_CUDA_TRY(cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        }
+    }
+    RN_CUDA_TRY(cudaMallocFromPoolAsync(out, bytes, p->pool, st));
+    return RN_OK;
+}
 
 int cone_views(rn_cone_plan* p, const RnConeGeom& g, const float* dc, const float* du_, const float* dv_,
                const float* src, std::vector<ConeView>& out, double& max_slope) {
@@ -982,15 +980,23 @@ int rn_cone_plan_create(rn_cone_plan** out, const RnConeGeom* g, const float* ho
     }
     cudaStream_t st = (cudaStream_t)stream;
     const long long nrays = (long long)g->nview * g->nv * g->nu;
+    std::vector<ColView> col;
+    p->col = cone_col_views(views, cd, col);
     cudaError_t e = cudaMalloc(&p->d_views, sizeof(ConeView) * views.size());
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_rays, sizeof(float4) * 2 * nrays);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(p->d_views, views.data(), sizeof(ConeView) * views.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) {
+    if (p->col) {
+        if (e == cudaSuccess) e = cudaMalloc(&p->d_col, sizeof(ColView) * col.size());
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(p->d_col, col.data(), sizeof(ColView) * col.size(), cudaMemcpyHostToDevice, st);
+    } else if (e == cudaSuccess) {
+        e = cudaMalloc(&p->d_rays, sizeof(float4) * 2 * nrays);
+    }
+    if (e == cudaSuccess && !p->col) {
         cone_ray_kernel<<<(unsigned)((nrays + 255) / 256), 256, 0, st>>>(p->d_rays, p->d_views, cd);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // `views` goes out of scope
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // `views` and `col` go out of scope
     if (e != cudaSuccess) {
         rn_cone_plan_destroy(p);
         return set_cuda_error(e, "rn_cone_plan_create");
@@ -1004,6 +1010,8 @@ int rn_cone_plan_destroy(rn_cone_plan* p) {
     cudaFree(p->d_views);
     cudaFree(p->d_rays);
     cudaFree(p->d_prjw);
+    cudaFree(p->d_col);
+    if (p->pool) cudaMemPoolDestroy(p->pool);
     delete p;
     return RN_OK;
 }
@@ -1014,6 +1022,10 @@ int rn_cone_project(rn_cone_plan* p, float* d_prj, const float* d_img, void* str
     const ConeDims& cd = p->cd;
     const long long nz = (long long)cd.nb * cd.nview * cd.nc;
     if (nz > 65535) return set_error(RN_ERR_ARG, "cone projection: more than 65535 views x batches x channels");
+    if (p->col) {
+        p->launches++;
+        return cone_col_project(p->d_col, cd, d_prj, d_img, (cudaStream_t)stream);
+    }
     const int gx = p->lanes_v ? (cd.nu + 7) / 8 : (cd.nu + 31) / 32;
     const int gy = p->lanes_v ? (cd.nv + 31) / 32 : (cd.nv + 7) / 8;
     dim3 grid(gx, gy, (unsigned)nz);
@@ -1037,6 +1049,15 @@ int rn_cone_backproject(rn_cone_plan* p, float* d_img, const float* d_prj, int a
     const long long nvox = (long long)cd.n[0] * cd.n[1] * cd.n[2];
     const int slices = cd.nb * cd.nc;
     if (slices > 65535) return set_error(RN_ERR_ARG, "cone backprojection: too many batches x channels");
+    if (p->col) {
+        cudaStream_t st = (cudaStream_t)stream;
+        void* tab = nullptr;
+        RN_TRY(scratch_get(p, cone_col_table_bytes(cd), st, &tab));
+        p->launches += 2LL * slices;
+        const int s = cone_col_backproject(p->d_col, cd, static_cast<double*>(tab), d_img, d_prj, accumulate, st);
+        cudaFreeAsync(tab, st);
+        return s;
+    }
     if (p->bp_sep) {
         // one warp per 2 (U) x 32 (V) voxels at one m
         const ConeView& v0 = p->h_view0;
