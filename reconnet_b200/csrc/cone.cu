@@ -34,7 +34,8 @@
 // along the two lateral axes: tomosynthesis) cone_bp_sep_kernel runs
 // instead, on projections pre-multiplied by seg (cone_prj_seg_kernel).  Plans
 // of upright detectors (v along z, u in the x-y plane) run the kernels of
-// cone_col.cu, which trace each detector column's in-plane path once.
+// cone_col.cu, which trace each detector column's in-plane path once;
+// tomosynthesis plans (u along x, v along y, main axis z) those of cone_tile.cu.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -43,6 +44,7 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
+#include <string>
 #include <vector>
 
 #include "cone_internal.h"
@@ -776,6 +778,9 @@ struct rn_cone_plan {
     bool unit = true;          // every ray's lateral slopes are at most 1
     bool col = false;          // upright detectors: the kernels of cone_col.cu
     ColView* d_col = nullptr;
+    bool tile = false;         // tomosynthesis: the kernels of cone_tile.cu
+    TilePlan tp;
+    TileView* d_tile = nullptr;
     // scratch of one call: taken from and given back to the plan's own pool in
     // stream order, so calls on several streams or threads each have theirs;
     // the pool keeps the memory for the next call until the plan goes
@@ -981,7 +986,14 @@ int rn_cone_plan_create(rn_cone_plan** out, const RnConeGeom* g, const float* ho
     cudaStream_t st = (cudaStream_t)stream;
     const long long nrays = (long long)g->nview * g->nv * g->nu;
     std::vector<ColView> col;
+    std::vector<TileView> tiles;
     p->col = cone_col_views(views, cd, col);
+    p->tile = !p->col && cone_tile_views(views, cd, tiles, p->tp);
+    if (p->tile && cone_tile_attributes() != RN_OK) {
+        const std::string msg = rn_last_error();
+        delete p;
+        return set_error(RN_ERR_CUDA, msg);
+    }
     cudaError_t e = cudaMalloc(&p->d_views, sizeof(ConeView) * views.size());
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(p->d_views, views.data(), sizeof(ConeView) * views.size(), cudaMemcpyHostToDevice, st);
@@ -989,14 +1001,18 @@ int rn_cone_plan_create(rn_cone_plan** out, const RnConeGeom* g, const float* ho
         if (e == cudaSuccess) e = cudaMalloc(&p->d_col, sizeof(ColView) * col.size());
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(p->d_col, col.data(), sizeof(ColView) * col.size(), cudaMemcpyHostToDevice, st);
+    } else if (p->tile) {
+        if (e == cudaSuccess) e = cudaMalloc(&p->d_tile, sizeof(TileView) * tiles.size());
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(p->d_tile, tiles.data(), sizeof(TileView) * tiles.size(), cudaMemcpyHostToDevice, st);
     } else if (e == cudaSuccess) {
         e = cudaMalloc(&p->d_rays, sizeof(float4) * 2 * nrays);
     }
-    if (e == cudaSuccess && !p->col) {
+    if (e == cudaSuccess && p->d_rays) {
         cone_ray_kernel<<<(unsigned)((nrays + 255) / 256), 256, 0, st>>>(p->d_rays, p->d_views, cd);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // `views` and `col` go out of scope
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // the host copies go out of scope
     if (e != cudaSuccess) {
         rn_cone_plan_destroy(p);
         return set_cuda_error(e, "rn_cone_plan_create");
@@ -1011,6 +1027,7 @@ int rn_cone_plan_destroy(rn_cone_plan* p) {
     cudaFree(p->d_rays);
     cudaFree(p->d_prjw);
     cudaFree(p->d_col);
+    cudaFree(p->d_tile);
     if (p->pool) cudaMemPoolDestroy(p->pool);
     delete p;
     return RN_OK;
@@ -1025,6 +1042,15 @@ int rn_cone_project(rn_cone_plan* p, float* d_prj, const float* d_img, void* str
     if (p->col) {
         p->launches++;
         return cone_col_project(p->d_col, cd, d_prj, d_img, (cudaStream_t)stream);
+    }
+    if (p->tile) {
+        cudaStream_t st = (cudaStream_t)stream;
+        void* vol = nullptr;
+        RN_TRY(scratch_get(p, cone_tile_fp_bytes(cd), st, &vol));
+        p->launches += 2LL * cd.nb * cd.nc;
+        const int s = cone_tile_project(p->d_tile, cd, p->tp, static_cast<float*>(vol), d_prj, d_img, st);
+        cudaFreeAsync(vol, st);
+        return s;
     }
     const int gx = p->lanes_v ? (cd.nu + 7) / 8 : (cd.nu + 31) / 32;
     const int gy = p->lanes_v ? (cd.nv + 31) / 32 : (cd.nv + 7) / 8;
@@ -1056,6 +1082,15 @@ int rn_cone_backproject(rn_cone_plan* p, float* d_img, const float* d_prj, int a
         p->launches += 2LL * slices;
         const int s = cone_col_backproject(p->d_col, cd, static_cast<double*>(tab), d_img, d_prj, accumulate, st);
         cudaFreeAsync(tab, st);
+        return s;
+    }
+    if (p->tile) {
+        cudaStream_t st = (cudaStream_t)stream;
+        void* wp = nullptr;
+        RN_TRY(scratch_get(p, cone_tile_bp_bytes(cd), st, &wp));
+        p->launches += 2LL * slices;
+        const int s = cone_tile_backproject(p->d_tile, cd, p->tp, static_cast<float*>(wp), d_img, d_prj, accumulate, st);
+        cudaFreeAsync(wp, st);
         return s;
     }
     if (p->bp_sep) {

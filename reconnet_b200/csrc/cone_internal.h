@@ -60,4 +60,27 @@ size_t cone_col_table_bytes(const ConeDims& cd);
 int cone_col_backproject(const ColView* d_views, const ConeDims& cd, double* d_tab, float* d_img, const float* d_prj,
                          int accumulate, cudaStream_t st);
 
+// ---------------------------------------------------------------------------
+// Tomosynthesis (cone_tile.cu): z the main axis, u along x, v along y.
+// ---------------------------------------------------------------------------
+struct TileView {
+    double su, sv, sm;             // source, voxels (x, y, z)
+    double ru0, ru1, rv0, rv1;     // slopes ru0 + iu ru1 along x and rv0 + iv rv1 along y, per slab
+    float gu_max, gv_max;          // widest ray spacing inside the grid, voxels
+};
+struct TilePlan {
+    bool fp_narrow = false;        // rays under a voxel apart
+    int kv = 0;                    // rows of rays that can meet one voxel
+    int bp_patch = 0, bp_smem = 0; // floats of a backprojection patch, shared memory of a block
+};
+// Fills `out` and `tp` where the tile kernels can take the plan (false otherwise).
+bool cone_tile_views(const std::vector<ConeView>& views, const ConeDims& cd, std::vector<TileView>& out, TilePlan& tp);
+int cone_tile_attributes();
+size_t cone_tile_fp_bytes(const ConeDims& cd);
+size_t cone_tile_bp_bytes(const ConeDims& cd);
+int cone_tile_project(const TileView* d_views, const ConeDims& cd, const TilePlan& tp, float* d_vol, float* d_prj,
+                      const float* d_img, cudaStream_t st);
+int cone_tile_backproject(const TileView* d_views, const ConeDims& cd, const TilePlan& tp, float* d_wp, float* d_img,
+                          const float* d_prj, int accumulate, cudaStream_t st);
+
 }  // namespace rn

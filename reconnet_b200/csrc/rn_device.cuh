@@ -97,6 +97,12 @@ __device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
     return r;
 }
 
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // floor(x) and frac(x) for 0 <= x < 2^22 on the FMA/ALU pipes: the integer
 // part comes from rounding (x - 0.5) with a 1.5 * 2^23 bias.  At exact
 // integers it may return (n-1, 1.0) instead of (n, 0.0); both evaluate the
