@@ -32,6 +32,7 @@
 #include <string>
 #include <vector>
 
+#include "fan_bp.cuh"
 #include "rn_device.cuh"
 #include "rn_internal.h"
 
@@ -54,6 +55,7 @@ constexpr int kSmemBudget = 227 * 1024;
 
 
 constexpr int kBpViews = 8;          // views per staged chunk
+using BpShared = BpSharedT<kBpViews>;
 
 __host__ __device__ inline long long align4(long long v) { return (v + 3) & ~3ll; }
 
@@ -639,7 +641,6 @@ __global__ void bp_parts_sum_kernel(float* __restrict__ out, const float* __rest
 }
 
 
-// Per-view parameters the BP inner loop reads, staged in shared memory.
 // Siddon BP table: per view, entry e holds the slope of ray e - 1 as hi / lo
 // floats and the prefix C_e = sum_{u < e} c_u as hi / lo floats (FP64 scan),
 // c_u = w_u * (ray length per band), w_u the sinogram value mixed over the
@@ -740,51 +741,11 @@ __global__ void pd_table_kernel(const float* __restrict__ prj, const BpSlice* __
     }
 }
 
-struct BpView {
-    double pard, perpd;   // source coordinates (Siddon band positions)
-    float par, perp, kappa, tA, tB, sigma;
-    int xcls;
-};
-
-struct BpShared {
-    ViewGeo rec[2][kBpViews];   // view records staged for the next chunk
-    uint64_t bars[2];
-    int elo[3][kBpViews];       // first staged table entry per view
-    BpView vw[3][kBpViews];
-};
-
-// Edge index t of the matched parametrisation for a slope r
-// (r = (q - par) / (l - perp) at lattice point (line l, position q)).
-__device__ __forceinline__ float matched_t(const ViewGeo& vg, float r) {
-    return vg.tA + vg.tB * atanf(vg.kappa * r);
-}
-
 // Matched backprojection: lane i of a warp owns pixel column x = X0 + i and
 // kBmRows pixel rows from y0; lane 31 owns no pixel and only supplies the
 // right edge of lane 30's column.  The staged table window T starts at table
 // index ilo; entries carry the prefix (hi, lo), the slope scaled by sigma / 2
 // and the edge slope r_e.
-//
-// Edge index t(r) = tA + tB atan(kappa r) as a cubic around the slope r_t at
-// the lane's middle lattice point: along one lane the lattice points differ
-// in one coordinate only, and the truncation stays below 4e-5 cells over 17
-// points (it only selects the cell; the value inside it is exact).
-struct TCubic {
-    float rt, c0, c1, c2, c3;
-};
-__device__ __forceinline__ TCubic t_cubic(const BpView& vg, float rt) {
-    const float ut = vg.kappa * rt;
-    const float iw = __fdividef(1.0f, fmaf(ut, ut, 1.0f));
-    const float k1 = vg.tB * vg.kappa * iw;
-    TCubic c;
-    c.rt = rt;
-    c.c0 = fmaf(vg.tB, atanf(ut), vg.tA);
-    c.c1 = k1;
-    c.c2 = -k1 * vg.kappa * ut * iw;
-    c.c3 = k1 * vg.kappa * vg.kappa * (fmaf(3.0f * ut, ut, -1.0f) * (1.0f / 3.0f)) * iw * iw;
-    return c;
-}
-
 // H at slope r: prefix (hi) and the rest (lo + slope * (r - r_e)) of the
 // table entry of the cell that contains r.
 __device__ __forceinline__ void bp_h(const TCubic& c, float r, const float4* T, int ilo, int imax, float& hi,
@@ -878,11 +839,6 @@ __device__ __forceinline__ float siddon_below(const float4 E, float Ah, float Al
     return ar > 1e-6f ? fr : (xa < 0.f ? 1.f : 0.f);
 }
 
-// floor(x) for |x| < 2^22 on the FMA / ALU pipes (round-down add of 1.5 * 2^23).
-__device__ __forceinline__ int floor_small(float x) {
-    return __float_as_int(__fadd_rd(x, 12582912.0f)) - 0x4B400000;
-}
-
 // F(q) = sum_u c_u b_u(q) (up to the total, for sigma < 0) as hi + rest, for
 // the band between the lattice points with edge indices ta and tb.  Table
 // indices clamp into the staged window [ilo, imax].  Kept out of line: the
@@ -921,18 +877,6 @@ __device__ __noinline__ void siddon_F(const float4* T, int ilo, int imax, int nu
         fhi = -ch;
         frest = part - cl;
     }
-}
-
-__device__ __forceinline__ void split_hilo(double v, float& h, float& l) {
-    h = (float)v;
-    l = (float)(v - (double)h);
-}
-
-// s + e = a + b exactly (TwoSum).
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-    s = a + b;
-    const float bb = s - a;
-    e = (a - (s - bb)) + (b - bb);
 }
 
 __device__ __forceinline__ void bp_siddon_x(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
@@ -1130,42 +1074,6 @@ __device__ __forceinline__ void bp_pixel_y(float (&acc)[kBmRows], const BpView& 
     }
 }
 
-// Warp 0 of a backprojection CTA prepares chunk c (views c*kBpViews ...) of
-// its tile at (X0, Y0): lane = view * 4 + tile corner evaluates the edge index
-// at its corner, a 4-lane min gives the first staged table entry, and the
-// view's parameters go to slot c % 3.  Kept out of line: it runs once per
-// chunk in one warp, and inlined its temporaries would raise the register
-// count of the whole accumulation loop.
-template <int kMode>
-__device__ __noinline__ void bp_prep(BpShared* sh, const ViewGeo* src, int c, int nview, int X0, int Y0,
-                                     int tabn, int win, const FanDims d) {
-    const int lane = threadIdx.x & 31, v = lane >> 2, corner = lane & 3;
-    const bool valid = c * kBpViews + v < nview;
-    const ViewGeo& vg = src[valid ? v : 0];
-    const int cx = corner & 1, cy = corner >> 1;
-    const int xcls = vg.xcls;
-    const float X = (float)(X0 + cx * kBmCols), Y = (float)(Y0 + cy * kBmTileY);
-    const float l = xcls ? Y : X, q = xcls ? X : Y;
-    float t = matched_t(vg, (q - (float)vg.par) / (l - (float)vg.perp));
-    t = fminf(t, __shfl_xor_sync(0xffffffffu, t, 1));
-    t = fminf(t, __shfl_xor_sync(0xffffffffu, t, 2));
-    if (valid && corner == 0) {
-        const int slot = c % 3;
-        const int lo = (int)floorf(t) + 1 - 2;   // table index = edge/cell index + 1
-        sh->elo[slot][v] = max(0, min(lo, tabn - win));
-        BpView& w = sh->vw[slot][v];
-        w.pard = vg.par;
-        w.perpd = vg.perp;
-        w.par = (float)vg.par;
-        w.perp = (float)vg.perp;
-        w.kappa = vg.kappa;
-        w.tA = vg.tA;
-        w.tB = vg.tB;
-        w.sigma = vg.sigma;
-        w.xcls = vg.xcls;
-    }
-}
-
 // kMode: 0 reference-mode (typeProjector 0 / 1), 1 matched, 2 Siddon, 3 pixel-driven.
 // Siddon tiles run three CTAs per SM (80 registers, 180 vs 174 Gupd/s at two
 // CTAs); the DD modes keep the compiler's register choice (71 / 80).
@@ -1214,7 +1122,8 @@ __global__ void __launch_bounds__(kBpThreads, (kMode == 2 || kMode == 0) ? 3 : 0
 
     const int nchunks = (gs.nview + kBpViews - 1) / kBpViews;
     auto prep = [&](int c, const ViewGeo* src) {
-        bp_prep<kMode>(sh, src, c, gs.nview, X0, Y0, tabn, p.win, p.d);
+        // table index = edge / cell index + 1
+        bp_prep<kBpViews, kBmCols, kBmTileY>(sh, src, c, gs.nview, X0, Y0, tabn, p.win, 1, 2);
     };
     // tid 0: stage chunk c's table windows into buffer c & 1 and the view
     // records of chunk c + 1 into record slot (c + 1) & 1, on barrier c & 1.
@@ -1354,6 +1263,7 @@ int fan_kernel_attributes() {
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
+    RN_TRY(fan_group_attributes());
     g_attr_done[dev] = 1;
     return RN_OK;
 }
@@ -1614,6 +1524,22 @@ int fan_backproject(rn_fan_plan* p, float* d_img, const float* d_prj, int type, 
         const int s1 = bp_wave_end(p, bps, s0);
         const long long base = bps[s0].table_off;
         const int ns = s1 - s0;
+        auto sum_parts = [&](int nparts) -> int {
+            if (nparts <= 1) return RN_OK;
+            LaunchScope ls4(p, st, 4);
+            const long long n = p->img_elems;
+            bp_parts_sum_kernel<<<(unsigned)std::min<long long>((n + 255) / 256, 148LL * 8), 256, 0, st>>>(
+                d_img, p->d_bp_parts, nparts, p->img_elems, n, accumulate);
+            RN_CUDA_TRY(cudaGetLastError());
+            return RN_OK;
+        };
+        if (fan_group_ok(p, type, ns)) {   // slices that share their views (fan_group.cu)
+            int nparts = 1;
+            RN_TRY(fan_group_backproject(p, d_img, d_prj, type, accumulate, s0, ns, &nparts, st));
+            RN_TRY(sum_parts(nparts));
+            s0 = s1;
+            continue;
+        }
         const int maxv = bp_max_views(p, bps, s0, s1);
         dim3 tg((maxv + 7) / 8, ns);
         {
@@ -1662,13 +1588,7 @@ int fan_backproject(rn_fan_plan* p, float* d_img, const float* d_prj, int type, 
         else if (type == RN_TYPE_MATCHED) fan_bp_kernel<1><<<grid, kBpThreads, smem, st>>>(bp);
         else fan_bp_kernel<0><<<grid, kBpThreads, smem, st>>>(bp);
         RN_CUDA_TRY(cudaGetLastError());
-        if (bp.nparts > 1) {
-            LaunchScope ls4(p, st, 4);
-            const long long n = p->img_elems;
-            bp_parts_sum_kernel<<<(unsigned)std::min<long long>((n + 255) / 256, 148LL * 8), 256, 0, st>>>(
-                d_img, bp.parts, bp.nparts, bp.part_stride, n, accumulate);
-            RN_CUDA_TRY(cudaGetLastError());
-        }
+        RN_TRY(sum_parts(bp.nparts));
         s0 = s1;
     }
     return RN_OK;

@@ -231,6 +231,13 @@ int fan_slope_tables(rn_fan_plan* p, const double2* d_vcs, const int* d_vx, cons
 // Parts over which fan_backproject splits a backprojection of `type` (1 when
 // it does not split), and the number of slices in its first launch.
 int fan_bp_split(const rn_fan_plan* p, int type, int* first_wave_slices);
+// Backprojection of slices that share their views (fan_group.cu): whether it
+// takes a launch of `ns` slices, its kernels' attributes, and the launch of
+// slices s0 .. s0 + ns - 1 (`nparts` partial images to sum where above 1).
+bool fan_group_ok(const rn_fan_plan* p, int type, int ns);
+int fan_group_attributes();
+int fan_group_backproject(rn_fan_plan* p, float* d_img, const float* d_prj, int type, int accumulate, int s0, int ns,
+                          int* nparts, cudaStream_t st);
 // Most lines per staged forward-projection chunk that shared memory holds.
 int fan_fp_lines_max(const rn_fan_plan* p);
 int fan_project(rn_fan_plan* p, float* d_prj, const float* d_img, cudaStream_t st, bool siddon = false);
