@@ -777,6 +777,7 @@ struct rn_cone_plan {
     ConeView h_view0;          // host copy of view 0 (axes of a separable plan)
     bool unit = true;          // every ray's lateral slopes are at most 1
     bool col = false;          // upright detectors: the kernels of cone_col.cu
+    bool col_one = false;      // (their single-crossing form)
     ColView* d_col = nullptr;
     bool tile = false;         // tomosynthesis: the kernels of cone_tile.cu
     TilePlan tp;
@@ -987,7 +988,7 @@ int rn_cone_plan_create(rn_cone_plan** out, const RnConeGeom* g, const float* ho
     const long long nrays = (long long)g->nview * g->nv * g->nu;
     std::vector<ColView> col;
     std::vector<TileView> tiles;
-    p->col = cone_col_views(views, cd, col);
+    p->col = cone_col_views(views, cd, col, p->col_one);
     p->tile = !p->col && cone_tile_views(views, cd, tiles, p->tp);
     if (p->tile && cone_tile_attributes() != RN_OK) {
         const std::string msg = rn_last_error();
@@ -1080,7 +1081,8 @@ int rn_cone_backproject(rn_cone_plan* p, float* d_img, const float* d_prj, int a
         void* tab = nullptr;
         RN_TRY(scratch_get(p, cone_col_table_bytes(cd), st, &tab));
         p->launches += 2LL * slices;
-        const int s = cone_col_backproject(p->d_col, cd, static_cast<double*>(tab), d_img, d_prj, accumulate, st);
+        const int s = cone_col_backproject(p->d_col, cd, p->col_one, static_cast<double*>(tab), d_img, d_prj,
+                                           accumulate, st);
         cudaFreeAsync(tab, st);
         return s;
     }

@@ -28,9 +28,9 @@
 // multiply-add per face and interval end, good to 2.4e-7 rays.  The intervals
 // of 32 views are worked out at a time, one view per lane.
 //
-// Measured, 256x256x128 voxels, 90 views of 512x128 cells: forward 2.24 ms
+// Measured, 256x256x128 voxels, 90 views of 512x128 cells: forward 1.77 ms
 // (3.84 ms with one thread per ray stepping through global memory,
-// cone_fp_kernel), back 3.45 ms with its table (19.8 ms with the shadow gather
+// cone_fp_kernel), back 3.52 ms with its table (19.8 ms with the shadow gather
 // of cone_bp_kernel).  Both are bound by instruction issue and L1 reads.
 #include <cuda_runtime.h>
 
@@ -58,6 +58,37 @@ __device__ __forceinline__ ColRay col_ray(const ColView& V, int iu) {
     r.Da = r.m ? d0 : d1;
     r.ra = r.Da / r.Dm;
     return r;
+}
+
+// `cnt` slabs of a warp's rays; kIn: no bounds checks on the heights.
+template <int R, bool kIn>
+__device__ __forceinline__ void col_slabs(float (&acc)[R], long long (&B)[R], const long long (&RB)[R],
+                                          const float (&sb)[R], const float (&ob)[R], const float4* slabs, int cnt,
+                                          const float* __restrict__ vol, int nc, int nz) {
+    auto voxel = [&](int o, int b) {
+        return kIn || (unsigned)b < (unsigned)nz ? __ldg(vol + (o + b * nc)) : 0.f;
+    };
+    for (int j = 0; j < cnt; j++) {
+        const float4 e = slabs[j];
+        const int o0 = __float_as_int(e.x), o1 = __float_as_int(e.y);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int b0 = (int)(B[r] >> 32);
+            const float tb = fminf(fmaf(sb[r], __uint_as_float(0x3f800000u | ((unsigned)B[r] >> 9)), ob[r]), 1.f);
+            B[r] += RB[r];
+            const int b1 = (int)(B[r] >> 32);
+            if (o1 == o0) {   // the same for the warp: one image column
+                if (o0 >= 0) acc[r] = fmaf(tb, voxel(o0, b0), fmaf(1.f - tb, voxel(o0, b1), acc[r]));
+            } else {
+                const float t0 = fminf(e.z, tb), t1 = fmaxf(e.z, tb);
+                const bool afirst = e.z < tb;
+                const int om = afirst ? o1 : o0, bm = afirst ? b0 : b1;
+                if (o0 >= 0) acc[r] = fmaf(t0, voxel(o0, b0), acc[r]);
+                if (om >= 0) acc[r] = fmaf(t1 - t0, voxel(om, bm), acc[r]);
+                if (o1 >= 0) acc[r] = fmaf(1.f - t1, voxel(o1, b1), acc[r]);
+            }
+        }
+    }
 }
 
 template <int R>
@@ -102,6 +133,14 @@ __global__ void __launch_bounds__(32 * kColWarps) cone_fp_col_kernel(float* __re
         seg[r] = (float)sqrt(dm * dm + ra * ra * da * da + rz * rz * dz * dz);
         acc[r] = 0.f;
     }
+    // the time of the height crossing in a slab as one FMA on 1 + the position's
+    // fraction; at or above 1 where there is none
+    float sb[R], ob[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        sb[r] = RB[r] > 0 ? -irb[r] : irb[r];
+        ob[r] = RB[r] > 0 ? 2.f * irb[r] : -irb[r];
+    }
     const float* vol = img + bt * cd.img_b + c;
     const int nc = cd.nc;
     for (int kb = ks; kb < ke; kb += 32) {
@@ -118,35 +157,17 @@ __global__ void __launch_bounds__(32 * kColWarps) cone_fp_col_kernel(float* __re
             s_slab[warp][lane] = make_float4(__int_as_float(o0), __int_as_float(o1), ta, 0.f);
         }
         __syncwarp();
-        for (int j = 0; j < cnt; j++) {
-            const float4 e = s_slab[warp][j];
-            const int o0 = __float_as_int(e.x), o1 = __float_as_int(e.y);
+        // rays that stay inside the volume's height over these slabs need no bounds checks
+        bool inside = true;
 #pragma unroll
-            for (int r = 0; r < R; r++) {
-                const int b0 = (int)(B[r] >> 32);
-                const float fb = fixed_frac(B[r]);
-                B[r] += RB[r];
-                const int b1 = (int)(B[r] >> 32);
-                // |rise| <= 1: at most one height crossing, at tb (1 where there is none)
-                const float tb = b1 != b0 ? fminf((RB[r] > 0 ? 1.f - fb : fb) * irb[r], 1.f) : 1.f;
-                const bool in0 = (unsigned)b0 < (unsigned)nz, in1 = (unsigned)b1 < (unsigned)nz;
-                if (o1 == o0) {   // the same for the warp: one image column
-                    if (o0 >= 0) {
-                        const float x0 = in0 ? __ldg(vol + (o0 + b0 * nc)) : 0.f;
-                        const float x1 = in1 ? __ldg(vol + (o0 + b1 * nc)) : 0.f;
-                        acc[r] = fmaf(tb, x0, fmaf(1.f - tb, x1, acc[r]));
-                    }
-                } else {
-                    const float t0 = fminf(e.z, tb), t1 = fmaxf(e.z, tb);
-                    const bool afirst = e.z < tb;
-                    const int om = afirst ? o1 : o0, bm = afirst ? b0 : b1;
-                    const float x0 = in0 && o0 >= 0 ? __ldg(vol + (o0 + b0 * nc)) : 0.f;
-                    const float xm = (afirst ? in0 : in1) && om >= 0 ? __ldg(vol + (om + bm * nc)) : 0.f;
-                    const float x1 = in1 && o1 >= 0 ? __ldg(vol + (o1 + b1 * nc)) : 0.f;
-                    acc[r] = fmaf(t0, x0, fmaf(t1 - t0, xm, fmaf(1.f - t1, x1, acc[r])));
-                }
-            }
+        for (int r = 0; r < R; r++) {
+            const int b0 = (int)(B[r] >> 32), b1 = (int)((B[r] + cnt * RB[r]) >> 32);
+            inside = inside && (unsigned)b0 < (unsigned)nz && (unsigned)b1 < (unsigned)nz;
         }
+        if (__all_sync(0xffffffffu, inside))
+            col_slabs<R, true>(acc, B, RB, sb, ob, s_slab[warp], cnt, vol, nc, nz);
+        else
+            col_slabs<R, false>(acc, B, RB, sb, ob, s_slab[warp], cnt, vol, nc, nz);
     }
 #pragma unroll
     for (int r = 0; r < R; r++) {
@@ -194,37 +215,49 @@ constexpr int kColFrac = 28;   // fractional bits of kappa
 
 // One in-plane interval of a pixel: kappa at its two ends as a function of the
 // face, kappa' = b + (q - z0) g in fixed point, raised by 2^28 - 1 so that its
-// integer part counts the rays below the face.
+// integer part counts the rays below the face; kappa + c at the first end and
+// the difference of the two kappas as floats, a + (q - z0) ga and e + (q - z0) ge.
 struct ColTask {
     longlong2 b;
-    int4 g;        // g at the two ends, table row, c as a float
+    int4 g;        // g at the two ends, table row
+    float4 f;      // a, ga, e, ge
     double t;      // length of the interval
 };
 
-// F(q) / t for the face dq above z0.
-__device__ __forceinline__ double col_below(const longlong2 b, const int4 g, int dq, const double* __restrict__ tab,
-                                            int nv) {
+// What face dq above z0 has below it: t C(k) into `sum` and t x the share of
+// the rays that cross the face over the pixel into `part`.  kOne: at most one
+// ray does (the heights that count move by less than one ray over a pixel).
+template <bool kOne>
+__device__ __forceinline__ void col_below(double& sum, float& part, const longlong2 b, const int4 g, const float4 f,
+                                          double t, float tf, int dq, const double* __restrict__ tab, int nv) {
     const long long k0 = b.x + (long long)dq * g.x, k1 = b.y + (long long)dq * g.y;
-    const int n0 = min(max((int)(k0 >> kColFrac), 0), nv), n1 = min(max((int)(k1 >> kColFrac), 0), nv);
+    const int n0 = (int)(k0 >> kColFrac), n1 = (int)(k1 >> kColFrac);
+    const float fq = (float)dq;
+    // ray i crosses the face at the share s of the interval from its first
+    // end: 1 / (kappa + c) is linear in t.  d0 = kappa_0 - i, d01 = kappa_0 -
+    // kappa_1; kappa_0's fraction comes from its fixed point
+    const float a0 = fmaf(fq, f.y, f.x), d01 = fmaf(fq, f.w, f.z);
+    const float f1 = __uint_as_float(0x3f800000u | (((unsigned)k0 >> (kColFrac - 23)) & 0x7fffffu));   // 1 + fraction
+    auto share = [&](float d0) {
+        const float s = __saturatef(__fdividef(d0 * (a0 - d01), d01 * (a0 - d0)));
+        return n0 > n1 ? s : 1.f - s;   // kappa falls: below until it crosses
+    };
+    const int lo = min(n0, n1);
     const double* row = tab + (long long)g.z * (nv + 1);
-    const int lo = min(n0, n1), hi = max(n0, n1);
-    double v = __ldg(row + lo);
-    for (int i = lo; i < hi; i++) {
-        // ray i crosses the face at the share s of the interval from its
-        // first end: 1 / (kappa + c) is linear in t
-        const long long ki = ((long long)i << kColFrac) + ((1 << kColFrac) - 1);
-        constexpr float kUnit = 1.0f / (1 << kColFrac);
-        const float d0 = (float)(int)(k0 - ki), d01 = (float)(int)(k0 - k1);
-        const float c = __int_as_float(g.w), a1 = fmaf((float)(int)(k1 - ki), kUnit, (float)i) + c, ai = (float)i + c;
-        const float s = fminf(fmaxf(__fdividef(d0 * a1, d01 * ai), 0.f), 1.f);
-        const float below = n0 > n1 ? s : 1.f - s;   // kappa falls: below until it crosses
-        v = fma((double)below, __ldg(row + i + 1) - __ldg(row + i), v);
+    if (kOne) {
+        sum = fma(t, __ldg(row + min(max(lo, 0), nv)), sum);
+        if (n0 != n1 && (unsigned)lo < (unsigned)nv)
+            part = fmaf(tf * share(f1 - (n0 > n1 ? 1.f : 2.f)), (float)(__ldg(row + lo + 1) - __ldg(row + lo)), part);
+    } else {
+        const int l = min(max(lo, 0), nv), h = min(max(max(n0, n1), 0), nv);
+        sum = fma(t, __ldg(row + l), sum);
+        for (int i = l; i < h; i++)
+            part = fmaf(tf * share((f1 - 1.f) + (float)(n0 - 1 - i)), (float)(__ldg(row + i + 1) - __ldg(row + i)), part);
     }
-    return v;
 }
 
-template <int R>
-__global__ void __launch_bounds__(32 * kColWarps) cone_bp_col_kernel(float* __restrict__ img, const double* __restrict__ tab,
+template <int R, bool kOne>
+__global__ void __launch_bounds__(32 * kColWarps, 3) cone_bp_col_kernel(float* __restrict__ img, const double* __restrict__ tab,
                                                                       const ColView* __restrict__ views, ConeDims cd,
                                                                       int bt, int c, int accumulate) {
     __shared__ ColTask s_task[kColWarps][32];
@@ -235,8 +268,12 @@ __global__ void __launch_bounds__(32 * kColWarps) cone_bp_col_kernel(float* __re
     const int nz = cd.n[2], z0 = blockIdx.z * 32 * R;
     const int top = min(nz - z0, 32 * R);   // the chunk's upper face, evaluated by the lanes' own views
     double acc[R], acct = 0.0;
+    float part[R], partt = 0.f;
 #pragma unroll
-    for (int r = 0; r < R; r++) acc[r] = 0.0;
+    for (int r = 0; r < R; r++) {
+        acc[r] = 0.0;
+        part[r] = 0.f;
+    }
     ColTask* task = s_task[warp];
     for (int vb = 0; vb < cd.nview; vb += 32) {
         const int view = vb + lane;
@@ -260,7 +297,7 @@ __global__ void __launch_bounds__(32 * kColWarps) cone_bp_col_kernel(float* __re
             for (int k = 0; k < 4; k++) {
                 // iu of the in-plane ray through (M + k0, k1 - A) from the source
                 const double wm = M + (k & 1), wa = (k >> 1) - A;
-                const float q = (float)(Da0 * wm - Dm0 * wa) / (float)(Em * wa - Ea * wm);
+                const float q = __fdividef((float)(Da0 * wm - Dm0 * wa), (float)(Em * wa - Ea * wm));
                 lo = fminf(lo, q);
                 hi = fmaxf(hi, q);
             }
@@ -276,7 +313,7 @@ __global__ void __launch_bounds__(32 * kColWarps) cone_bp_col_kernel(float* __re
                 const double ra = Da / Dm, xa = fma(ra, M, A);   // lateral offset at the pixel's low face
                 double ta = 0.0, tb = 1.0;
                 if (fabs(ra) > 1e-12) {
-                    const double ir = Dm / Da, p = -xa * ir, q = (1.0 - xa) * ir;
+                    const double ir = 1.0 / ra, p = -xa * ir, q = (1.0 - xa) * ir;
                     ta = fmax(0.0, fmin(p, q));
                     tb = fmin(1.0, fmax(p, q));
                 } else if (!(xa >= 0.0 && xa < 1.0)) {
@@ -284,14 +321,14 @@ __global__ void __launch_bounds__(32 * kColWarps) cone_bp_col_kernel(float* __re
                 }
                 hit = tb - ta > 1e-12;
                 if (hit) {
-                    const double s = Dm * iez, g0 = s / (M + ta), g1 = s / (M + tb);
-                    constexpr double kOne = (double)(1 << kColFrac);
-                    T.b = make_longlong2(llrint(fma(zr, g0, -cc) * kOne) + ((1 << kColFrac) - 1),
-                                         llrint(fma(zr, g1, -cc) * kOne) + ((1 << kColFrac) - 1));
-                    T.g = make_int4((int)llrint(g0 * kOne), (int)llrint(g1 * kOne), view * cd.nu + iu,
-                                    __float_as_int((float)cc));
+                    const double s = Dm * iez, g0 = s / (M + ta), g1 = s / (M + tb), a = zr * g0, e = zr * (g0 - g1);
+                    constexpr double kOneFixed = (double)(1 << kColFrac);
+                    T.b = make_longlong2(llrint((a - cc) * kOneFixed) + ((1 << kColFrac) - 1),
+                                         llrint((a - e - cc) * kOneFixed) + ((1 << kColFrac) - 1));
+                    T.g = make_int4((int)llrint(g0 * kOneFixed), (int)llrint(g1 * kOneFixed), view * cd.nu + iu, 0);
+                    T.f = make_float4((float)a, (float)g0, (float)e, (float)(g0 - g1));
                     T.t = tb - ta;
-                    acct = fma(T.t, col_below(T.b, T.g, top, tab, cd.nv), acct);
+                    col_below<kOne>(acct, partt, T.b, T.g, T.f, T.t, (float)T.t, top, tab, cd.nv);
                 }
             }
             const unsigned hits = __ballot_sync(0xffffffffu, hit);
@@ -302,24 +339,34 @@ __global__ void __launch_bounds__(32 * kColWarps) cone_bp_col_kernel(float* __re
             for (int e = 0; e < n; e++) {
                 const longlong2 b = task[e].b;
                 const int4 g = task[e].g;
+                const float4 f = task[e].f;
                 const double t = task[e].t;
+                const float tf = (float)t;
 #pragma unroll
-                for (int r = 0; r < R; r++) acc[r] = fma(t, col_below(b, g, lane + 32 * r, tab, cd.nv), acc[r]);
+                for (int r = 0; r < R; r++)
+                    col_below<kOne>(acc[r], part[r], b, g, f, t, tf, lane + 32 * r, tab, cd.nv);
             }
         }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acct += __shfl_xor_sync(0xffffffffu, acct, o);
+    for (int o = 16; o > 0; o >>= 1) {
+        acct += __shfl_xor_sync(0xffffffffu, acct, o);
+        partt += __shfl_xor_sync(0xffffffffu, partt, o);
+    }
     float* out = img + bt * cd.img_b + (long long)x * cd.st[0] + (long long)y * cd.st[1] + c;
 #pragma unroll
     for (int r = 0; r < R; r++) {
-        const double up = __shfl_down_sync(0xffffffffu, acc[r], 1);
-        const double over = __shfl_sync(0xffffffffu, acc[r + 1 < R ? r + 1 : r], 0);   // face 32 (r + 1)
+        // the voxel's upper face: the next lane's, the next 32 faces' first, or the chunk's top
+        const int rn = r + 1 < R ? r + 1 : r;
+        const double up = __shfl_down_sync(0xffffffffu, acc[r], 1), over = __shfl_sync(0xffffffffu, acc[rn], 0);
+        const float upp = __shfl_down_sync(0xffffffffu, part[r], 1), overp = __shfl_sync(0xffffffffu, part[rn], 0);
         const int dz = lane + 32 * r;
         if (dz < top) {
-            const double hi = dz + 1 == top ? acct : lane == 31 ? over : up;
+            const bool last = dz + 1 == top;
+            const double hi = last ? acct : lane == 31 ? over : up;
+            const float hip = last ? partt : lane == 31 ? overp : upp;
             float* o = out + (long long)(z0 + dz) * cd.nc;
-            const float v = (float)(hi - acc[r]);
+            const float v = (float)(hi - acc[r]) + (hip - part[r]);
             *o = accumulate ? *o + v : v;
         }
     }
@@ -333,8 +380,9 @@ __global__ void __launch_bounds__(32 * kColWarps) cone_bp_col_kernel(float* __re
 // the detector; rays rise by at most one voxel per in-plane voxel step; and
 // kappa fits its fixed point (under 7.9 rays per voxel height, and under 3.9
 // rays crossed inside one pixel).  Anything else stays on the general kernels.
-bool cone_col_views(const std::vector<ConeView>& views, const ConeDims& cd, std::vector<ColView>& out) {
+bool cone_col_views(const std::vector<ConeView>& views, const ConeDims& cd, std::vector<ColView>& out, bool& one) {
     out.clear();
+    one = true;
     const double nx = cd.n[0], ny = cd.n[1], nz = cd.n[2];
     if ((long long)cd.nview * cd.nu > 0x7fffffff || (long long)cd.nview * cd.nb * cd.nc > 65535) return false;
     for (const ConeView& v : views) {
@@ -389,6 +437,7 @@ bool cone_col_views(const std::vector<ConeView>& views, const ConeDims& cd, std:
         if (!(lmin > 0.0)) return false;
         const double g = 1.0 / (lmin * ez), zmax = std::max(std::fabs(q.Sz), std::fabs(nz + 128 - q.Sz));
         if (!(g < 7.9 && mmin > 1.0 && zmax * g / mmin < 3.9 && zmax * g < 1e6 && std::fabs(q.c) < 1e6)) return false;
+        one = one && std::max(std::fabs(q.Sz), std::fabs(nz - q.Sz)) * g / mmin < 0.99;
         out.push_back(q);
     }
     return true;
@@ -408,8 +457,17 @@ int cone_col_project(const ColView* d_views, const ConeDims& cd, float* d_prj, c
 
 size_t cone_col_table_bytes(const ConeDims& cd) { return sizeof(double) * (size_t)cd.nview * cd.nu * (cd.nv + 1); }
 
-int cone_col_backproject(const ColView* d_views, const ConeDims& cd, double* d_tab, float* d_img, const float* d_prj,
-                         int accumulate, cudaStream_t st) {
+template <int R>
+static void launch_bp_col(const dim3& grid, const ColView* d_views, const ConeDims& cd, bool one, const double* d_tab,
+                          float* d_img, int accumulate, int b, int c, cudaStream_t st) {
+    if (one)
+        cone_bp_col_kernel<R, true><<<grid, 32 * kColWarps, 0, st>>>(d_img, d_tab, d_views, cd, b, c, accumulate);
+    else
+        cone_bp_col_kernel<R, false><<<grid, 32 * kColWarps, 0, st>>>(d_img, d_tab, d_views, cd, b, c, accumulate);
+}
+
+int cone_col_backproject(const ColView* d_views, const ConeDims& cd, bool one, double* d_tab, float* d_img,
+                         const float* d_prj, int accumulate, cudaStream_t st) {
     const long long rows = (long long)cd.nview * cd.nu;
     const int R = cd.n[2] > 64 ? 4 : cd.n[2] > 32 ? 2 : 1;
     const dim3 grid((unsigned)((cd.n[0] + 3) / 4), (unsigned)((cd.n[1] + 1) / 2),
@@ -417,12 +475,9 @@ int cone_col_backproject(const ColView* d_views, const ConeDims& cd, double* d_t
     for (int b = 0; b < cd.nb; b++)
         for (int c = 0; c < cd.nc; c++) {
             cone_col_table_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(d_tab, d_prj, d_views, cd, b, c);
-            if (R == 4)
-                cone_bp_col_kernel<4><<<grid, 32 * kColWarps, 0, st>>>(d_img, d_tab, d_views, cd, b, c, accumulate);
-            else if (R == 2)
-                cone_bp_col_kernel<2><<<grid, 32 * kColWarps, 0, st>>>(d_img, d_tab, d_views, cd, b, c, accumulate);
-            else
-                cone_bp_col_kernel<1><<<grid, 32 * kColWarps, 0, st>>>(d_img, d_tab, d_views, cd, b, c, accumulate);
+            if (R == 4) launch_bp_col<4>(grid, d_views, cd, one, d_tab, d_img, accumulate, b, c, st);
+            else if (R == 2) launch_bp_col<2>(grid, d_views, cd, one, d_tab, d_img, accumulate, b, c, st);
+            else launch_bp_col<1>(grid, d_views, cd, one, d_tab, d_img, accumulate, b, c, st);
         }
     RN_CUDA_TRY(cudaGetLastError());
     return RN_OK;

@@ -53,12 +53,13 @@ struct ColView {
     double c, iez;             // the same with ez > 0 (rays renumbered where flip): dz0' / ez', 1 / ez'
     int m, flip;
 };
-// Fills `out` where the column kernels can take the plan (false otherwise).
-bool cone_col_views(const std::vector<ConeView>& views, const ConeDims& cd, std::vector<ColView>& out);
+// Fills `out` where the column kernels can take the plan (false otherwise);
+// `one`: no height moves over more than one ray inside a pixel.
+bool cone_col_views(const std::vector<ConeView>& views, const ConeDims& cd, std::vector<ColView>& out, bool& one);
 int cone_col_project(const ColView* d_views, const ConeDims& cd, float* d_prj, const float* d_img, cudaStream_t st);
 size_t cone_col_table_bytes(const ConeDims& cd);
-int cone_col_backproject(const ColView* d_views, const ConeDims& cd, double* d_tab, float* d_img, const float* d_prj,
-                         int accumulate, cudaStream_t st);
+int cone_col_backproject(const ColView* d_views, const ConeDims& cd, bool one, double* d_tab, float* d_img,
+                         const float* d_prj, int accumulate, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
 // Tomosynthesis (cone_tile.cu): z the main axis, u along x, v along y.
