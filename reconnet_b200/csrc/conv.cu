@@ -41,6 +41,7 @@ namespace rn {
 constexpr int kConvThreads = 128;     // one warpgroup: the 128 accumulator lanes
 constexpr int kConvTile = 128;        // output pixels per tile (MMA M)
 constexpr int kBoxW = kConvTile + 2;  // pixels per box row (halo of one on each side)
+constexpr int kWgStages = 4;          // stages of the weight gradient's load pipeline
 constexpr int kZeroBytes = 2048;      // zero rows standing in for the tenth tap of an 8-channel layer
 
 // ---- tcgen05 / TMA primitives ------------------------------------------------
@@ -136,6 +137,36 @@ __device__ __forceinline__ uint32_t tap_off(int t, int ch, int boxw = kBoxW) {
     return (uint32_t)(((t / 3) * boxw + (t % 3)) * 16);
 }
 
+// The tiles of a CTA, blockIdx.x + i gridDim.x over (n, h, tw) with tw fastest:
+// the coordinates step by the grid's own, with carries.  (Dividing a 64-bit
+// tile index out for every tile cost the producer and the epilogue about a
+// thousand cycles of latency each per tile.)
+struct TileWalk {
+    int tw, h, n;
+    int stw, sh, sn, tiles_w, H;
+    __device__ __forceinline__ TileWalk(long long first, long long step, int tiles_w_, int H_) : tiles_w(tiles_w_), H(H_) {
+        tw = (int)(first % tiles_w);
+        h = (int)(first / tiles_w % H);
+        n = (int)(first / tiles_w / H);
+        stw = (int)(step % tiles_w);
+        sh = (int)(step / tiles_w % H);
+        sn = (int)(step / tiles_w / H);
+    }
+    __device__ __forceinline__ void next() {
+        tw += stw;
+        h += sh;
+        n += sn;
+        if (tw >= tiles_w) {
+            tw -= tiles_w;
+            h++;
+        }
+        if (h >= H) {
+            h -= H;
+            n++;
+        }
+    }
+};
+
 // ---- forward / input-gradient convolution --------------------------------------
 // mode 0: out bf16 blocked = relu(conv + bias); mode 1: out fp32 [N][H][W] =
 // conv[0] + bias[0] + aux (the residual); mode 2: out bf16 blocked = conv *
@@ -217,14 +248,7 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
 
-    auto tile_coords = [&](long long i, int& n, int& h, int& w0) {
-        const long long t = blockIdx.x + i * gridDim.x;
-        const int tw = (int)(t % tiles_w);
-        const long long r = t / tiles_w;
-        h = (int)(r % a.H);
-        n = (int)(r / a.H);
-        w0 = tw * kConvTile;
-    };
+    TileWalk walk(blockIdx.x, gridDim.x, tiles_w, a.H);   // the producer's next box, or the epilogue's next tile
 
     if (warp == kConvThreads / 32) {
         if (lane == 0) {
@@ -234,10 +258,10 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
             auto issue_tma = [&](long long i) -> bool {
                 const int s = (int)(i % S);
                 if (i >= S && !mbar_wait(&bar_empty[s], (uint32_t)((i / S - 1) & 1))) return false;
-                int n, h, w0;
-                tile_coords(i, n, h, w0);
                 mbar_arrive_expect_tx(&bar_full[s], BOX_BYTES);
-                tma_load_5d(smem + s * BOX_ALLOC, &tm_in, 0, w0 / PIX - 1, h - 1, 0, n, &bar_full[s]);
+                tma_load_5d(smem + s * BOX_ALLOC, &tm_in, 0, walk.tw * (kConvTile / PIX) - 1, walk.h - 1, 0, walk.n,
+                            &bar_full[s]);
+                walk.next();
                 return true;
             };
             while (tma_next < nmine && tma_next < S - 1) issue_tma(tma_next++);
@@ -301,9 +325,8 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar_acce[acc]);
-            int n, h, w0;
-            tile_coords(j, n, h, w0);
-            const int w = w0 + tid;
+            const int n = walk.n, h = walk.h, w = walk.tw * kConvTile + tid;
+            walk.next();
             if (w < a.W) {
                 const long long pix = ((long long)n * a.H + h) * a.W + w;   // pixel index within one channel plane
                 const long long plane = (long long)a.H * a.W;
@@ -347,11 +370,36 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
     if (warp == 0) tmem_dealloc(tmem, 64);
 }
 
+// Shared memory of the weight gradient: per stage the X box as [3 rows][CH
+// chunks][box pixels][16 B], a group of ones, then the dY box, padded so that
+// the 16 groups of the A operand stay inside the allocation.
+template <int CH, int CHO, int PIX>
+struct WgradLayout {
+    static constexpr uint32_t GROUP = (kConvTile + 2 * PIX) * 16;
+    static constexpr uint32_t XBOX = 3 * CH * GROUP;
+    static constexpr uint32_t DY = (XBOX + GROUP + 127) & ~127u;
+    static constexpr uint32_t DYBOX = CHO * kConvTile * 16;
+    static constexpr uint32_t STAGE = (DY + DYBOX + 1023) & ~1023u;
+    // the last stage's operands: 16 groups of X from a start up to PIX + 1
+    // pixels in, and two dY groups where one is real
+    static constexpr uint32_t TAIL = 16 * GROUP + 1024;
+    static constexpr uint32_t BYTES = (kWgStages - 1) * STAGE + (STAGE > TAIL ? STAGE : TAIL) + 2048;
+};
+
 // ---- weight gradient -------------------------------------------------------------
-// D[co][col] accumulates over the CTA's tiles; col = tap * 32 + ci (32-channel
-// input) or pair * 16 + (tap & 1) * 8 + ci (8-channel input, taps in pairs),
-// then 16 columns of sum_p dY[p][co] (the bias gradient).  Each CTA writes its
-// partial [32][ncols] to `partial`; conv_wgrad_reduce sums them.
+// D_dx[(dy, ci)][co] = sum_p X[p + (dy, dx)][ci] dY[p][co] for the three dx, both
+// operands MN-major (8 pixels x 8 channels per 128-byte core matrix).  The X box
+// of a tile lies in shared memory as [row][chunk][pixel][8 channels], so the
+// (row, chunk) groups of 8 channels follow one another at one stride and the M
+// = 128 rows of the A operand are the 3 dy x CH chunks of 8 channels; the group
+// after them is a block of ones, whose rows give the bias gradient sum_p
+// dY[p][co].  (The groups after that read whatever follows in shared memory,
+// which only feeds accumulator rows that are never read.)  dx moves the operand
+// by one pixel.  So a tile takes 3 x 8 MMAs with N = 16 or 32; with the output
+// channels as rows (32 of 128 real) and one tap per MMA it took 80, and 0.29 ms
+// per 32-channel layer of 8 images of 512 x 512; now 0.13 ms.
+// Each CTA writes its partial [32][ncols] to `partial`; conv_wgrad_reduce sums
+// them.
 struct WgradArgs {
     float* partial;       // [gridDim.x][32][ncols]
     int N, H, W;
@@ -359,170 +407,154 @@ struct WgradArgs {
     int* err;
 };
 
-// kWgStages - 1 tiles' loads (a dY box and an X box each) stay in flight
-// ahead of the tile whose MMAs are issued; each tile's MMA groups commit to
-// its stage's "empty" barriers, which the load kWgStages - 1 tiles later
-// waits for.  Boxes take PIX pixels per TMA row as in the forward kernel.
-// The A operand (dY, M = 128 output-channel rows of which the first 8 CHO are
-// real) spans 16 groups of 8 rows 2048 bytes apart: groups past the dY box
-// read whatever shared memory follows it (more boxes), which only feeds
-// accumulator rows that are never read.
-constexpr int kWgStages = 4;
-constexpr int kWgIssuers = 2;   // MMA-issuing threads (lane 0 of warps 0 and 1)
-
+// kWgStages - 1 tiles' loads (a dY box and an X box each) stay in flight ahead
+// of the tile whose MMAs are issued; each tile's MMA group commits to its
+// stage's "empty" barrier, which the load kWgStages - 1 tiles later waits for.
+// Boxes take PIX pixels per TMA row as in the forward kernel.
 template <int CH, int CHO, int PIX>
 __global__ void __launch_bounds__(kConvThreads) conv3x3_wgrad_kernel(const __grid_constant__ CUtensorMap tm_x,
                                                                     const __grid_constant__ CUtensorMap tm_dy,
                                                                     WgradArgs a) {
+    using L = WgradLayout<CH, CHO, PIX>;
     constexpr int S = kWgStages;
-    constexpr int BOXW = kConvTile + 2 * PIX;
     constexpr uint32_t A0 = 16 * (PIX - 1);
-    constexpr uint32_t XBOX = CH * 3 * BOXW * 16;
-    constexpr uint32_t DYBOX = CHO * kConvTile * 16;
-    constexpr uint32_t DY_ALLOC = (DYBOX + 1023) & ~1023u;
-    constexpr uint32_t X_ALLOC = (XBOX + kZeroBytes + 1023) & ~1023u;
-    constexpr int NCOLS_TMEM = CH == 4 ? 512 : 128;
+    constexpr int N = CHO == 4 ? 32 : 16;          // MMA columns per dx
+    constexpr int ONES = 3 * CH;                   // first accumulator row / 8 of the bias gradient
     constexpr int BIAS_COL = CH == 4 ? 288 : 80;
-    static_assert(DY_ALLOC + S * X_ALLOC >= 16 * 2048, "the A operand's 16 row groups must stay in shared memory");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
-    unsigned char* xbox0 = smem + S * DY_ALLOC;
-    unsigned char* ones = xbox0 + S * X_ALLOC;   // 512 B of bf16 ones: the bias-gradient B operand
-    __shared__ __align__(8) uint64_t bar_full[S], bar_empty[kWgIssuers][S];
+    __shared__ __align__(8) uint64_t bar_full[S], bar_empty[S];
     __shared__ uint32_t tmem_slot;
     __shared__ int s_fail;
     const int tid = threadIdx.x, warp = tid >> 5;
     const int tiles_w = (a.W + kConvTile - 1) / kConvTile;
     const long long ntiles = (long long)a.N * a.H * tiles_w;
     const long long nmine = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    for (int i = tid; i < (int)(S * DY_ALLOC / 16); i += kConvThreads) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
-    for (int s = 0; s < S; s++)
-        for (int i = tid; i < kZeroBytes / 16; i += kConvThreads)
-            reinterpret_cast<uint4*>(xbox0 + s * X_ALLOC + XBOX)[i] = make_uint4(0, 0, 0, 0);
-    for (int i = tid; i < 512 / 4; i += kConvThreads) reinterpret_cast<uint32_t*>(ones)[i] = 0x3F803F80u;   // bf16 1.0 pairs
+    // ones after each X box; everything else cleared once (the rows that are
+    // never read stay finite)
+    for (int i = tid; i < (int)(L::BYTES / 16); i += kConvThreads) {
+        const uint32_t o = (uint32_t)i * 16 % L::STAGE;
+        const uint32_t v = o >= L::XBOX && o < L::XBOX + L::GROUP ? 0x3F803F80u : 0u;   // bf16 1.0 pairs
+        reinterpret_cast<uint4*>(smem)[i] = make_uint4(v, v, v, v);
+    }
     if (tid == 0) {
         for (int s = 0; s < S; s++) {
             mbar_init(&bar_full[s], 1);
-            for (int q = 0; q < kWgIssuers; q++) mbar_init(&bar_empty[q][s], 1);
+            mbar_init(&bar_empty[s], 1);
         }
         fence_mbar_init();
         s_fail = 0;
     }
-    if (warp == 0) tmem_alloc(&tmem_slot, NCOLS_TMEM);
+    if (warp == 0) tmem_alloc(&tmem_slot, 128);
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    auto tile_coords = [&](long long i, int& n, int& h, int& w0) {
-        const long long t = blockIdx.x + i * gridDim.x;
-        const int tw = (int)(t % tiles_w);
-        const long long r = t / tiles_w;
-        h = (int)(r % a.H);
-        n = (int)(r / a.H);
-        w0 = tw * kConvTile;
-    };
-    // kWgIssuers issuers, lane 0 of warps 0, 1, .. (warp 0's also issues the
-    // loads), split each K step's MMA slots (k < 9: tap k with 32 channels;
-    // CH = 1: k < 5 a pair of taps; the last slot the bias columns) into
-    // contiguous runs, one per issuer.  Each commits to its own "empty"
-    // barrier of the stage; a stage is refilled once every issuer's group has
-    // read it.  (Two issuers: 0.59 ms per 32-channel layer against 0.77 for
-    // one; four, dealing slots round-robin, 0.71.)
-    if ((tid & 31) == 0 && warp < kWgIssuers) {
-        const int q = warp;
+    if (tid == 0) {
         long long tma_next = 0, full_seen = 0, mma_done = 0;
         bool ok = true;
+        TileWalk walk(blockIdx.x, gridDim.x, tiles_w, a.H);
         auto issue_loads = [&](long long i) -> bool {
             const int s = (int)(i % S);
-            if (i >= S)
-                for (int r = 0; r < kWgIssuers; r++)
-                    if (!mbar_wait(&bar_empty[r][s], (uint32_t)((i / S - 1) & 1))) return false;
-            int n, h, w0;
-            tile_coords(i, n, h, w0);
-            mbar_arrive_expect_tx(&bar_full[s], XBOX + DYBOX);
-            tma_load_5d(smem + s * DY_ALLOC, &tm_dy, 0, w0 / PIX, h, 0, n, &bar_full[s]);
-            tma_load_5d(xbox0 + s * X_ALLOC, &tm_x, 0, w0 / PIX - 1, h - 1, 0, n, &bar_full[s]);
+            if (i >= S && !mbar_wait(&bar_empty[s], (uint32_t)((i / S - 1) & 1))) return false;
+            unsigned char* st = smem + s * L::STAGE;
+            mbar_arrive_expect_tx(&bar_full[s], L::XBOX + L::DYBOX);
+            tma_load_5d(st + L::DY, &tm_dy, 0, walk.tw * (kConvTile / PIX), walk.h, 0, walk.n, &bar_full[s]);
+            tma_load_5d(st, &tm_x, 0, walk.tw * (kConvTile / PIX) - 1, 0, walk.h - 1, walk.n, &bar_full[s]);
+            walk.next();
             return true;
         };
-        if (q == 0)
-            while (tma_next < nmine && tma_next < S - 1) issue_loads(tma_next++);
-        const uint32_t ob = smem_u32(ones);
+        while (tma_next < nmine && tma_next < S - 1) issue_loads(tma_next++);
+        constexpr uint32_t idesc = umma_idesc(N, true, true);
         uint32_t accum = 0;
         for (long long j = 0; j < nmine; j++) {
             const int s = (int)(j % S);
             if (!mbar_wait(&bar_full[s], (uint32_t)((j / S) & 1))) { ok = false; break; }
             full_seen = j + 1;
             tc_fence_after();
-            const uint32_t dyb = smem_u32(smem + s * DY_ALLOC), xb = smem_u32(xbox0 + s * X_ALLOC) + A0;
-            for (int k0 = 0; k0 < kConvTile; k0 += 16) {
-                const uint64_t da = umma_desc(dyb + (uint32_t)(k0 * 16), 128, kConvTile * 16);
-                constexpr int NSLOT = CH == 4 ? 10 : 6;   // taps (or tap pairs), then the bias
+            const uint32_t xb = smem_u32(smem + s * L::STAGE) + A0, dyb = smem_u32(smem + s * L::STAGE + L::DY);
 #pragma unroll
-                for (int k = 0; k < NSLOT; k++) {
-                    constexpr int PER = (NSLOT + kWgIssuers - 1) / kWgIssuers;
-                    if (k / PER != q) continue;
-                    if (k == NSLOT - 1) {
-                        const uint64_t dbo = umma_desc(ob, 128, 256);
-                        umma_bf16(tmem + (uint32_t)BIAS_COL, da, dbo, umma_idesc(16, true, true), accum);
-                    } else if (CH == 4) {
-                        const uint64_t db = umma_desc(xb + tap_off(k, CH, BOXW) + (uint32_t)(k0 * 16), 128, 3 * BOXW * 16);
-                        umma_bf16(tmem + (uint32_t)(k * 32), da, db, umma_idesc(32, true, true), accum);
-                    } else {
-                        // tap 9 is the zero rows after the box (the offset
-                        // from the shifted start is the plain one minus A0)
-                        const uint32_t o0 = tap_off(2 * k, CH, BOXW) - (2 * k >= 9 ? A0 : 0);
-                        const uint32_t o1 = tap_off(2 * k + 1, CH, BOXW) - (2 * k + 1 >= 9 ? A0 : 0);
-                        const uint64_t db = umma_desc(xb + o0 + (uint32_t)(k0 * 16), 128, o1 - o0);
-                        umma_bf16(tmem + (uint32_t)(k * 16), da, db, umma_idesc(16, true, true), accum);
-                    }
+            for (int k0 = 0; k0 < kConvTile; k0 += 16) {
+                const uint64_t db = umma_desc(dyb + (uint32_t)(k0 * 16), 128, kConvTile * 16);
+#pragma unroll
+                for (int dx = 0; dx < 3; dx++) {
+                    const uint64_t da = umma_desc(xb + (uint32_t)((k0 + dx) * 16), 128, L::GROUP);
+                    umma_bf16(tmem + (uint32_t)(dx * N), da, db, idesc, accum);
                 }
                 accum = 1;
             }
-            umma_commit(&bar_empty[q][s]);
+            umma_commit(&bar_empty[s]);
             mma_done = j + 1;
-            if (q == 0 && tma_next < nmine) {
+            if (tma_next < nmine) {
                 if (!issue_loads(tma_next)) { ok = false; break; }
                 tma_next++;
             }
         }
-        // the last group of this issuer completes after every earlier one
-        if (ok && mma_done > 0)
-            ok = mbar_wait(&bar_empty[q][(mma_done - 1) % S], (uint32_t)(((mma_done - 1) / S) & 1));
+        // the last group completes after every earlier one
+        if (ok && mma_done > 0) ok = mbar_wait(&bar_empty[(mma_done - 1) % S], (uint32_t)(((mma_done - 1) / S) & 1));
         if (!ok) {
             s_fail = 1;
             // give what is in flight its own bounded wait before the shared
             // memory and the accumulator columns are released
-            if (q == 0)
-                for (long long i = full_seen; i < tma_next; i++) mbar_wait(&bar_full[i % S], (uint32_t)((i / S) & 1));
-            if (mma_done > 0) mbar_wait(&bar_empty[q][(mma_done - 1) % S], (uint32_t)(((mma_done - 1) / S) & 1));
+            for (long long i = full_seen; i < tma_next; i++) mbar_wait(&bar_full[i % S], (uint32_t)((i / S) & 1));
+            if (mma_done > 0) mbar_wait(&bar_empty[(mma_done - 1) % S], (uint32_t)(((mma_done - 1) / S) & 1));
         }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (!s_fail && warp == 0) {
-        // lanes 0..31 hold output channels 0..31; columns in blocks of 32
+    if (!s_fail) {
+        // thread = accumulator row (dy, chunk, ci) or a bias row; columns dx N + co
         float* dst = a.partial + (long long)blockIdx.x * 32 * a.ncols;
         const bool any = nmine > 0;
-        for (int cb = 0; cb < a.ncols; cb += 32) {
+        const int g = tid >> 3, ci = tid & 7;
+#pragma unroll
+        for (int dx = 0; dx < 3; dx++) {
             float v[32];
-            tmem_ld32(tmem + (uint32_t)cb, v);
-            for (int i = 0; i < 32 && cb + i < a.ncols; i++) dst[(long long)tid * a.ncols + cb + i] = any ? v[i] : 0.f;
+            tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(dx * N), v);
+            if (g < ONES) {
+                const int tap = (g / CH) * 3 + dx;
+                const int col = CH == 4 ? tap * 32 + (g % CH) * 8 + ci : (tap / 2) * 16 + (tap % 2) * 8 + ci;
+#pragma unroll
+                for (int co = 0; co < 32; co++)
+                    dst[(long long)co * a.ncols + col] = any && co < 8 * CHO ? v[co] : 0.f;
+            } else if (g == ONES && dx == 0) {
+#pragma unroll
+                for (int co = 0; co < 32; co++) {
+                    const float t = any && co < 8 * CHO ? v[co] : 0.f;
+                    dst[(long long)co * a.ncols + BIAS_COL + ci] = t;
+                    dst[(long long)co * a.ncols + BIAS_COL + 8 + ci] = t;
+                }
+            } else if (CH == 1 && g == ONES + 1 && dx == 0) {
+                // the tenth tap of the 8-channel layout
+#pragma unroll
+                for (int co = 0; co < 32; co++) dst[(long long)co * a.ncols + 72 + ci] = 0.f;
+            }
         }
     }
     if (s_fail && tid == 0) atomicExch(a.err, RN_ERR_TIMEOUT);
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, NCOLS_TMEM);
+    if (warp == 0) tmem_dealloc(tmem, 128);
 }
 
-__global__ void conv_wgrad_reduce(float* __restrict__ out, const float* __restrict__ partial, int nparts, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// out[i] = the partials' sum in FP64, in a fixed order: 8 threads take every
+// eighth partial, then their sums in turn.  Block (32, 8).
+__global__ void __launch_bounds__(256) conv_wgrad_reduce(float* __restrict__ out, const float* __restrict__ partial,
+                                                         int nparts, int n) {
+    __shared__ double sums[8][32];
+    const int i = blockIdx.x * 32 + threadIdx.x;
     double s = 0;
-    for (int p = 0; p < nparts; p++) s += partial[(long long)p * n + i];
-    out[i] = (float)s;
+    if (i < n)
+        for (int p = threadIdx.y; p < nparts; p += 8) s += partial[(long long)p * n + i];
+    sums[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y == 0 && i < n) {
+        s = 0;
+        for (int k = 0; k < 8; k++) s += sums[k][threadIdx.x];
+        out[i] = (float)s;
+    }
 }
 
 // FP32 image [N][H][W] -> bf16 blocked with 8 channels (channel 0 = image).
@@ -555,9 +587,10 @@ static EncodeTiledFn encode_fn() {
 
 // Tensor map over a blocked activation [N][ch][H][W][8] bf16 with the pixels
 // taken in groups of `pix` (W a multiple of pix): a box of (8 pix, box_w /
-// pix, box_h, ch, 1), each of its rows 16 pix bytes.
+// pix, box_h, ch, 1), each of its rows 16 pix bytes; with `rows_outside` (8 pix,
+// box_w / pix, ch, box_h, 1).
 static int make_act_map(CUtensorMap* m, const void* base, int N, int ch, int H, int W, int box_w, int box_h,
-                        int pix = 1) {
+                        int pix = 1, bool rows_outside = false) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return set_error(RN_ERR_CUDA, "conv: cuTensorMapEncodeTiled unavailable");
     if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) return set_error(RN_ERR_ARG, "conv: activations must be 16-byte aligned");
@@ -566,6 +599,11 @@ static int make_act_map(CUtensorMap* m, const void* base, int N, int ch, int H, 
     cuuint64_t strides[4] = {(cuuint64_t)(16 * p), (cuuint64_t)W * 16, (cuuint64_t)H * W * 16, (cuuint64_t)ch * H * W * 16};
     cuuint32_t box[5] = {(cuuint32_t)(8 * p), (cuuint32_t)(box_w / p), (cuuint32_t)box_h, (cuuint32_t)ch, 1};
     cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    if (rows_outside) {   // the box's rows outside its chunks
+        std::swap(dims[2], dims[3]);
+        std::swap(strides[1], strides[2]);
+        std::swap(box[2], box[3]);
+    }
     CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -653,19 +691,17 @@ extern "C" int rn_conv3x3_wgrad(float* d_dw, float* d_partial, size_t partial_by
     auto run = [&](auto pix) -> int {
         constexpr int P = decltype(pix)::value;
         CUtensorMap mx, mdy;
-        RN_TRY(make_act_map(&mx, d_x, N, cin / 8, H, W, kConvTile + 2 * P, 3, P));
+        RN_TRY(make_act_map(&mx, d_x, N, cin / 8, H, W, kConvTile + 2 * P, 3, P, true));
         RN_TRY(make_act_map(&mdy, d_dy, N, cout / 8, H, W, kConvTile, 1, P));
-        const uint32_t xbox = (cin / 8) * 3 * (kConvTile + 2 * P) * 16;
-        const uint32_t dyb = (cout / 8) * kConvTile * 16;
-        const size_t smem = kWgStages * (((dyb + 1023) & ~1023u) + ((xbox + kZeroBytes + 1023) & ~1023u)) + 512 + 1024;
-        auto launch = [&](auto kern) -> int {
+        auto launch = [&](auto kern, size_t bytes) -> int {
+            const size_t smem = bytes + 1024;
             RN_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             kern<<<grid, kConvThreads, smem, st>>>(mx, mdy, a);
             return RN_OK;
         };
-        if (cin == 32 && cout == 32) return launch(conv3x3_wgrad_kernel<4, 4, P>);
-        if (cin == 32 && cout == 8) return launch(conv3x3_wgrad_kernel<4, 1, P>);
-        if (cin == 8 && cout == 32) return launch(conv3x3_wgrad_kernel<1, 4, P>);
+        if (cin == 32 && cout == 32) return launch(conv3x3_wgrad_kernel<4, 4, P>, WgradLayout<4, 4, P>::BYTES);
+        if (cin == 32 && cout == 8) return launch(conv3x3_wgrad_kernel<4, 1, P>, WgradLayout<4, 1, P>::BYTES);
+        if (cin == 8 && cout == 32) return launch(conv3x3_wgrad_kernel<1, 4, P>, WgradLayout<1, 4, P>::BYTES);
         return set_error(RN_ERR_ARG, "conv wgrad: unsupported channel pair");
     };
     if (W % 8 == 0) RN_TRY(run(std::integral_constant<int, 8>{}));
@@ -673,7 +709,7 @@ extern "C" int rn_conv3x3_wgrad(float* d_dw, float* d_partial, size_t partial_by
     else RN_TRY(run(std::integral_constant<int, 1>{}));
     RN_CUDA_TRY(cudaGetLastError());
     const int n = 32 * ncols;
-    conv_wgrad_reduce<<<(n + 255) / 256, 256, 0, st>>>(d_dw, d_partial, grid, n);
+    conv_wgrad_reduce<<<(n + 31) / 32, dim3(32, 8), 0, st>>>(d_dw, d_partial, grid, n);
     RN_CUDA_TRY(cudaGetLastError());
     return RN_OK;
 }
