@@ -15,6 +15,7 @@
 #include <tuple>
 #include <vector>
 
+#include "rn_device.cuh"
 #include "rn_internal.h"
 
 namespace rn {
@@ -494,8 +495,6 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool val
                  "l"(src), "r"(valid ? 4 : 0)
                  : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 struct FiltTiles {
     const float* prj;
@@ -611,7 +610,7 @@ __global__ void __launch_bounds__(256, 1) filter_reg_kernel(FiltTiles f, const f
         float* tile = tiles + b * tile_floats;
         if (it + gridDim.x < nitems) filt_issue(f, tiles + (b ^ 1) * tile_floats, it + gridDim.x);
         cp_async_commit();
-        cp_async_wait_prev();
+        cp_async_wait<1>();
         __syncthreads();
         int v0;
         filt_item(f, it, v0);
@@ -708,7 +707,7 @@ __global__ void __launch_bounds__(256, 1) filter_tr_kernel(FiltTiles f, const fl
         float* tile = tiles + b * tile_floats;
         if (it + gridDim.x < nitems) filt_issue(f, tiles + (b ^ 1) * tile_floats, it + gridDim.x);
         cp_async_commit();
-        cp_async_wait_prev();
+        cp_async_wait<1>();
         __syncthreads();
         int v0;
         filt_item(f, it, v0);
@@ -886,6 +885,14 @@ struct TvTerms {
     float grad, norm, var;
 };
 
+// 1 / sqrt(a) to about one rounding: the hardware's estimate and a Newton step
+// (a correctly rounded root and reciprocal take four times the instructions
+// and are two roundings).
+__device__ __forceinline__ float inv_sqrt(float a) {
+    const float r = rsqrtf(a);
+    return fmaf(0.5f * r, fmaf(-a * r, r, 1.0f), r);
+}
+template <bool kVar>
 __device__ __forceinline__ TvTerms tv_terms(const float* __restrict__ img, int ix, int iy, int nx, int ny,
                                             long long isx, long long isy) {
     const float* p = img + ix * isx + iy * isy;
@@ -895,14 +902,12 @@ __device__ __forceinline__ TvTerms tv_terms(const float* __restrict__ img, int i
     float dy0 = iy == 0 ? x : x - p[-isy];
     float dy1 = iy == ny - 1 ? x : x - p[isy];
     const float eps = 1e-6f;
-    float t0 = sqrtf(dx0 * dx0 + eps), t1 = sqrtf(dx1 * dx1 + eps);
-    float t2 = sqrtf(dy0 * dy0 + eps), t3 = sqrtf(dy1 * dy1 + eps);
-    // one correctly rounded reciprocal per difference instead of two divides
-    const float r0 = __frcp_rn(t0), r1 = __frcp_rn(t1), r2 = __frcp_rn(t2), r3 = __frcp_rn(t3);
+    const float a0 = dx0 * dx0 + eps, a1 = dx1 * dx1 + eps, a2 = dy0 * dy0 + eps, a3 = dy1 * dy1 + eps;
+    const float r0 = inv_sqrt(a0), r1 = inv_sqrt(a1), r2 = inv_sqrt(a2), r3 = inv_sqrt(a3);
     TvTerms r;
     r.grad = (dx0 * r0 + dx1 * r1 + dy0 * r2 + dy1 * r3) / 2;
     r.norm = r0 + r1 + r2 + r3;
-    r.var = (t0 + t1 + t2 + t3) / 2;
+    r.var = kVar ? (sqrtf(a0) + sqrtf(a1) + sqrtf(a2) + sqrtf(a3)) / 2 : 0.f;
     return r;
 }
 
@@ -913,7 +918,7 @@ __global__ void tv_kernel(float* grad, float* norm, double* tv, const float* __r
     double v = 0.0;
     if (i < nx * ny) {
         int ix = i / ny, iy = i - (i / ny) * ny;
-        TvTerms t = tv_terms(img + base, ix, iy, nx, ny, ny, 1);
+        TvTerms t = tv_terms<true>(img + base, ix, iy, nx, ny, ny, 1);
         if (grad) grad[base + i] = t.grad;
         if (norm) norm[base + i] = t.norm;
         v = (double)t.var;
@@ -960,11 +965,11 @@ __global__ void sqs_update_kernel(float* __restrict__ xo, const float* __restric
         const int iy = nzc == 1 ? j : j / nzc;
         const int zc = j - iy * nzc;
         const float* plane = xi + (long long)bb * nx * isx + zc;
-        TvTerms t = tv_terms(plane, ix, iy, nx, ny, isx, nzc);
+        TvTerms t = tv_terms<false>(plane, ix, iy, nx, ny, isx, nzc);
         num += (double)beta * t.grad;
         den += (double)beta * t.norm;
     }
-    float v = (float)((double)xi[i] - (double)lam * num / den);
+    float v = (float)((double)xi[i] - (double)lam * num * reciprocal(den));
     if (clamp) v = fminf(fmaxf(v, lb), ub);
     xo[i] = v;
 }

@@ -103,6 +103,13 @@ __device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
     return r;
 }
 
+// round-down add (for floors against 1.5 * 2^23)
+__device__ __forceinline__ f32x2 f2_add_rd(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // floor(x) and frac(x) for 0 <= x < 2^22 on the FMA/ALU pipes: the integer
 // part comes from rounding (x - 0.5) with a 1.5 * 2^23 bias.  At exact
 // integers it may return (n-1, 1.0) instead of (n, 0.0); both evaluate the
@@ -120,6 +127,17 @@ __device__ __forceinline__ float2 split_double(double v) {
     float hi = __double2float_rn(v);
     float lo = __double2float_rn(v - (double)hi);
     return make_float2(hi, lo);
+}
+
+// 1 / d in FP64 from the FP32 reciprocal by two Newton steps (each squares the
+// relative error: 1e-7, 1e-14, below FP64's own rounding), a fifth of a
+// division's instructions; outside FP32's comfortable range the division.
+__device__ __forceinline__ double reciprocal(double d) {
+    const double a = fabs(d);
+    if (!(a > 1e-30 && a < 1e30)) return 1.0 / d;
+    double r = (double)__frcp_rn((float)d);
+    r = fma(r, fma(-d, r, 1.0), r);
+    return fma(r, fma(-d, r, 1.0), r);
 }
 
 // Inclusive prefix sum over the 32 lanes of a warp (all lanes participate).
