@@ -45,9 +45,16 @@ constexpr int kWgStages = 4;          // stages of the weight gradient's load pi
 constexpr int kZeroBytes = 2048;      // zero rows standing in for the tenth tap of an 8-channel layer
 
 // ---- tcgen05 / TMA primitives ------------------------------------------------
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);   // version 1, no swizzle
+// (addresses and offsets stay below 2^18 bytes, so sums of low words do not carry
+// between their fields)
+__host__ __device__ constexpr uint32_t desc_lo(uint32_t offset, uint32_t lbo) { return (offset >> 4) + ((lbo >> 4) << 16); }
+__host__ __device__ constexpr uint32_t desc_hi(uint32_t sbo) { return (sbo >> 4) | (1u << 14); }   // version 1, no swizzle
+
+// one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
 }
 
 // kind::f16 instruction descriptor: BF16 A and B, FP32 D, M = 128.
@@ -56,12 +63,17 @@ __host__ __device__ constexpr uint32_t umma_idesc(int n, bool a_mn, bool b_mn) {
            ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accum) {
+// Matrix descriptors are given as their low word (start address and leading
+// byte offset: the loops add constants to it) and their constant high word.
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint32_t da_lo, uint32_t da_hi, uint32_t db_lo,
+                                          uint32_t db_hi, uint32_t idesc, uint32_t accum) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(accum));
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "mov.b64 a, {%1, %2};\n\t"
+        "mov.b64 b, {%3, %4};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}" ::"r"(tmem_d),
+        "r"(da_lo), "r"(da_hi), "r"(db_lo), "r"(db_hi), "r"(idesc), "r"(accum));
 }
 
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -183,14 +195,18 @@ struct ConvArgs {
     int* err;
 };
 
-// Warp-specialised pipeline.  Warp 4 (one elected lane) is the producer: it
-// keeps kConvStages - 1 TMA boxes in flight ahead of the tile whose MMAs it
-// issues, and commits each tile's MMA group twice, to the box's "empty"
-// barrier (the box may be refilled) and to the accumulator's "full" barrier.
+// Warp-specialised pipeline.  Warp 5 loads: it keeps kConvStages TMA boxes in
+// flight, refilling a stage when its "empty" barrier says that the MMAs on it are
+// done.  Warp 4 issues each tile's MMA group (one elected lane) and commits it
+// twice, to the box's "empty" barrier and to the accumulator's "full" barrier.
 // Warps 0-3 are the epilogue: thread t reads TMEM lane t (output pixel w0 + t
 // of the tile's row) from one of two accumulators of 32 columns, releases the
 // accumulator (one arrival per warp on its "empty" barrier) and stores.  So
 // the TMA copies, the MMAs of tile i and the epilogue of tile i - 1 overlap.
+// A tile's issue is one warp's serial instruction stream, which bounds the
+// kernel: the descriptors are a base and constants, stages and phases are
+// counted, and loading has its own warp.  8 images of 512 x 512, 32 to 32
+// channels: 128 us with one lane loading and issuing from 64-bit indices, now 82.
 //
 // Boxes: the tensor map views each image row as groups of PIX pixels (16 PIX
 // bytes; PIX = 8 when the width allows, else 2, else 1), so a TMA row is a
@@ -198,7 +214,7 @@ struct ConvArgs {
 // PIX - 1 pixels before the halo pixel w0 - 1 (128 + 2 PIX pixels) and the
 // operands start 16 (PIX - 1) bytes into each box row.
 constexpr int kConvStages = 3;
-constexpr int kConvWsThreads = kConvThreads + 32;
+constexpr int kConvWsThreads = kConvThreads + 64;
 
 template <int CH, int NPAD, int PIX>
 __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, ConvArgs a) {
@@ -221,7 +237,7 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tiles_w = (a.W + kConvTile - 1) / kConvTile;
     const long long ntiles = (long long)a.N * a.H * tiles_w;
-    const long long nmine = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+    const int nmine = blockIdx.x < ntiles ? (int)((ntiles - 1 - blockIdx.x) / gridDim.x) + 1 : 0;
 
     // zero rows, weights (B operand image), barriers, accumulator columns
     for (int s = 0; s < S; s++)
@@ -248,31 +264,48 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
 
-    TileWalk walk(blockIdx.x, gridDim.x, tiles_w, a.H);   // the producer's next box, or the epilogue's next tile
+    TileWalk walk(blockIdx.x, gridDim.x, tiles_w, a.H);   // the next box, or the epilogue's next tile
 
-    if (warp == kConvThreads / 32) {
-        if (lane == 0) {
-            // ---- producer ----
-            long long tma_next = 0, full_seen = 0, mma_done = 0;   // TMA issued / consumed; MMA groups issued
-            bool ok = true;
-            auto issue_tma = [&](long long i) -> bool {
-                const int s = (int)(i % S);
-                if (i >= S && !mbar_wait(&bar_empty[s], (uint32_t)((i / S - 1) & 1))) return false;
+    if (warp == kConvThreads / 32 + 1) {
+        // ---- loads ----
+        const bool leader = elect_one();
+        int s = 0, phase = 1, i = 0;   // stage, parity of its previous use
+        bool ok = true;
+        for (; i < nmine; i++) {
+            if (i >= S) ok = __all_sync(0xffffffffu, mbar_wait(&bar_empty[s], (uint32_t)phase));
+            if (!ok) break;
+            if (leader) {
                 mbar_arrive_expect_tx(&bar_full[s], BOX_BYTES);
                 tma_load_5d(smem + s * BOX_ALLOC, &tm_in, 0, walk.tw * (kConvTile / PIX) - 1, walk.h - 1, 0, walk.n,
                             &bar_full[s]);
-                walk.next();
-                return true;
-            };
-            while (tma_next < nmine && tma_next < S - 1) issue_tma(tma_next++);
-            const uint32_t idesc = umma_idesc(NPAD, false, false), bbase = smem_u32(bsm);
-            for (long long j = 0; j < nmine; j++) {
-                const int s = (int)(j % S), acc = (int)(j & 1);
-                if (!mbar_wait(&bar_full[s], (uint32_t)((j / S) & 1))) { ok = false; break; }
-                full_seen = j + 1;
-                if (j >= 2 && !mbar_wait(&bar_acce[acc], (uint32_t)(((j >> 1) - 1) & 1))) { ok = false; break; }
-                tc_fence_after();
-                const uint32_t abase = smem_u32(smem + s * BOX_ALLOC) + A0;
+            }
+            walk.next();
+            if (++s == S) {
+                s = 0;
+                phase ^= 1;
+            }
+        }
+        if (!ok) {
+            s_fail = 1;
+            // the copies in flight, before the shared memory is released
+            for (int k = max(0, i - S); k < i; k++) mbar_wait(&bar_full[k % S], (uint32_t)((k / S) & 1));
+        }
+    } else if (warp == kConvThreads / 32) {
+        // ---- MMAs ----
+        const bool leader = elect_one();
+        constexpr uint32_t idesc = umma_idesc(NPAD, false, false), hi = desc_hi(128);
+        const uint32_t a0 = desc_lo(smem_u32(smem) + A0, 0), b0 = desc_lo(smem_u32(bsm), NPAD * 16);
+        int s = 0, phase = 0, j = 0;
+        bool ok = true;
+        for (; j < nmine; j++) {
+            const int acc = j & 1;
+            ok = mbar_wait(&bar_full[s], (uint32_t)phase);
+            if (j >= 2) ok = mbar_wait(&bar_acce[acc], (uint32_t)(((j >> 1) - 1) & 1)) && ok;
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();
+            if (leader) {
+                const uint32_t alo = a0 + (uint32_t)s * (BOX_ALLOC >> 4);
 #pragma unroll
                 for (int k = 0; k < KSTEPS; k++) {
                     uint32_t aoff, lbo;
@@ -286,35 +319,43 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
                         aoff = tap_off(2 * k, CH, BOXW) - (2 * k >= 9 ? A0 : 0);
                         lbo = tap_off(2 * k + 1, CH, BOXW) - (2 * k + 1 >= 9 ? A0 : 0) - aoff;
                     }
-                    const uint64_t da = umma_desc(abase + aoff, lbo, 128);
-                    const uint64_t db = umma_desc(bbase + (uint32_t)(2 * k * NPAD * 16), NPAD * 16, 128);
-                    umma_bf16(tmem + (uint32_t)(acc * 32), da, db, idesc, k > 0 ? 1u : 0u);
+                    umma_bf16(tmem + (uint32_t)(acc * 32), alo + desc_lo(aoff, lbo), hi, b0 + (uint32_t)(2 * k * NPAD),
+                              hi, idesc, k > 0 ? 1u : 0u);
                 }
                 umma_commit(&bar_empty[s]);
                 umma_commit(&bar_accf[acc]);
-                mma_done = j + 1;
-                // the box after the ones in flight goes into the stage that
-                // tile j - 1's group is releasing
-                if (tma_next < nmine) {
-                    if (!issue_tma(tma_next)) { ok = false; break; }
-                    tma_next++;
-                }
             }
-            if (!ok) {
-                s_fail = 1;
-                // before the shared memory and the accumulator columns are
-                // released: the copies issued and not yet seen, and the last
-                // MMA group (its barrier completes after every earlier group)
-                for (long long i = full_seen; i < tma_next; i++)
-                    mbar_wait(&bar_full[i % S], (uint32_t)((i / S) & 1));
-                if (mma_done > 0)
-                    mbar_wait(&bar_empty[(mma_done - 1) % S], (uint32_t)(((mma_done - 1) / S) & 1));
+            __syncwarp();
+            if (++s == S) {
+                s = 0;
+                phase ^= 1;
             }
+        }
+        if (!ok) {
+            s_fail = 1;
+            // before the shared memory and the accumulator columns are
+            // released: the last MMA group (its barrier completes after every
+            // earlier group)
+            if (j > 0) mbar_wait(&bar_empty[(j - 1) % S], (uint32_t)(((j - 1) / S) & 1));
         }
     } else {
         // ---- epilogue: thread tid owns output pixel w0 + tid ----
-        for (long long j = 0; j < nmine; j++) {
-            const int acc = (int)(j & 1);
+        for (int j = 0; j < nmine; j++) {
+            const int acc = j & 1;
+            const int n = walk.n, h = walk.h, w = walk.tw * kConvTile + tid;
+            walk.next();
+            // the aux input is on its way while the MMAs are
+            uint4 act[NPAD / 8];
+            float res = 0.f;
+            if (w < a.W && a.mode == 2) {
+                const long long plane = (long long)a.H * a.W, o = (long long)h * a.W + w;
+#pragma unroll
+                for (int c = 0; c < NPAD / 8; c++)
+                    if (c < a.cout / 8)
+                        act[c] = reinterpret_cast<const uint4*>(a.aux)[((long long)n * (a.cout / 8) + c) * plane + o];
+            }
+            if (w < a.W && a.mode == 1)
+                res = reinterpret_cast<const float*>(a.aux)[((long long)n * a.H + h) * a.W + w];
             if (!mbar_wait(&bar_accf[acc], (uint32_t)((j >> 1) & 1))) {
                 s_fail = 1;
                 break;
@@ -325,14 +366,11 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar_acce[acc]);
-            const int n = walk.n, h = walk.h, w = walk.tw * kConvTile + tid;
-            walk.next();
             if (w < a.W) {
                 const long long pix = ((long long)n * a.H + h) * a.W + w;   // pixel index within one channel plane
                 const long long plane = (long long)a.H * a.W;
                 if (a.mode == 0 || a.mode == 2) {
                     uint4* o = reinterpret_cast<uint4*>(a.out);
-                    const uint4* act = reinterpret_cast<const uint4*>(a.aux);
                     const int cho = a.cout / 8;
 #pragma unroll
                     for (int c = 0; c < NPAD / 8; c++) {
@@ -346,19 +384,19 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
                             for (int i = 0; i < 8; i++) q[i] = fmaxf(q[i] + s_bias[c * 8 + i], 0.f);
                         } else {
                             float m[8];
-                            unpack_bf16x8(act[idx], m);
+                            unpack_bf16x8(act[c], m);
 #pragma unroll
                             for (int i = 0; i < 8; i++) q[i] = m[i] > 0.f ? q[i] : 0.f;
                         }
                         o[idx] = pack_bf16x8(q);
                     }
                 } else if (a.mode == 1) {
-                    const float* res = reinterpret_cast<const float*>(a.aux);
-                    reinterpret_cast<float*>(a.out)[pix] = v[0] + s_bias[0] + res[pix];
+                    reinterpret_cast<float*>(a.out)[pix] = v[0] + s_bias[0] + res;
                 } else {
                     float* o = reinterpret_cast<float*>(a.out);
-                    for (int c = 0; c < a.cout; c++)
-                        o[((long long)n * a.cout + c) * plane + (long long)h * a.W + w] = v[c] + s_bias[c];
+#pragma unroll
+                    for (int c = 0; c < NPAD; c++)   // (constant indices keep v in registers)
+                        if (c < a.cout) o[((long long)n * a.cout + c) * plane + (long long)h * a.W + w] = v[c] + s_bias[c];
                 }
             }
         }
@@ -396,8 +434,10 @@ struct WgradLayout {
 // dY[p][co].  (The groups after that read whatever follows in shared memory,
 // which only feeds accumulator rows that are never read.)  dx moves the operand
 // by one pixel.  So a tile takes 3 x 8 MMAs with N = 16 or 32; with the output
-// channels as rows (32 of 128 real) and one tap per MMA it took 80, and 0.29 ms
-// per 32-channel layer of 8 images of 512 x 512; now 0.13 ms.
+// channels as rows (32 of 128 real) and one tap per MMA it took 80.  The issue of
+// a tile is one warp's serial stream and bounds the kernel: a 32-channel layer of 8
+// images of 512 x 512 took 0.29 ms with 80 MMAs, 0.13 with 24 issued by the lane
+// that also loads, and takes 0.076 ms with the loads in their own warp.
 // Each CTA writes its partial [32][ncols] to `partial`; conv_wgrad_reduce sums
 // them.
 struct WgradArgs {
@@ -407,9 +447,9 @@ struct WgradArgs {
     int* err;
 };
 
-// kWgStages - 1 tiles' loads (a dY box and an X box each) stay in flight ahead
-// of the tile whose MMAs are issued; each tile's MMA group commits to its
-// stage's "empty" barrier, which the load kWgStages - 1 tiles later waits for.
+// Warp 1 keeps kWgStages tiles' loads (a dY box and an X box each) in flight;
+// warp 0 issues the MMAs, and each tile's group commits to its stage's "empty"
+// barrier, which the load kWgStages tiles later waits for.
 // Boxes take PIX pixels per TMA row as in the forward kernel.
 template <int CH, int CHO, int PIX>
 __global__ void __launch_bounds__(kConvThreads) conv3x3_wgrad_kernel(const __grid_constant__ CUtensorMap tm_x,
@@ -429,7 +469,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_wgrad_kernel(const __gri
     const int tid = threadIdx.x, warp = tid >> 5;
     const int tiles_w = (a.W + kConvTile - 1) / kConvTile;
     const long long ntiles = (long long)a.N * a.H * tiles_w;
-    const long long nmine = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+    const int nmine = blockIdx.x < ntiles ? (int)((ntiles - 1 - blockIdx.x) / gridDim.x) + 1 : 0;
     // ones after each X box; everything else cleared once (the rows that are
     // never read stay finite)
     for (int i = tid; i < (int)(L::BYTES / 16); i += kConvThreads) {
@@ -451,55 +491,64 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_wgrad_kernel(const __gri
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    if (tid == 0) {
-        long long tma_next = 0, full_seen = 0, mma_done = 0;
-        bool ok = true;
+    if (warp == 1) {
+        // ---- loads ----
+        const bool leader = elect_one();
         TileWalk walk(blockIdx.x, gridDim.x, tiles_w, a.H);
-        auto issue_loads = [&](long long i) -> bool {
-            const int s = (int)(i % S);
-            if (i >= S && !mbar_wait(&bar_empty[s], (uint32_t)((i / S - 1) & 1))) return false;
-            unsigned char* st = smem + s * L::STAGE;
-            mbar_arrive_expect_tx(&bar_full[s], L::XBOX + L::DYBOX);
-            tma_load_5d(st + L::DY, &tm_dy, 0, walk.tw * (kConvTile / PIX), walk.h, 0, walk.n, &bar_full[s]);
-            tma_load_5d(st, &tm_x, 0, walk.tw * (kConvTile / PIX) - 1, 0, walk.h - 1, walk.n, &bar_full[s]);
-            walk.next();
-            return true;
-        };
-        while (tma_next < nmine && tma_next < S - 1) issue_loads(tma_next++);
-        constexpr uint32_t idesc = umma_idesc(N, true, true);
-        uint32_t accum = 0;
-        for (long long j = 0; j < nmine; j++) {
-            const int s = (int)(j % S);
-            if (!mbar_wait(&bar_full[s], (uint32_t)((j / S) & 1))) { ok = false; break; }
-            full_seen = j + 1;
-            tc_fence_after();
-            const uint32_t xb = smem_u32(smem + s * L::STAGE) + A0, dyb = smem_u32(smem + s * L::STAGE + L::DY);
-#pragma unroll
-            for (int k0 = 0; k0 < kConvTile; k0 += 16) {
-                const uint64_t db = umma_desc(dyb + (uint32_t)(k0 * 16), 128, kConvTile * 16);
-#pragma unroll
-                for (int dx = 0; dx < 3; dx++) {
-                    const uint64_t da = umma_desc(xb + (uint32_t)((k0 + dx) * 16), 128, L::GROUP);
-                    umma_bf16(tmem + (uint32_t)(dx * N), da, db, idesc, accum);
-                }
-                accum = 1;
+        int s = 0, phase = 1, i = 0;   // stage, parity of its previous use
+        bool ok = true;
+        for (; i < nmine; i++) {
+            if (i >= S) ok = __all_sync(0xffffffffu, mbar_wait(&bar_empty[s], (uint32_t)phase));
+            if (!ok) break;
+            if (leader) {
+                unsigned char* st = smem + s * L::STAGE;
+                mbar_arrive_expect_tx(&bar_full[s], L::XBOX + L::DYBOX);
+                tma_load_5d(st + L::DY, &tm_dy, 0, walk.tw * (kConvTile / PIX), walk.h, 0, walk.n, &bar_full[s]);
+                tma_load_5d(st, &tm_x, 0, walk.tw * (kConvTile / PIX) - 1, 0, walk.h - 1, walk.n, &bar_full[s]);
             }
-            umma_commit(&bar_empty[s]);
-            mma_done = j + 1;
-            if (tma_next < nmine) {
-                if (!issue_loads(tma_next)) { ok = false; break; }
-                tma_next++;
+            walk.next();
+            if (++s == S) {
+                s = 0;
+                phase ^= 1;
             }
         }
-        // the last group completes after every earlier one
-        if (ok && mma_done > 0) ok = mbar_wait(&bar_empty[(mma_done - 1) % S], (uint32_t)(((mma_done - 1) / S) & 1));
         if (!ok) {
             s_fail = 1;
-            // give what is in flight its own bounded wait before the shared
-            // memory and the accumulator columns are released
-            for (long long i = full_seen; i < tma_next; i++) mbar_wait(&bar_full[i % S], (uint32_t)((i / S) & 1));
-            if (mma_done > 0) mbar_wait(&bar_empty[(mma_done - 1) % S], (uint32_t)(((mma_done - 1) / S) & 1));
+            // the copies in flight, before the shared memory is released
+            for (int k = max(0, i - S); k < i; k++) mbar_wait(&bar_full[k % S], (uint32_t)((k / S) & 1));
         }
+    } else if (warp == 0) {
+        // ---- MMAs ----
+        const bool leader = elect_one();
+        constexpr uint32_t idesc = umma_idesc(N, true, true);
+        constexpr uint32_t ahi = desc_hi(L::GROUP), bhi = desc_hi(kConvTile * 16);
+        const uint32_t a0 = desc_lo(smem_u32(smem) + A0, 128), b0 = desc_lo(smem_u32(smem) + L::DY, 128);
+        int s = 0, phase = 0, j = 0;
+        bool ok = true;
+        for (; j < nmine; j++) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&bar_full[s], (uint32_t)phase));
+            if (!ok) break;
+            tc_fence_after();
+            if (leader) {
+                const uint32_t alo = a0 + (uint32_t)s * (L::STAGE >> 4), blo = b0 + (uint32_t)s * (L::STAGE >> 4);
+#pragma unroll
+                for (int k0 = 0; k0 < kConvTile; k0 += 16)
+#pragma unroll
+                    for (int dx = 0; dx < 3; dx++)
+                        umma_bf16(tmem + (uint32_t)(dx * N), alo + (uint32_t)(k0 + dx), ahi, blo + (uint32_t)k0, bhi,
+                                  idesc, k0 > 0 || j > 0 ? 1u : 0u);
+                umma_commit(&bar_empty[s]);
+            }
+            __syncwarp();
+            if (++s == S) {
+                s = 0;
+                phase ^= 1;
+            }
+        }
+        if (!ok) s_fail = 1;
+        // the last group completes after every earlier one; where a wait gave
+        // up, before the shared memory and the accumulator columns are released
+        if (j > 0 && !mbar_wait(&bar_empty[(j - 1) % S], (uint32_t)(((j - 1) / S) & 1))) s_fail = 1;
     }
     tc_fence_before();
     __syncthreads();
