@@ -97,7 +97,7 @@ __global__ void edge_slope_kernel(double* edges, const double2* view_cs, const i
 // each warp scans lines from there, 128 positions at a time, a lane owning 4
 // consecutive ones.  Where that makes too few blocks to fill the chip (or a
 // block's lines do not fit in shared memory) a CTA takes 8 lines, one per warp,
-// straight from the image: one slice of 512 x 512 takes 5.9 us that way and 9.5
+// straight from the image: one slice of 512 x 512 takes 12 us that way and 19
 // in blocks of 16, 16 slices 65 us against 44 in blocks.
 constexpr int kLineBlock = 16;
 constexpr int kLineCols = kLineBlock + 1;
@@ -592,6 +592,8 @@ __global__ void __launch_bounds__(FpCfg<kSiddon>::threads, 1) fan_fp_kernel(FpPa
 //   matched (type 2): W_u = prj * L_u; entry e < nu = {Qhi, Qlo, W_e/(r_{e+1}-r_e), r_e}
 //   reference (0/1):  W_u = prj * (L_u if type 0); entry k <= nu = {Uhi, Ulo, W_k, 0}
 // with Q/U the FP64 prefix over u; stored at index e+1 after a guard entry.
+// The rows of every backprojection table are in the class-sorted view order
+// (X-class views first).
 //
 // First all threads load the views' weighted values into shared memory, eight
 // neighbouring views per 32-byte sector and every load in flight at once; then
@@ -605,6 +607,7 @@ static size_t table_smem_bytes(int nu) { return sizeof(float) * kTabViews * (siz
 
 __global__ void __launch_bounds__(256) fan_table_kernel(const float* __restrict__ prj, const BpSlice* __restrict__ bps,
                                                         int s_begin, int ns, const GeoSet* __restrict__ sets,
+                                                        const int* __restrict__ perm,
                                                         const ViewGeo* __restrict__ views,
                                                         const double* __restrict__ edges,
                                                         const float2* __restrict__ cell, FanDims d, int type,
@@ -619,9 +622,10 @@ __global__ void __launch_bounds__(256) fan_table_kernel(const float* __restrict_
     if (v0 >= gs.nview) return;   // the whole block
     const int nu = d.nu, nup = (nu + 127) & ~127, stride = nup + 4;
     {
-        const int v = threadIdx.x & (kTabViews - 1), vl = v0 + v;
-        const bool have = vl < gs.nview;
-        const ViewGeo& vg = views[gs.view_off + min(vl, gs.nview - 1)];
+        const int v = threadIdx.x & (kTabViews - 1);
+        const bool have = v0 + v < gs.nview;
+        const int vl = perm[gs.view_off + min(v0 + v, gs.nview - 1)];
+        const ViewGeo& vg = views[gs.view_off + vl];
         const float lenA = vg.xcls ? d.dy : d.dx;
         const float half = 0.5f * vg.sigma;
 #pragma unroll 4
@@ -647,13 +651,13 @@ __global__ void __launch_bounds__(256) fan_table_kernel(const float* __restrict_
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int vl = v0 + warp;
-    if (vl >= gs.nview) return;   // the whole warp
-    const double* ed = edges + (long long)(gs.view_off + vl) * (nu + 1);
+    const int row = v0 + warp;
+    if (row >= gs.nview) return;   // the whole warp
+    const double* ed = edges + (long long)(gs.view_off + perm[gs.view_off + row]) * (nu + 1);
     // per view: index 0 is a guard entry (prefix 0, slope 0), index e+1 holds
     // edge / cell e, index nu+1 the total with slope 0; indices outside the
     // detector therefore evaluate to 0 or the total without clamping
-    float4* out = tab + (bs.table_off - tab_base) + (long long)vl * (nu + 2);
+    float4* out = tab + (bs.table_off - tab_base) + (long long)row * (nu + 2);
     const bool matched = type == RN_TYPE_MATCHED;
     if (lane == 0) out[0] = make_float4(0.f, 0.f, 0.f, matched ? (float)ed[0] : 0.f);
     out += 1;
@@ -738,20 +742,21 @@ __global__ void bp_parts_sum_kernel(float* __restrict__ out, const float* __rest
 // slice's detector rows; entry 0 is a guard (C = 0) and entry nu + 1 holds
 // the total.  c_u is C_(u+1) - C_u of two neighbouring entries.
 __global__ void siddon_table_kernel(const float* __restrict__ prj, const BpSlice* __restrict__ bps, int s_begin,
-                                    int ns, const GeoSet* __restrict__ sets, const ViewGeo* __restrict__ views,
-                                    const double* __restrict__ cslopes, FanDims d, float4* __restrict__ tab,
+                                    int ns, const GeoSet* __restrict__ sets, const int* __restrict__ perm,
+                                    const ViewGeo* __restrict__ views, const double* __restrict__ cslopes, FanDims d,
+                                    float4* __restrict__ tab,
                                     long long tab_base) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int si = blockIdx.y;
     if (si >= ns) return;
     const BpSlice bs = bps[s_begin + si];
     const GeoSet gs = sets[bs.set];
-    const int vl = blockIdx.x * 8 + warp;
-    if (vl >= gs.nview) return;
-    const int gv = gs.view_off + vl;
+    const int row = blockIdx.x * 8 + warp;
+    if (row >= gs.nview) return;
+    const int vl = perm[gs.view_off + row], gv = gs.view_off + vl;
     const int nu = d.nu;
     const double along = views[gv].xcls ? d.dx : d.dy, across = views[gv].xcls ? d.dy : d.dx;
-    float4* out = tab + (bs.table_off - tab_base) + (long long)vl * (nu + 2);
+    float4* out = tab + (bs.table_off - tab_base) + (long long)row * (nu + 2);
     double carry = 0.0;
     for (int u0 = 0; u0 < nu; u0 += 32) {
         const int u = u0 + lane;
@@ -790,21 +795,22 @@ __global__ void siddon_table_kernel(const float* __restrict__ prj, const BpSlice
 // pitch: with rho = kappa r = tan(psi), psi moving by +du (X class) or -du
 // (Y class) per cell towards negative u.
 __global__ void pd_table_kernel(const float* __restrict__ prj, const BpSlice* __restrict__ bps, int s_begin, int ns,
-                                const GeoSet* __restrict__ sets, const ViewGeo* __restrict__ views,
-                                const double* __restrict__ cslopes, FanDims d, float4* __restrict__ tab,
+                                const GeoSet* __restrict__ sets, const int* __restrict__ perm,
+                                const ViewGeo* __restrict__ views, const double* __restrict__ cslopes, FanDims d,
+                                float4* __restrict__ tab,
                                 long long tab_base) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int si = blockIdx.y;
     if (si >= ns) return;
     const BpSlice bs = bps[s_begin + si];
     const GeoSet gs = sets[bs.set];
-    const int vl = blockIdx.x * 8 + warp;
-    if (vl >= gs.nview) return;
-    const int gv = gs.view_off + vl;
+    const int row = blockIdx.x * 8 + warp;
+    if (row >= gs.nview) return;
+    const int vl = perm[gs.view_off + row], gv = gs.view_off + vl;
     const int nu = d.nu;
     const int xcls = views[gv].xcls;
     const double dso2 = (double)d.dso * d.dso;
-    float4* out = tab + (bs.table_off - tab_base) + (long long)vl * (nu + 2);
+    float4* out = tab + (bs.table_off - tab_base) + (long long)row * (nu + 2);
     auto value = [&](int u) -> float {
         if (u < 0 || u >= nu) return 0.f;
         float w = 0.f;
@@ -837,67 +843,94 @@ __global__ void pd_table_kernel(const float* __restrict__ prj, const BpSlice* __
 // right edge of lane 30's column.  The staged table window T starts at table
 // index ilo; entries carry the prefix (hi, lo), the slope scaled by sigma / 2
 // and the edge slope r_e.
-// H at slope r: prefix (hi) and the rest (lo + slope * (r - r_e)) of the
-// table entry of the cell that contains r.
-__device__ __forceinline__ void bp_h(const TCubic& c, float r, const float4* T, int ilo, int imax, float& hi,
-                                     float& rest) {
-    const float h = r - c.rt;
-    const float t = fmaf(h, fmaf(h, fmaf(h, c.c3, c.c2), c.c1), c.c0);
-    // table index floor(t) + 1 for |t| < 2^22 via a round-down add; beyond
-    // the detector it reaches a zero-slope guard entry
-    int i = __float_as_int(__fadd_rd(t, 12582912.0f)) - (0x4B400000 - 1);
-    i = min(max(i, ilo), imax);
-    const float4 E = T[i - ilo];
-    hi = E.x;
-    rest = fmaf(E.z, r - E.w, E.y);
+// Two neighbouring lattice points of a lane: their edge indices are packed FP32
+// arithmetic (one instruction for both), the table entries and the values H =
+// hi + rest = prefix + (lo + slope * (r - r_e)) of the cells that contain the
+// slopes are not.  kFast: the staged window holds every entry the tile touches
+// (BpView::inside), so the index needs no clamp; `tbase` is then the byte
+// address of the entry of edge index 0 less the bias of the round-down add.
+struct HPair {
+    float hi[2], rest[2];
+};
+// The slopes are a * b (+ 0): a * b - r_e and a * b - r_t are each rounded once.
+template <bool kFast>
+__device__ __forceinline__ HPair bp_h2(const TCubic& c, f32x2 a, f32x2 b, f32x2 nrt, const float4* T, uint32_t tbase,
+                                       int ilo, int imax) {
+    const f32x2 h = f2_fma(a, b, nrt);
+    const f32x2 t = f2_fma(h, f2_fma(h, f2_fma(h, f2_pack(c.c3, c.c3), f2_pack(c.c2, c.c2)), f2_pack(c.c1, c.c1)),
+                           f2_pack(c.c0, c.c0));
+    const float2 tt = f2_unpack(t), aa = f2_unpack(a), bb = f2_unpack(b);
+    HPair o;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const float tk = k ? tt.y : tt.x, ak = k ? aa.y : aa.x, bk = k ? bb.y : bb.x;
+        // table index floor(t) + 1 for |t| < 2^22 via a round-down add; beyond
+        // the detector it reaches a zero-slope guard entry
+        const int bits = __float_as_int(__fadd_rd(tk, 12582912.0f));
+        float4 E;
+        if (kFast) {
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(E.x), "=f"(E.y), "=f"(E.z), "=f"(E.w)
+                         : "r"(tbase + (uint32_t)bits * 16u));
+        } else {
+            E = T[min(max(bits - (0x4B400000 - 1), ilo), imax) - ilo];
+        }
+        o.hi[k] = E.x;
+        o.rest[k] = fmaf(E.z, fmaf(ak, bk, -E.w), E.y);
+    }
+    return o;
 }
 
-// X-class view (lattice lines are rows): the lane's lattice column q = x,
-// lines y0 .. y0 + kBmRows.  Pixel (x, y) receives the footprint difference
-// with the next lane's column on line y and, if line y + 1 exists, on line
-// y + 1.
-__device__ __forceinline__ void bp_matched_x(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
-                                             int imax, int x, int y0, int ny) {
+// X-class view (lattice lines are rows): the lane's lattice column q = x, lines
+// y0 .. y0 + kBmRows.  Line j's footprint difference with the next lane's column
+// goes to line[j]; a pixel is the sum of its two lines' totals, formed once
+// after all views.
+template <bool kFast>
+__device__ __forceinline__ void bp_matched_x(float (&line)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
+                                             int imax, int x, int y0) {
     const float A = (float)x - vg.par;
     // (approximate reciprocals: a relative error in 1 / (l - perp) scales all
     // slopes of a line alike)
     const TCubic c = t_cubic(vg, A * __fdividef(1.0f, (float)(y0 + kBmRows / 2) - vg.perp));
-    float dprev = 0.f;
+    const uint32_t tbase = smem_u32(T) + (uint32_t)(1 - ilo - 0x4B400000) * 16u;
+    const f32x2 nrt = f2_pack(-c.rt, -c.rt), A2 = f2_pack(A, A);
+    const f32x2 y2 = f2_pack((float)y0, (float)y0), nperp2 = f2_pack(-vg.perp, -vg.perp);
 #pragma unroll
-    for (int j = 0; j <= kBmRows; j++) {
-        const float r = A * __fdividef(1.0f, (float)(y0 + j) - vg.perp);
-        float hi, rest;
-        bp_h(c, r, T, ilo, imax, hi, rest);
-        const float nhi = __shfl_down_sync(0xffffffffu, hi, 1);
-        const float nrest = __shfl_down_sync(0xffffffffu, rest, 1);
-        const float d = (nhi - hi) + (nrest - rest);
-        if (j > 0) acc[j - 1] += fmaf((y0 + j < ny) ? 1.f : 0.f, d, dprev);
-        dprev = d;
+    for (int j = 0; j <= kBmRows; j += 2) {
+        // (y0 + j is exact: one rounding per line, the same for its points)
+        const float2 D = f2_unpack(f2_add(f2_add(y2, f2_pack((float)j, (float)min(j + 1, kBmRows))), nperp2));
+        const f32x2 g = f2_pack(__fdividef(1.0f, D.x), __fdividef(1.0f, D.y));
+        const HPair H = bp_h2<kFast>(c, A2, g, nrt, T, tbase, ilo, imax);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            if (j + k > kBmRows) break;
+            const float nhi = __shfl_down_sync(0xffffffffu, H.hi[k], 1);
+            const float nrest = __shfl_down_sync(0xffffffffu, H.rest[k], 1);
+            line[j + k] += (nhi - H.hi[k]) + (nrest - H.rest[k]);
+        }
     }
 }
 
 // Y-class view (lattice lines are columns): the lane's line l = x, lattice
-// points q = y0 .. y0 + kBmRows.  Pixel (x, y) receives the difference along
-// line x and, if line x + 1 exists, the next lane's difference along it.
-__device__ __forceinline__ void bp_matched_y(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
-                                             int imax, int x, int y0, int nx) {
+// points q = y0 .. y0 + kBmRows.  The differences along line x go to line[j];
+// pixel (x, y) is its own and the next lane's, formed once after all views.
+template <bool kFast>
+__device__ __forceinline__ void bp_matched_y(float (&line)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
+                                             int imax, int x, int y0) {
     const float g = __fdividef(1.0f, (float)x - vg.perp);
     const float r0 = ((float)y0 - vg.par) * g;
     const TCubic c = t_cubic(vg, fmaf((float)(kBmRows / 2), g, r0));
-    const float m = (x + 1 < nx) ? 1.f : 0.f;
-    float hprev = 0.f, rprev = 0.f;
+    const uint32_t tbase = smem_u32(T) + (uint32_t)(1 - ilo - 0x4B400000) * 16u;
+    const f32x2 nrt = f2_pack(-c.rt, -c.rt), g2 = f2_pack(g, g), r02 = f2_pack(r0, r0);
+    float hp = 0.f, rp = 0.f;
 #pragma unroll
-    for (int j = 0; j <= kBmRows; j++) {
-        const float r = fmaf((float)j, g, r0);
-        float hi, rest;
-        bp_h(c, r, T, ilo, imax, hi, rest);
-        if (j > 0) {
-            const float d = (hi - hprev) + (rest - rprev);
-            const float nd = __shfl_down_sync(0xffffffffu, d, 1);
-            acc[j - 1] += fmaf(m, nd, d);
-        }
-        hprev = hi;
-        rprev = rest;
+    for (int j = 0; j <= kBmRows; j += 2) {
+        const HPair H = bp_h2<kFast>(c, f2_fma(f2_pack((float)j, (float)min(j + 1, kBmRows)), g2, r02), f2_pack(1.f, 1.f),
+                                     nrt, T, tbase, ilo, imax);
+        if (j > 0) line[j - 1] += (H.hi[0] - hp) + (H.rest[0] - rp);
+        if (j < kBmRows) line[j] += (H.hi[1] - H.hi[0]) + (H.rest[1] - H.rest[0]);
+        hp = H.hi[1];
+        rp = H.rest[1];
     }
 }
 
@@ -970,7 +1003,7 @@ __device__ __noinline__ void siddon_F(const float4* T, int ilo, int imax, int nu
     }
 }
 
-__device__ __forceinline__ void bp_siddon_x(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
+__device__ __forceinline__ void bp_siddon_x(float (&acc)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
                                             int imax, int x, int y0, int nu) {
     const float A = (float)x - vg.par;
     const TCubic c = t_cubic(vg, A * __fdividef(1.0f, (float)(y0 + kBmRows / 2) - vg.perp));
@@ -995,7 +1028,7 @@ __device__ __forceinline__ void bp_siddon_x(float (&acc)[kBmRows], const BpView&
     }
 }
 
-__device__ __forceinline__ void bp_siddon_y(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
+__device__ __forceinline__ void bp_siddon_y(float (&acc)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
                                             int imax, int x, int y0, int nu) {
     const float g = __fdividef(1.0f, (float)x - vg.perp);
     const float r0 = ((float)y0 - vg.par) * g;
@@ -1043,7 +1076,7 @@ __device__ __forceinline__ void ref_u(float t, const float4* T, int ilo, int ima
     rest = fmaf(fr, E.z, E.y);
 }
 
-__device__ __forceinline__ void bp_ref_x(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
+__device__ __forceinline__ void bp_ref_x(float (&acc)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
                                          int imax, int x, int y0, int nu, bool fbp, float dq, float dl, float dso2) {
     const float A = (float)x - vg.par;
     const TCubic c = t_cubic(vg, A * __fdividef(1.0f, (float)(y0 + kBmRows / 2) - vg.perp));
@@ -1067,7 +1100,7 @@ __device__ __forceinline__ void bp_ref_x(float (&acc)[kBmRows], const BpView& vg
     }
 }
 
-__device__ __forceinline__ void bp_ref_y(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
+__device__ __forceinline__ void bp_ref_y(float (&acc)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
                                          int imax, int x, int y0, int nu, bool fbp, float dq, float dl, float dso2) {
     const float D = (float)x + 0.5f - vg.perp;
     const float g = __fdividef(1.0f, D);
@@ -1127,7 +1160,7 @@ __device__ __forceinline__ float pd_sample(const float4* T, int ilo, int imax, f
 
 
 // X-class view: lane column q = x, pixel rows y0 + j (centres l = y0 + j + 1/2).
-__device__ __forceinline__ void bp_pixel_x(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
+__device__ __forceinline__ void bp_pixel_x(float (&acc)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
                                            int imax, int x, int y0, float dq, float dl) {
     const float A = (float)x + 0.5f - vg.par;
     const TCubic c = t_cubic(vg, A * __fdividef(1.0f, (float)(y0 + kBmRows / 2) - vg.perp));
@@ -1146,7 +1179,7 @@ __device__ __forceinline__ void bp_pixel_x(float (&acc)[kBmRows], const BpView& 
 }
 
 // Y-class view: lane line l = x (centre x + 1/2), positions q = y0 + j + 1/2.
-__device__ __forceinline__ void bp_pixel_y(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
+__device__ __forceinline__ void bp_pixel_y(float (&acc)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
                                            int imax, int x, int y0, float dq, float dl) {
     const float g = __fdividef(1.0f, (float)x + 0.5f - vg.perp);
     const float r0 = ((float)y0 + 0.5f - vg.par) * g;
@@ -1169,7 +1202,7 @@ __device__ __forceinline__ void bp_pixel_y(float (&acc)[kBmRows], const BpView& 
 // Siddon tiles run three CTAs per SM (80 registers, 180 vs 174 Gupd/s at two
 // CTAs); the DD modes keep the compiler's register choice (71 / 80).
 template <int kMode>
-__global__ void __launch_bounds__(kBpThreads, (kMode == 2 || kMode == 0) ? 3 : 0) fan_bp_kernel(BpParams p) {
+__global__ void __launch_bounds__(kBpThreads, kMode == 3 ? 0 : 3) fan_bp_kernel(BpParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     BpShared* sh = reinterpret_cast<BpShared*>(smem);
     size_t off = (sizeof(BpShared) + 127) & ~size_t(127);
@@ -1239,10 +1272,21 @@ __global__ void __launch_bounds__(kBpThreads, (kMode == 2 || kMode == 0) ? 3 : 0
     __syncthreads();
     if (tid == 0) issue(0);
 
-    // accumulators: acc[j] = pixel (x0, y0 + j)
-    float acc[kBmRows];
+    // accumulators: acc[j] = pixel (x0, y0 + j); in matched mode line totals,
+    // first of the X-class views (line y0 + j), whose pixels go to `px` when
+    // the Y-class ones begin
+    float acc[kBmRows + 1], px[kBmRows];
 #pragma unroll
-    for (int a = 0; a < kBmRows; a++) acc[a] = 0.f;
+    for (int a = 0; a <= kBmRows; a++) acc[a] = 0.f;
+#pragma unroll
+    for (int a = 0; a < kBmRows; a++) px[a] = 0.f;
+    bool xphase = kMode == 1;
+    // an X-class line y0 + j counts for the pixels on both sides of it; line ny
+    // does not exist
+    auto x_pixels = [&]() {
+#pragma unroll
+        for (int a = 0; a < kBmRows; a++) px[a] = acc[a] + (y0 + a + 1 < ny ? acc[a + 1] : 0.f);
+    };
 
     // One barrier per chunk: after it every warp has finished chunk c - 1, so
     // buffer (c + 1) & 1 and record slot c & 1 may be refilled; window and
@@ -1279,8 +1323,19 @@ __global__ void __launch_bounds__(kBpThreads, (kMode == 2 || kMode == 0) ? 3 : 0
                 if (vg.xcls) bp_siddon_x(acc, vg, T, ilo, imax, x0, y0, nu);
                 else bp_siddon_y(acc, vg, T, ilo, imax, x0, y0, nu);
             } else if (kMode == 1) {
-                if (vg.xcls) bp_matched_x(acc, vg, T, ilo, imax, x0, y0, ny);
-                else bp_matched_y(acc, vg, T, ilo, imax, x0, y0, nx);
+                if (xphase && !vg.xcls) {   // once: views are sorted by class
+                    x_pixels();
+                    xphase = false;
+#pragma unroll
+                    for (int a = 0; a <= kBmRows; a++) acc[a] = 0.f;
+                }
+                if (vg.inside) {
+                    if (xphase) bp_matched_x<true>(acc, vg, T, ilo, imax, x0, y0);
+                    else bp_matched_y<true>(acc, vg, T, ilo, imax, x0, y0);
+                } else {
+                    if (xphase) bp_matched_x<false>(acc, vg, T, ilo, imax, x0, y0);
+                    else bp_matched_y<false>(acc, vg, T, ilo, imax, x0, y0);
+                }
             } else {
                 const bool fbp = p.type == RN_TYPE_FBP;
                 const float dso2 = p.d.dso * p.d.dso;
@@ -1290,6 +1345,20 @@ __global__ void __launch_bounds__(kBpThreads, (kMode == 2 || kMode == 0) ? 3 : 0
         }
     }
     if (!ok) return;
+    if (kMode == 1) {
+        if (xphase) {
+            x_pixels();
+#pragma unroll
+            for (int j = 0; j < kBmRows; j++) acc[j] = px[j];
+        } else {
+            // a Y-class line x counts for the pixels on both sides of it; line nx does not exist
+#pragma unroll
+            for (int j = 0; j < kBmRows; j++) {
+                const float next = __shfl_down_sync(0xffffffffu, acc[j], 1);
+                acc[j] = px[j] + (acc[j] + (x0 + 1 < nx ? next : 0.f));
+            }
+        }
+    }
 
     float* out = (p.nparts > 1 ? p.parts + part * p.part_stride : p.img) + bs.img_off;
     const bool add = p.nparts == 1 && p.accumulate;
@@ -1432,7 +1501,16 @@ int fan_build_geometry(rn_fan_plan* p, const float* host_deg, FanGeoHost& gh) {
             int nl = xc ? g.ny : g.nx;
             double side = (nl / 2.0 - q.perp) > 0 ? 1.0 : -1.0;
             q.sigma = (float)((r1 > r0 ? 1.0 : -1.0) * side);
-            q.pad[0] = q.pad[1] = q.pad[2] = 0;
+            // The edge-index cubic (t_cubic) over a lane's 17 lattice points, for
+            // any lane of the image's tiles (31 columns, 128 rows; the last ones
+            // reach past the image): atan's fourth derivative is at most 4.7,
+            // and a slope differs from the middle point's by at most h / kappa.
+            const double lines = xc ? (g.ny + 127) / 128 * 128 : (g.nx + 30) / 31 * 31;
+            const double cells = xc ? (g.nx + 30) / 31 * 31 : (g.ny + 127) / 128 * 128;
+            const double D = q.perp < 0 ? -q.perp : q.perp - lines;
+            const double h = kap * 9 / D * (xc ? std::max(std::fabs(q.par), std::fabs(cells - q.par)) / D : 1.0);
+            q.cubic = D > 0 && 4.7 / 24 * std::fabs(tB) * h * h * h * h < 0.25 && std::isfinite(tB * q.par);
+            q.pad[0] = q.pad[1] = 0;
             vcs[v] = make_double2(c, s);
             vx[v] = xc;
             if (xc) nxv++;
@@ -1447,6 +1525,7 @@ int fan_build_geometry(rn_fan_plan* p, const float* host_deg, FanGeoHost& gh) {
             if (vx[v]) perm[gs.view_off + a++] = k;
             else perm[gs.view_off + b++] = k;
         }
+        for (int k = 0; k < gs.nview; k++) gh.views_s.push_back(vg[gs.view_off + perm[gs.view_off + k]]);
     }
     if (std::fabs(nu * du / 2.0) >= M_PI / 4)
         return set_error(RN_ERR_ARG, "fan geometry: fan half-angle must be below 45 degrees");
@@ -1636,19 +1715,19 @@ int fan_backproject(rn_fan_plan* p, float* d_img, const float* d_prj, int type, 
         {
             LaunchScope ls2(p, st, 2);
             if (siddon)
-                siddon_table_kernel<<<tg, 256, 0, st>>>(d_prj, dbp, s0, ns, p->d_sets, p->d_views, p->d_cslopes, d,
+                siddon_table_kernel<<<tg, 256, 0, st>>>(d_prj, dbp, s0, ns, p->d_sets, p->d_perm, p->d_views, p->d_cslopes, d,
                                                         p->d_tab, base);
             else if (pixel)
-                pd_table_kernel<<<tg, 256, 0, st>>>(d_prj, dbp, s0, ns, p->d_sets, p->d_views, p->d_cslopes, d,
+                pd_table_kernel<<<tg, 256, 0, st>>>(d_prj, dbp, s0, ns, p->d_sets, p->d_perm, p->d_views, p->d_cslopes, d,
                                                     p->d_tab, base);
             else
-                fan_table_kernel<<<tg, 256, table_smem_bytes(d.nu), st>>>(d_prj, dbp, s0, ns, p->d_sets, p->d_views,
+                fan_table_kernel<<<tg, 256, table_smem_bytes(d.nu), st>>>(d_prj, dbp, s0, ns, p->d_sets, p->d_perm, p->d_views,
                                                                           p->d_edges, p->d_cell, d, type, p->d_tab,
                                                                           base);
         }
         RN_CUDA_TRY(cudaGetLastError());
         BpParams bp;
-        bp.views = p->d_views;
+        bp.views = p->d_views_s;
         bp.sets = p->d_sets;
         bp.bps = dbp;
         bp.tab = p->d_tab;
@@ -1858,7 +1937,8 @@ extern "C" int rn_fan_project_noalloc(float* d_prj, const float* d_img, const fl
         q.rmax = (float)std::max(r0, r1);
         int nl = xc ? ny : nx;
         q.sigma = (float)((r1 > r0 ? 1.0 : -1.0) * ((nl / 2.0 - q.perp) > 0 ? 1.0 : -1.0));
-        q.pad[0] = q.pad[1] = q.pad[2] = 0;
+        q.cubic = 0;
+        q.pad[0] = q.pad[1] = 0;
         if (std::fabs(q.perp - nl / 2.0) <= nl / 2.0 + 1.0)
             return set_error(RN_ERR_ARG, "fan geometry: source inside the image footprint");
         vcs[v] = make_double2(c, s);

@@ -15,6 +15,7 @@ struct BpView {
     double pard, perpd;   // source coordinates (Siddon band positions)
     float par, perp, kappa, tA, tB, sigma;
     int xcls;
+    int inside;           // the window holds every entry that the tile's edge-index cubics can select
 };
 
 // V views per staged chunk.
@@ -87,6 +88,8 @@ __device__ __noinline__ void bp_prep(BpSharedT<V>* sh, const ViewGeo* src, int c
     const float X = (float)(X0 + cx * kCols), Y = (float)(Y0 + cy * kRows);
     const float l = xcls ? Y : X, q = xcls ? X : Y;
     float t = matched_t(vg, (q - (float)vg.par) / (l - (float)vg.perp));
+    float tmax = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, 1));
+    tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
     t = fminf(t, __shfl_xor_sync(0xffffffffu, t, 1));
     t = fminf(t, __shfl_xor_sync(0xffffffffu, t, 2));
     if (valid && corner == 0) {
@@ -94,6 +97,9 @@ __device__ __noinline__ void bp_prep(BpSharedT<V>* sh, const ViewGeo* src, int c
         const int lo = (int)floorf(t) + pad - back;
         sh->elo[slot][v] = max(0, min(lo, tabn - win));
         BpView& w = sh->vw[slot][v];
+        // (an index may be a quarter of a cell off, hence one entry of room each side)
+        w.inside = vg.cubic && back >= 1 && lo >= 0 && lo <= tabn - win && tmax < 1e6f &&
+                   (int)floorf(tmax) + pad + 1 < lo + win;
         w.pard = vg.par;
         w.perpd = vg.perp;
         w.par = (float)vg.par;

@@ -255,6 +255,7 @@ static int finish_plan(rn_fan_plan* p, const float* host_deg, cudaStream_t st) {
         dev.push_back(ArenaPart{reinterpret_cast<void**>(dst), std::max<size_t>(bytes, 16), nullptr, 0});
     };
     upload(&p->d_views, gh.views);
+    upload(&p->d_views_s, gh.views_s);
     upload(&p->d_cell, gh.cell);
     upload(&p->d_perm, gh.perm);
     upload(&p->d_sets, p->h_sets);

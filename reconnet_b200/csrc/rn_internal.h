@@ -51,7 +51,8 @@ struct ViewGeo {
     float rmin, rmax;   // slope range covered by the detector
     float sigma;        // +-1: do edge indices increase along the line?
     int xcls;           // 1 = X-class
-    int pad[3];         // 64-byte records: chunks of them are bulk-copyable
+    int cubic;            // t_cubic is good to a quarter of a cell over every tile of the image
+    int pad[2];         // 64-byte records: chunks of them are bulk-copyable
 };
 static_assert(sizeof(ViewGeo) == 64, "ViewGeo is staged by 16-byte bulk copies");
 
@@ -130,6 +131,7 @@ struct rn_fan_plan {
 
     // device tables
     rn::ViewGeo* d_views = nullptr;
+    rn::ViewGeo* d_views_s = nullptr;   // the same in class-sorted order (perm)
     double* d_edges = nullptr;      // [total_views][nu+1] slopes
     float2* d_cell = nullptr;       // [nu] (cos a_u, sin a_u)
     int* d_perm = nullptr;          // [total_views] class-sorted view order per set
@@ -214,7 +216,7 @@ struct LaunchScope {
 // Host-side geometry tables of a fan plan, built by fan_build_geometry and
 // uploaded with the rest of the plan.
 struct FanGeoHost {
-    std::vector<ViewGeo> views;
+    std::vector<ViewGeo> views, views_s;   // and in class-sorted order
     std::vector<double2> vcs;       // per view (cos theta, sin theta)
     std::vector<int> vx;            // per view: 1 for the X class
     std::vector<int> perm;          // class-sorted view order per set
