@@ -13,7 +13,7 @@ namespace rn {
 // Per-view parameters the BP inner loop reads, staged in shared memory.
 struct BpView {
     double pard, perpd;   // source coordinates (Siddon band positions)
-    float par, perp, kappa, tA, tB, sigma;
+    float par, perp, kappa, tA, tB, sigma, round;
     int xcls;
     int inside;           // the window holds every entry that the tile's edge-index cubics can select
 };
@@ -98,7 +98,7 @@ __device__ __noinline__ void bp_prep(BpSharedT<V>* sh, const ViewGeo* src, int c
         sh->elo[slot][v] = max(0, min(lo, tabn - win));
         BpView& w = sh->vw[slot][v];
         // (an index may be a quarter of a cell off, hence one entry of room each side)
-        w.inside = vg.cubic && back >= 1 && lo >= 0 && lo <= tabn - win && tmax < 1e6f &&
+        w.inside = vg.cubic && back >= 1 && lo >= 0 && lo < tabn - win && tmax < 1e6f &&
                    (int)floorf(tmax) + pad + 1 < lo + win;
         w.pard = vg.par;
         w.perpd = vg.perp;
@@ -108,6 +108,7 @@ __device__ __noinline__ void bp_prep(BpSharedT<V>* sh, const ViewGeo* src, int c
         w.tA = vg.tA;
         w.tB = vg.tB;
         w.sigma = vg.sigma;
+        w.round = vg.round;
         w.xcls = vg.xcls;
     }
 }

@@ -52,7 +52,8 @@ struct ViewGeo {
     float sigma;        // +-1: do edge indices increase along the line?
     int xcls;           // 1 = X-class
     int cubic;            // t_cubic is good to a quarter of a cell over every tile of the image
-    int pad[2];         // 64-byte records: chunks of them are bulk-copyable
+    float round;          // rounds stepped coordinates (split_step)
+    int pad;         // 64-byte records: chunks of them are bulk-copyable
 };
 static_assert(sizeof(ViewGeo) == 64, "ViewGeo is staged by 16-byte bulk copies");
 
