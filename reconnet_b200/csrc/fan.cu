@@ -10,16 +10,17 @@
 // line arrays built here are exactly those blended rows.
 //
 // Design:
-//   * line prologue: one warp per line, FP64 prefix split into hi/lo floats
-//     (so prefix differences keep full precision), written once per call;
+//   * line prologue: FP64 prefix sums of every line, written once per call;
 //   * FP kernel: one CTA per (slice, view class, 4 views); lines are staged
 //     into shared memory in chunks with bulk async copies (cp.async.bulk +
 //     mbarrier, double buffered); each thread integrates whole rays across
 //     the staged lines; per-ray accumulators live in shared memory;
 //   * BP: edge tables (FP64 prefix of the weighted sinogram, hi/lo) built per
-//     call, then a gather-form kernel (no atomics): each thread owns a 4x4
-//     pixel block and accumulates all views in registers; per-view table
-//     windows are staged with bulk async copies.
+//     call, then a gather-form kernel (no atomics): each lane owns 16 pixels of
+//     a column and accumulates all views in registers; per-view table windows
+//     are staged with bulk async copies.  The matched backprojection's kernel
+//     is in fan_matched.cu, that of slices that share their views in
+//     fan_group.cu.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -54,7 +55,7 @@ constexpr int kFpMaxLines = 16;      // lines per staged chunk (upper bound)
 constexpr int kSmemBudget = 227 * 1024;
 
 
-constexpr int kBpViews = 8;          // views per staged chunk
+constexpr int kBpViews = kBpSplitViews;   // views per staged chunk
 using BpShared = BpSharedT<kBpViews>;
 
 __host__ __device__ inline long long align4(long long v) { return (v + 3) & ~3ll; }
@@ -866,102 +867,6 @@ __global__ void pd_table_kernel(const float* __restrict__ prj, const BpSlice* __
     }
 }
 
-// Matched backprojection: lane i of a warp owns pixel column x = X0 + i and
-// kBmRows pixel rows from y0; lane 31 owns no pixel and only supplies the
-// right edge of lane 30's column.  The staged table window T starts at table
-// index ilo; entries carry the prefix (hi, lo), the slope scaled by sigma / 2
-// and the edge slope r_e.
-// Two neighbouring lattice points of a lane: their edge indices are packed FP32
-// arithmetic (one instruction for both), the table entries and the values H =
-// hi + rest = prefix + (lo + slope * (r - r_e)) of the cells that contain the
-// slopes are not.  kFast: the staged window holds every entry the tile touches
-// (BpView::inside), so the index needs no clamp; `tbase` is then the byte
-// address of the entry of edge index 0 less the bias of the round-down add.
-struct HPair {
-    float hi[2], rest[2];
-};
-// The slopes are a * b (+ 0): a * b - r_e and a * b - r_t are each rounded once.
-template <bool kFast>
-__device__ __forceinline__ HPair bp_h2(const TCubic& c, f32x2 a, f32x2 b, f32x2 nrt, const float4* T, uint32_t tbase,
-                                       int ilo, int imax) {
-    const f32x2 h = f2_fma(a, b, nrt);
-    const f32x2 t = f2_fma(h, f2_fma(h, f2_fma(h, f2_pack(c.c3, c.c3), f2_pack(c.c2, c.c2)), f2_pack(c.c1, c.c1)),
-                           f2_pack(c.c0, c.c0));
-    const float2 tt = f2_unpack(t), aa = f2_unpack(a), bb = f2_unpack(b);
-    HPair o;
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const float tk = k ? tt.y : tt.x, ak = k ? aa.y : aa.x, bk = k ? bb.y : bb.x;
-        // table index floor(t) + 1 for |t| < 2^22 via a round-down add; beyond
-        // the detector it reaches a zero-slope guard entry
-        const int bits = __float_as_int(__fadd_rd(tk, 12582912.0f));
-        float4 E;
-        if (kFast) {
-            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(E.x), "=f"(E.y), "=f"(E.z), "=f"(E.w)
-                         : "r"(tbase + (uint32_t)bits * 16u));
-        } else {
-            E = T[min(max(bits - (0x4B400000 - 1), ilo), imax) - ilo];
-        }
-        o.hi[k] = E.x;
-        o.rest[k] = fmaf(E.z, fmaf(ak, bk, -E.w), E.y);
-    }
-    return o;
-}
-
-// X-class view (lattice lines are rows): the lane's lattice column q = x, lines
-// y0 .. y0 + kBmRows.  Line j's footprint difference with the next lane's column
-// goes to line[j]; a pixel is the sum of its two lines' totals, formed once
-// after all views.
-template <bool kFast>
-__device__ __forceinline__ void bp_matched_x(float (&line)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
-                                             int imax, int x, int y0) {
-    const float A = (float)x - vg.par;
-    // (approximate reciprocals: a relative error in 1 / (l - perp) scales all
-    // slopes of a line alike)
-    const TCubic c = t_cubic(vg, A * __fdividef(1.0f, (float)(y0 + kBmRows / 2) - vg.perp));
-    const uint32_t tbase = smem_u32(T) + (uint32_t)(1 - ilo - 0x4B400000) * 16u;
-    const f32x2 nrt = f2_pack(-c.rt, -c.rt), A2 = f2_pack(A, A);
-    const f32x2 y2 = f2_pack((float)y0, (float)y0), nperp2 = f2_pack(-vg.perp, -vg.perp);
-#pragma unroll
-    for (int j = 0; j <= kBmRows; j += 2) {
-        // (y0 + j is exact: one rounding per line, the same for its points)
-        const float2 D = f2_unpack(f2_add(f2_add(y2, f2_pack((float)j, (float)min(j + 1, kBmRows))), nperp2));
-        const f32x2 g = f2_pack(__fdividef(1.0f, D.x), __fdividef(1.0f, D.y));
-        const HPair H = bp_h2<kFast>(c, A2, g, nrt, T, tbase, ilo, imax);
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            if (j + k > kBmRows) break;
-            const float nhi = __shfl_down_sync(0xffffffffu, H.hi[k], 1);
-            const float nrest = __shfl_down_sync(0xffffffffu, H.rest[k], 1);
-            line[j + k] += (nhi - H.hi[k]) + (nrest - H.rest[k]);
-        }
-    }
-}
-
-// Y-class view (lattice lines are columns): the lane's line l = x, lattice
-// points q = y0 .. y0 + kBmRows.  The differences along line x go to line[j];
-// pixel (x, y) is its own and the next lane's, formed once after all views.
-template <bool kFast>
-__device__ __forceinline__ void bp_matched_y(float (&line)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
-                                             int imax, int x, int y0) {
-    const float g = __fdividef(1.0f, (float)x - vg.perp);
-    const float r0 = ((float)y0 - vg.par) * g;
-    const TCubic c = t_cubic(vg, fmaf((float)(kBmRows / 2), g, r0));
-    const uint32_t tbase = smem_u32(T) + (uint32_t)(1 - ilo - 0x4B400000) * 16u;
-    const f32x2 nrt = f2_pack(-c.rt, -c.rt), g2 = f2_pack(g, g), r02 = f2_pack(r0, r0);
-    float hp = 0.f, rp = 0.f;
-#pragma unroll
-    for (int j = 0; j <= kBmRows; j += 2) {
-        const HPair H = bp_h2<kFast>(c, f2_fma(f2_pack((float)j, (float)min(j + 1, kBmRows)), g2, r02), f2_pack(1.f, 1.f),
-                                     nrt, T, tbase, ilo, imax);
-        if (j > 0) line[j - 1] += (H.hi[0] - hp) + (H.rest[0] - rp);
-        if (j < kBmRows) line[j] += (H.hi[1] - H.hi[0]) + (H.rest[1] - H.rest[0]);
-        hp = H.hi[1];
-        rp = H.rest[1];
-    }
-}
-
 // Siddon backprojection (kMode 2), the exact transpose of the Siddon forward
 // projection: pixel column q-range [q, q + 1] on the band between lattice
 // lines l and l + 1 receives, from every ray u, c_u (its sinogram value times
@@ -1001,12 +906,6 @@ __device__ __forceinline__ void split_step(double v, float round, float& h, floa
 // (BpView::inside): no index is clamped, and both entries of the usual case are
 // read at one address.  `tbase` is the byte address of table entry 0 less the
 // bias of the directed adds.
-__device__ __forceinline__ float4 lds4(uint32_t a) {
-    float4 v;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
-    return v;
-}
-
 // (siddon_F called out of line for both: 8.3 ms for 8 slices of 512 x 512 with
 // 576-1152 views, 6.6 so.)
 
@@ -1078,7 +977,7 @@ __device__ __noinline__ void siddon_F(const float4* T, int ilo, int imax, int nu
 }
 
 template <bool kInside>
-__device__ __forceinline__ void bp_siddon_x(float (&acc)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
+__device__ __forceinline__ void bp_siddon_x(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
                                             int imax, int x, int y0, int nu) {
     const float A = (float)x - vg.par, D0 = (float)y0 - vg.perp;
     const TCubic c = t_cubic(vg, A * __fdividef(1.0f, D0 + (float)(kBmRows / 2)));
@@ -1106,7 +1005,7 @@ __device__ __forceinline__ void bp_siddon_x(float (&acc)[kBmRows + 1], const BpV
 }
 
 template <bool kInside>
-__device__ __forceinline__ void bp_siddon_y(float (&acc)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
+__device__ __forceinline__ void bp_siddon_y(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
                                             int imax, int x, int y0, int nu) {
     const float g = __fdividef(1.0f, (float)x - vg.perp);
     const float r0 = ((float)y0 - vg.par) * g;
@@ -1155,7 +1054,7 @@ __device__ __forceinline__ void ref_u(float t, const float4* T, int ilo, int ima
     rest = fmaf(fr, E.z, E.y);
 }
 
-__device__ __forceinline__ void bp_ref_x(float (&acc)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
+__device__ __forceinline__ void bp_ref_x(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
                                          int imax, int x, int y0, int nu, bool fbp, float dq, float dl, float dso2) {
     const float A = (float)x - vg.par;
     const TCubic c = t_cubic(vg, A * __fdividef(1.0f, (float)(y0 + kBmRows / 2) - vg.perp));
@@ -1179,7 +1078,7 @@ __device__ __forceinline__ void bp_ref_x(float (&acc)[kBmRows + 1], const BpView
     }
 }
 
-__device__ __forceinline__ void bp_ref_y(float (&acc)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
+__device__ __forceinline__ void bp_ref_y(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
                                          int imax, int x, int y0, int nu, bool fbp, float dq, float dl, float dso2) {
     const float D = (float)x + 0.5f - vg.perp;
     const float g = __fdividef(1.0f, D);
@@ -1239,7 +1138,7 @@ __device__ __forceinline__ float pd_sample(const float4* T, int ilo, int imax, f
 
 
 // X-class view: lane column q = x, pixel rows y0 + j (centres l = y0 + j + 1/2).
-__device__ __forceinline__ void bp_pixel_x(float (&acc)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
+__device__ __forceinline__ void bp_pixel_x(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
                                            int imax, int x, int y0, float dq, float dl) {
     const float A = (float)x + 0.5f - vg.par;
     const TCubic c = t_cubic(vg, A * __fdividef(1.0f, (float)(y0 + kBmRows / 2) - vg.perp));
@@ -1258,7 +1157,7 @@ __device__ __forceinline__ void bp_pixel_x(float (&acc)[kBmRows + 1], const BpVi
 }
 
 // Y-class view: lane line l = x (centre x + 1/2), positions q = y0 + j + 1/2.
-__device__ __forceinline__ void bp_pixel_y(float (&acc)[kBmRows + 1], const BpView& vg, const float4* T, int ilo,
+__device__ __forceinline__ void bp_pixel_y(float (&acc)[kBmRows], const BpView& vg, const float4* T, int ilo,
                                            int imax, int x, int y0, float dq, float dl) {
     const float g = __fdividef(1.0f, (float)x + 0.5f - vg.perp);
     const float r0 = ((float)y0 + 0.5f - vg.par) * g;
@@ -1277,7 +1176,7 @@ __device__ __forceinline__ void bp_pixel_y(float (&acc)[kBmRows + 1], const BpVi
     }
 }
 
-// kMode: 0 reference-mode (typeProjector 0 / 1), 1 matched, 2 Siddon, 3 pixel-driven.
+// kMode: 0 reference-mode (typeProjector 0 / 1), 2 Siddon, 3 pixel-driven (matched: fan_matched.cu).
 // Siddon tiles run three CTAs per SM (80 registers, 180 vs 174 Gupd/s at two
 // CTAs); the DD modes keep the compiler's register choice (71 / 80).
 template <int kMode>
@@ -1326,7 +1225,7 @@ __global__ void __launch_bounds__(kBpThreads, kMode == 3 ? 0 : 3) fan_bp_kernel(
     const int nchunks = (gs.nview + kBpViews - 1) / kBpViews;
     auto prep = [&](int c, const ViewGeo* src) {
         // table index = edge / cell index + 1
-        bp_prep<kBpViews, kBmCols, kBmTileY>(sh, src, c, gs.nview, X0, Y0, tabn, p.win, 1, 2);
+        bp_prep<kBpViews, kBmCols, kBmTileY, kMode == 2 ? 3 : 0>(sh, src, c, gs.nview, X0, Y0, tabn, p.win, 1, 2);
     };
     // tid 0: stage chunk c's table windows into buffer c & 1 and the view
     // records of chunk c + 1 into record slot (c + 1) & 1, on barrier c & 1.
@@ -1351,21 +1250,10 @@ __global__ void __launch_bounds__(kBpThreads, kMode == 3 ? 0 : 3) fan_bp_kernel(
     __syncthreads();
     if (tid == 0) issue(0);
 
-    // accumulators: acc[j] = pixel (x0, y0 + j); in matched mode line totals,
-    // first of the X-class views (line y0 + j), whose pixels go to `px` when
-    // the Y-class ones begin
-    float acc[kBmRows + 1], px[kBmRows];
+    // accumulators: acc[j] = pixel (x0, y0 + j)
+    float acc[kBmRows];
 #pragma unroll
-    for (int a = 0; a <= kBmRows; a++) acc[a] = 0.f;
-#pragma unroll
-    for (int a = 0; a < kBmRows; a++) px[a] = 0.f;
-    bool xphase = kMode == 1;
-    // an X-class line y0 + j counts for the pixels on both sides of it; line ny
-    // does not exist
-    auto x_pixels = [&]() {
-#pragma unroll
-        for (int a = 0; a < kBmRows; a++) px[a] = acc[a] + (y0 + a + 1 < ny ? acc[a + 1] : 0.f);
-    };
+    for (int a = 0; a < kBmRows; a++) acc[a] = 0.f;
 
     // One barrier per chunk: after it every warp has finished chunk c - 1, so
     // buffer (c + 1) & 1 and record slot c & 1 may be refilled; window and
@@ -1406,20 +1294,6 @@ __global__ void __launch_bounds__(kBpThreads, kMode == 3 ? 0 : 3) fan_bp_kernel(
                     if (vg.xcls) bp_siddon_x<false>(acc, vg, T, ilo, imax, x0, y0, nu);
                     else bp_siddon_y<false>(acc, vg, T, ilo, imax, x0, y0, nu);
                 }
-            } else if (kMode == 1) {
-                if (xphase && !vg.xcls) {   // once: views are sorted by class
-                    x_pixels();
-                    xphase = false;
-#pragma unroll
-                    for (int a = 0; a <= kBmRows; a++) acc[a] = 0.f;
-                }
-                if (vg.inside) {
-                    if (xphase) bp_matched_x<true>(acc, vg, T, ilo, imax, x0, y0);
-                    else bp_matched_y<true>(acc, vg, T, ilo, imax, x0, y0);
-                } else {
-                    if (xphase) bp_matched_x<false>(acc, vg, T, ilo, imax, x0, y0);
-                    else bp_matched_y<false>(acc, vg, T, ilo, imax, x0, y0);
-                }
             } else {
                 const bool fbp = p.type == RN_TYPE_FBP;
                 const float dso2 = p.d.dso * p.d.dso;
@@ -1429,21 +1303,6 @@ __global__ void __launch_bounds__(kBpThreads, kMode == 3 ? 0 : 3) fan_bp_kernel(
         }
     }
     if (!ok) return;
-    if (kMode == 1) {
-        if (xphase) {
-            x_pixels();
-#pragma unroll
-            for (int j = 0; j < kBmRows; j++) acc[j] = px[j];
-        } else {
-            // a Y-class line x counts for the pixels on both sides of it; line nx does not exist
-#pragma unroll
-            for (int j = 0; j < kBmRows; j++) {
-                const float next = __shfl_down_sync(0xffffffffu, acc[j], 1);
-                acc[j] = px[j] + (acc[j] + (x0 + 1 < nx ? next : 0.f));
-            }
-        }
-    }
-
     float* out = (p.nparts > 1 ? p.parts + part * p.part_stride : p.img) + bs.img_off;
     const bool add = p.nparts == 1 && p.accumulate;
     if (lane < kBmCols && x0 < nx) {
@@ -1504,12 +1363,12 @@ int fan_kernel_attributes() {
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_fp_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_fp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
-    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_lines_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_table_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     RN_TRY(fan_group_attributes());
+    RN_TRY(fan_matched_attributes());
     g_attr_done[dev] = 1;
     return RN_OK;
 }
@@ -1585,16 +1444,24 @@ int fan_build_geometry(rn_fan_plan* p, const float* host_deg, FanGeoHost& gh) {
             int nl = xc ? g.ny : g.nx;
             double side = (nl / 2.0 - q.perp) > 0 ? 1.0 : -1.0;
             q.sigma = (float)((r1 > r0 ? 1.0 : -1.0) * side);
-            // The edge-index cubic (t_cubic) over a lane's 17 lattice points, for
-            // any lane of the image's tiles (31 columns, 128 rows; the last ones
-            // reach past the image): atan's fourth derivative is at most 4.7,
-            // and a slope differs from the middle point's by at most h / kappa.
-            const double lines = xc ? (g.ny + 127) / 128 * 128 : (g.nx + 30) / 31 * 31;
-            const double cells = xc ? (g.nx + 30) / 31 * 31 : (g.ny + 127) / 128 * 128;
-            const double D = q.perp < 0 ? -q.perp : q.perp - lines;
-            const double h = kap * 9 / D * (xc ? std::max(std::fabs(q.par), std::fabs(cells - q.par)) / D : 1.0);
-            q.cubic = D > 0 && 4.7 / 24 * std::fabs(tB) * h * h * h * h < 0.25 && std::isfinite(tB * q.par);
-            q.pad = 0;
+            // Whether the polynomials that pick a lattice point's cell are good to
+            // a quarter of a cell for any lane of the image's tiles (the last ones
+            // reach past the image): t_cubic over a lane's 17 points (atan's
+            // fourth derivative is at most 4.7), and the matched
+            // backprojection's quartic over 32 lines x 32 points (its fifth is at
+            // most 24).  Slopes step by 1 / D along a line and by q / D^2 across.
+            auto reach = [&](int tw, int th, double along, double across) {   // |kappa (r - middle slope)|
+                const int px = (g.nx + tw - 1) / tw * tw, py = (g.ny + th - 1) / th * th;
+                const double lines = xc ? py : px, cells = xc ? px : py;
+                const double D = q.perp < 0 ? -q.perp : q.perp - lines;
+                const double far = std::max(std::fabs(q.par), std::fabs(cells - q.par)) / D;
+                const double h = kap * (along + across * far) / D;
+                return D > 0 && std::isfinite(tB * q.par * h) ? h : 1e9;
+            };
+            const double hc = xc ? reach(kBmCols, kBmTileY, 0, 9) : reach(kBmCols, kBmTileY, 9, 0);
+            const double hm = reach(kMatchedTile, kMatchedTile, 17, 17);
+            q.cubic = 4.7 / 24 * std::fabs(tB) * std::pow(hc, 4) < 0.25;
+            q.quartic = 24.0 / 120 * std::fabs(tB) * std::pow(hm, 5) < 0.25;
             // adding and subtracting this rounds a coordinate relative to the
             // source to a multiple of 2^-22 of the largest (or more)
             const double far = std::max(std::fabs(q.par), std::fabs(q.perp)) + std::max(g.nx, g.ny) + 256.0;
@@ -1844,7 +1711,7 @@ int fan_backproject(rn_fan_plan* p, float* d_img, const float* d_prj, int type, 
         LaunchScope ls3(p, st, 3);
         if (pixel) fan_bp_kernel<3><<<grid, kBpThreads, smem, st>>>(bp);
         else if (siddon) fan_bp_kernel<2><<<grid, kBpThreads, smem, st>>>(bp);
-        else if (type == RN_TYPE_MATCHED) fan_bp_kernel<1><<<grid, kBpThreads, smem, st>>>(bp);
+        else if (type == RN_TYPE_MATCHED) RN_TRY(fan_matched_launch(p, d_img, accumulate, s0, ns, base, bp.nparts, st));
         else fan_bp_kernel<0><<<grid, kBpThreads, smem, st>>>(bp);
         RN_CUDA_TRY(cudaGetLastError());
         RN_TRY(sum_parts(bp.nparts));
@@ -2025,9 +1892,8 @@ extern "C" int rn_fan_project_noalloc(float* d_prj, const float* d_img, const fl
         q.rmax = (float)std::max(r0, r1);
         int nl = xc ? ny : nx;
         q.sigma = (float)((r1 > r0 ? 1.0 : -1.0) * ((nl / 2.0 - q.perp) > 0 ? 1.0 : -1.0));
-        q.cubic = 0;
+        q.cubic = q.quartic = 0;
         q.round = 0.f;
-        q.pad = 0;
         if (std::fabs(q.perp - nl / 2.0) <= nl / 2.0 + 1.0)
             return set_error(RN_ERR_ARG, "fan geometry: source inside the image footprint");
         vcs[v] = make_double2(c, s);

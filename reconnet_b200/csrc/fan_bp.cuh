@@ -74,10 +74,11 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
 // of kCols x kRows pixels at (X0, Y0): lane = view * 4 + tile corner evaluates
 // the edge index at its corner, a 4-lane min gives the first staged table entry
 // (edge 0 is entry `pad`; `back` entries of slack before it), and the
-// view's parameters go to slot c % 3.  Kept out of line: it runs once per
+// view's parameters go to slot c % 3.  kPoly 3 or 4: also whether the window holds
+// every entry that a cubic (quartic) index of the tile can select.  Kept out of line: it runs once per
 // chunk in one warp, and inlined its temporaries would raise the register
 // count of the whole accumulation loop.
-template <int V, int kCols, int kRows>
+template <int V, int kCols, int kRows, int kPoly = 0>
 __device__ __noinline__ void bp_prep(BpSharedT<V>* sh, const ViewGeo* src, int c, int nview, int X0, int Y0,
                                      int tabn, int win, int pad, int back) {
     const int lane = threadIdx.x & 31, v = lane >> 2, corner = lane & 3;
@@ -88,8 +89,11 @@ __device__ __noinline__ void bp_prep(BpSharedT<V>* sh, const ViewGeo* src, int c
     const float X = (float)(X0 + cx * kCols), Y = (float)(Y0 + cy * kRows);
     const float l = xcls ? Y : X, q = xcls ? X : Y;
     float t = matched_t(vg, (q - (float)vg.par) / (l - (float)vg.perp));
-    float tmax = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, 1));
-    tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
+    float tmax = t;
+    if (kPoly) {
+        tmax = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, 1));
+        tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
+    }
     t = fminf(t, __shfl_xor_sync(0xffffffffu, t, 1));
     t = fminf(t, __shfl_xor_sync(0xffffffffu, t, 2));
     if (valid && corner == 0) {
@@ -98,8 +102,9 @@ __device__ __noinline__ void bp_prep(BpSharedT<V>* sh, const ViewGeo* src, int c
         sh->elo[slot][v] = max(0, min(lo, tabn - win));
         BpView& w = sh->vw[slot][v];
         // (an index may be a quarter of a cell off, hence one entry of room each side)
-        w.inside = vg.cubic && back >= 1 && lo >= 0 && lo < tabn - win && tmax < 1e6f &&
-                   (int)floorf(tmax) + pad + 1 < lo + win;
+        if (kPoly)
+            w.inside = (kPoly == 4 ? vg.quartic : vg.cubic) && back >= 1 && lo >= 0 && lo < tabn - win && tmax < 1e6f &&
+                       (int)floorf(tmax) + pad + 1 < lo + win;
         w.pard = vg.par;
         w.perpd = vg.perp;
         w.par = (float)vg.par;

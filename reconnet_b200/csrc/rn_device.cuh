@@ -110,6 +110,13 @@ __device__ __forceinline__ f32x2 f2_add_rd(f32x2 a, f32x2 b) {
     return r;
 }
 
+// shared-memory load at a byte address
+__device__ __forceinline__ float4 lds4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+
 // floor(x) and frac(x) for 0 <= x < 2^22 on the FMA/ALU pipes: the integer
 // part comes from rounding (x - 0.5) with a 1.5 * 2^23 bias.  At exact
 // integers it may return (n-1, 1.0) instead of (n, 0.0); both evaluate the

@@ -35,6 +35,9 @@ void clear_error();
 // returns early instead of hanging the GPU.
 constexpr long long kSpinLimit = 1ll << 22;
 
+constexpr int kBpSplitViews = 8;   // a backprojection's views are split in multiples of this
+constexpr int kMatchedTile = 62;   // pixels per side of a matched backprojection tile
+
 // ---------------------------------------------------------------------------
 // Geometry tables (device).
 // ---------------------------------------------------------------------------
@@ -53,7 +56,7 @@ struct ViewGeo {
     int xcls;           // 1 = X-class
     int cubic;            // t_cubic is good to a quarter of a cell over every tile of the image
     float round;          // rounds stepped coordinates (split_step)
-    int pad;         // 64-byte records: chunks of them are bulk-copyable
+    int quartic;          // the same for the matched backprojection's quartic and tiles         // 64-byte records: chunks of them are bulk-copyable
 };
 static_assert(sizeof(ViewGeo) == 64, "ViewGeo is staged by 16-byte bulk copies");
 
@@ -155,6 +158,7 @@ struct rn_fan_plan {
     float* d_la = nullptr;          // FP line values
     long long line_slot_elems = 0;  // per FP slice: ny*lpx + nx*lpy
     long long fp_slots = 0;         // FP slices whose lines fit in the scratch
+    int table_win_t = 0;            // the same for the matched backprojection's tiles
     int table_win_m = 0;            // staged table entries per view (BP tiles of 31 x 128 pixels)
     float4* d_tab = nullptr;        // BP edge tables
     long long tab_elems = 0;
@@ -234,6 +238,10 @@ int fan_slope_tables(rn_fan_plan* p, const double2* d_vcs, const int* d_vx, cons
 // Parts over which fan_backproject splits a backprojection of `type` (1 when
 // it does not split), and the number of slices in its first launch.
 int fan_bp_split(const rn_fan_plan* p, int type, int* first_wave_slices);
+// Matched backprojection of slices whose tables are built (fan_matched.cu).
+int fan_matched_attributes();
+int fan_matched_launch(rn_fan_plan* p, float* d_img, int accumulate, int s0, int ns, long long table_base, int nparts,
+                       cudaStream_t st);
 // Backprojection of slices that share their views (fan_group.cu): whether it
 // takes a launch of `ns` slices, its kernels' attributes, and the launch of
 // slices s0 .. s0 + ns - 1 (`nparts` partial images to sum where above 1).
