@@ -127,7 +127,8 @@ __global__ void cyl_zprefix_kernel(float* __restrict__ zp, const float* __restri
 // instructions or bytes.  NC = 0 (rows that reach further): every edge reads
 // every column.  512 x 512 x 128 voxels, 736 x 64 cells, 123 views: 6.41 ms with
 // every edge reading every column, 6.45 with summed columns one plane at a time,
-// 4.72 with two.
+// 4.72 with two, 3.37 with a plane's first entry and byte offsets worked out in
+// its record instead of by every lane.
 template <int NC>
 __global__ void __launch_bounds__(32 * kCylFpWarps, NC ? 3 : 0) cyl_fp_kernel(float* __restrict__ prj,
                                                                  const float* __restrict__ zp,
@@ -137,8 +138,10 @@ __global__ void __launch_bounds__(32 * kCylFpWarps, NC ? 3 : 0) cyl_fp_kernel(fl
                                                                  const float* __restrict__ sedge,
                                                                  const float* __restrict__ rowlen, CylDims d,
                                                                  int zlo, int nbz) {
-    // per plane: overlaps of the first two voxel columns, |D|, weight; the two
-    // columns, the top edge's sum, how many columns; the last overlap and column
+    // per plane: overlaps of the first two voxel columns, |D|, weight; byte
+    // offsets of the lowest height the rows reach in the two columns, the top
+    // edge's sum, how many columns; the last overlap, that height as an entry and
+    // the offset of heights from it
     __shared__ __align__(16) float4 s_plane[kCylFpWarps][NC ? 32 : 1][3];
     __shared__ float s_sum[kCylFpWarps][2][2][32 * (NC ? NC : 1)];   // [parity][plane of the pair]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -235,12 +238,18 @@ __global__ void __launch_bounds__(32 * kCylFpWarps, NC ? 3 : 0) cyl_fp_kernel(fl
                 auto overlap = [&](int i) { return (i == l_hi ? l_fhi : 1.f) - (i == l_lo ? l_flo : 0.f); };
                 __syncwarp();   // the previous planes have been read
                 s_plane[warp][lane][0] = make_float4(n > 0 ? overlap(i0) : 0.f, n > 1 ? overlap(i0 + 1) : 0.f, l_aD, l_w);
-                s_plane[warp][lane][1] = make_float4(__int_as_float(col), __int_as_float(n > 1 ? col + cs : col), l_top,
-                                                     __int_as_float(n));
-                s_plane[warp][lane][2] = make_float4(overlap(i0 + n - 1), 0.f, 0.f, 0.f);
+                // the cell below the lowest height the warp's rows reach (one
+                // lower: an edge that rounds down must not leave the window)
+                const float yb = __fadd_rd(fmaxf(fmaf(szb, l_aD, zoffb) - 1.f, 0.f), kCylFloorBias);
+                const int m0 = __float_as_int(yb) - kCylFloorBiasBits;
+                const unsigned first = ((unsigned)col * (unsigned)nbz) * 4u;
+                s_plane[warp][lane][1] = make_float4(__uint_as_float(first), __uint_as_float(n > 1 ? first + cs * nbz * 4u : first),
+                                                     l_top, __int_as_float(n));
+                s_plane[warp][lane][2] = make_float4(overlap(i0 + n - 1), __int_as_float(m0), zoffb - (yb - kCylFloorBias), 0.f);
                 const unsigned live = __ballot_sync(0xffffffffu, n > 0);
                 __syncwarp();
                 // two planes at a time: their loads and chains overlap
+                auto at = [&](unsigned o) { return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(zb) + o)); };
                 for (unsigned todo = live; todo;) {
                     const int j0 = __ffs(todo) - 1;
                     todo &= todo - 1;
@@ -251,31 +260,25 @@ __global__ void __launch_bounds__(32 * kCylFpWarps, NC ? 3 : 0) cyl_fp_kernel(fl
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         const int j = h ? j1 : j0;
-                        const float4 P = s_plane[warp][j][0], C = s_plane[warp][j][1];
-                        const float* c0 = zb + (long long)__float_as_int(C.x) * nbz;
-                        const float* c1 = zb + (long long)__float_as_int(C.y) * nbz;
+                        const float4 P = s_plane[warp][j][0], C = s_plane[warp][j][1], E = s_plane[warp][j][2];
                         aD[h] = P.z;
                         wgt[h] = h && !two ? 0.f : P.w;
                         top[h] = C.z;
-                        // the cell below the lowest height the warp's rows reach (one
-                        // lower: an edge that rounds down must not leave the window)
-                        const float yb = __fadd_rd(fmaxf(fmaf(szb, aD[h], zoffb) - 1.f, 0.f), kCylFloorBias);
-                        const int m0 = __float_as_int(yb) - kCylFloorBiasBits + lane;
-                        zrel[h] = zoffb - (yb - kCylFloorBias);
+                        zrel[h] = E.z;
+                        const int m0 = __float_as_int(E.y) + lane;
+                        unsigned o[NC ? NC : 1];
 #pragma unroll
                         for (int q = 0; q < NC; q++) {
-                            const int i = min(m0 + 32 * q, nbz - 1);
-                            g[h][q] = fmaf(P.y, __ldg(c1 + i), P.x * __ldg(c0 + i));
+                            o[q] = (unsigned)min(m0 + 32 * q, nbz - 1) * 4u;
+                            g[h][q] = fmaf(P.y, at(__float_as_uint(C.y) + o[q]), P.x * at(__float_as_uint(C.x) + o[q]));
                         }
                         const int nc = __float_as_int(C.w);
                         if (nc > 2) {   // wide footprints
-                            const float wl = s_plane[warp][j][2].x;
-                            const float* c = c1;
+                            unsigned c = __float_as_uint(C.y);
                             for (int t = 2; t < nc; t++) {
-                                c += cstride;
+                                c += (unsigned)cstride * 4u;
 #pragma unroll
-                                for (int q = 0; q < NC; q++)
-                                    g[h][q] = fmaf(t == nc - 1 ? wl : 1.f, __ldg(c + min(m0 + 32 * q, nbz - 1)), g[h][q]);
+                                for (int q = 0; q < NC; q++) g[h][q] = fmaf(t == nc - 1 ? E.x : 1.f, at(c + o[q]), g[h][q]);
                             }
                         }
                     }
@@ -767,8 +770,10 @@ extern "C" int rn_cyl_project(rn_cyl_plan* p, float* d_prj, const float* d_vol, 
         kern<<<grid, 32 * kCylFpWarps, 0, st>>>(d_prj, p->d_zp, p->d_views, p->d_redge, p->d_inplane, p->d_sedge,
                                                 p->d_rowlen, d, p->zlo, p->nbz);
     };
-    if (p->fp_span + 5 <= 64) launch(cyl_fp_kernel<2>);
-    else if (p->fp_span + 5 <= 96) launch(cyl_fp_kernel<3>);
+    // (and the band of one batch is addressed with 32-bit byte offsets)
+    const bool small = (long long)d.nx * d.ny * p->nbz < (1ll << 30);
+    if (small && p->fp_span + 5 <= 64) launch(cyl_fp_kernel<2>);
+    else if (small && p->fp_span + 5 <= 96) launch(cyl_fp_kernel<3>);
     else launch(cyl_fp_kernel<0>);
     p->launches++;
     RN_CUDA_TRY(cudaGetLastError());
