@@ -99,7 +99,7 @@ __global__ void edge_slope_kernel(double* edges, const double2* view_cs, const i
 // consecutive ones.  Where that makes too few blocks to fill the chip (or a
 // block's lines do not fit in shared memory) a CTA takes 8 lines, one per warp,
 // straight from the image: one slice of 512 x 512 takes 12 us that way and 19
-// in blocks of 16, 16 slices 65 us against 44 in blocks.
+// in blocks of 16, 16 slices 65 us against 40 in blocks.
 constexpr int kLineBlock = 16;
 constexpr int kLineCols = kLineBlock + 1;
 static size_t lines_smem_bytes(int n) { return sizeof(float) * (size_t)n * kLineCols; }
@@ -187,21 +187,39 @@ __global__ void __launch_bounds__(256) fan_lines_kernel(const float* __restrict_
         return v;
     };
     if (tiled) {
-        // the tile's element i: X lines are neighbours in memory along the line
-        // index, Y lines along the position
-        const int total = n * kLineCols, lead = xl ? kLineCols : n;
-        const unsigned inv = (unsigned)((0x100000000ull + lead - 1) / lead);   // i / lead = umulhi(i, inv) for i lead < 2^32
-        for (int i0 = threadIdx.x; i0 < total; i0 += 16 * 256) {
-            float v[16];
+        // X lines are neighbours in memory along the line index (16 lanes per
+        // position), Y lines along the position; addresses step by constants
+        const float w0 = fs.img_w[0], w1 = fs.img_w[1];
+        const long long second = fs.img_off[1] - fs.img_off[0];
+        auto load = [&](const float* q) {
+            float v = w0 != 0.f ? w0 * __ldg(q) : 0.f;
+            if (w1 != 0.f) v = fmaf(w1, __ldg(q + second), v);
+            return v;
+        };
+        const float* base0 = img + fs.img_off[0] + (long long)l0 * across;
+        if (xl) {
+            const int lo = threadIdx.x & 15, hi = threadIdx.x >> 4;
+            const float* q = base0 + (long long)lo * across + (long long)hi * along;
+            const long long step = 16 * along;
+            for (int k0 = hi; k0 < n; k0 += 8 * 16, q += 8 * step) {
+                float v[8];
 #pragma unroll
-            for (int k = 0; k < 16; k++) {
-                const int i = i0 + 256 * k, hi = lead == 1 ? i : (int)__umulhi((unsigned)i, inv), lo = i - hi * lead;
-                const int l = l0 - 1 + (xl ? lo : hi), pos = xl ? hi : lo;
-                v[k] = i < total && l < nl ? pixel(pos, l) : 0.f;
+                for (int k = 0; k < 8; k++) v[k] = k0 + 16 * k < n && lo < cnt ? load(q + k * step) : 0.f;
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (k0 + 16 * k < n) s_tile[(k0 + 16 * k) * kLineCols + lo + 1] = v[k];
             }
+            for (int k = threadIdx.x; k < n; k += 256)   // the line before the first
+                s_tile[k * kLineCols] = l0 > 0 ? load(base0 + (long long)k * along - across) : 0.f;
+        } else {
+            for (int k = threadIdx.x; k < n; k += 256) {
+                const float* q = base0 + (long long)k * along - across;
+                float v[kLineCols];
 #pragma unroll
-            for (int k = 0; k < 16; k++)
-                if (i0 + 256 * k < total) s_tile[i0 + 256 * k] = v[k];
+                for (int c = 0; c < kLineCols; c++, q += across) v[c] = c <= cnt && (c > 0 || l0 > 0) ? load(q) : 0.f;
+#pragma unroll
+                for (int c = 0; c < kLineCols; c++) s_tile[c * n + k] = v[c];
+            }
         }
         __syncthreads();
     }
