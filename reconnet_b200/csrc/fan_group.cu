@@ -4,7 +4,7 @@
 //
 // fan.cu's kernels work out a pixel's detector coordinates for every slice
 // again: about 30 of their 40 instructions per pixel and view.  Here a block
-// takes kBgSlices slices at once.  The per-view table holds the slices'
+// takes four or eight slices at once.  The per-view table holds the slices'
 // sinogram values side by side (one float4 per detector cell), a pixel's cells
 // and their weights are worked out once, and each slice adds a few packed
 // multiply-adds:
@@ -15,13 +15,14 @@
 //   pixel driven: the two cells around the ray through the pixel centre
 //     (pd_sample in fan.cu has the derivation).
 // Tiles are 32 columns (31 in reference mode, whose last lane only supplies an
-// edge) x 64 rows: a warp's lanes are the columns, a lane holds kBgRows rows of
-// every slice.
+// edge) x 64 rows, or 32 rows with eight slices: a warp's lanes are the columns, a
+// lane holds 16 or 8 rows of every slice.
 //
-// Measured against fan.cu's kernels: 16 slices of 512 x 512, 701 views of 888
-// channels, pixel driven: 2.16 ms against 5.62 ms (tables 0.04 against 0.11 ms);
-// 12 slices of 301 x 333, 413 views of 611 channels, reference mode: 0.52 ms
-// against 0.93 ms.
+// Measured: 16 slices of 512 x 512, 701 views of 888 channels, pixel driven: 5.62
+// ms with fan.cu's kernel, 2.18 ms with four slices per block, 1.88 with eight
+// (tables 0.11 and 0.04 ms); 12 slices of 301 x 333, 413 views of 611 channels,
+// reference mode: 0.93, 0.52 and 0.53 ms (three quads fill two blocks of two by
+// three quarters).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -33,11 +34,11 @@
 
 namespace rn {
 
-constexpr int kBgSlices = 4;    // slices per block
+constexpr int kBgSlices = 4;    // slices per table entry (a quad); a block takes one or two quads
 constexpr int kBgViews = 4;     // views per staged chunk
 constexpr int kBgWarps = 4;
-constexpr int kBgRows = 16;     // rows per lane
-constexpr int kBgTileY = kBgWarps * kBgRows;
+__host__ __device__ constexpr int bg_rows(int quads) { return 16 / quads; }   // rows per lane
+__host__ __device__ constexpr int bg_tile_y(int quads) { return kBgWarps * bg_rows(quads); }
 constexpr int kBgPad = 4;       // zero cells on both sides of a table row: cell u at entry u + kBgPad
 constexpr int kBgSmem = 100 * 1024;   // at least two blocks per SM
 using BgShared = BpSharedT<kBgViews>;
@@ -132,23 +133,27 @@ __global__ void __launch_bounds__(256) fan_group_table_kernel(float4* __restrict
 
 __device__ __forceinline__ f32x2 f2_dup(float v) { return f2_pack(v, v); }
 
-// acc += sum_k w[k] T[i + k], the four slices of each entry in two pairs.
-template <int K>
-__device__ __forceinline__ void add_cells(f32x2 (&acc)[2], const float4* T, const float (&w)[K]) {
+// acc += sum_k w[k] T[i + k], the four slices of each entry in two pairs; the
+// second quad's window is `win` entries on.
+template <int K, int Q>
+__device__ __forceinline__ void add_cells(f32x2 (&acc)[2 * Q], const float4* T, int win, const float (&w)[K]) {
 #pragma unroll
     for (int k = 0; k < K; k++) {
-        const ulonglong2 E = *reinterpret_cast<const ulonglong2*>(T + k);
         const f32x2 ww = f2_dup(w[k]);
-        acc[0] = f2_fma(ww, E.x, acc[0]);
-        acc[1] = f2_fma(ww, E.y, acc[1]);
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const ulonglong2 E = *reinterpret_cast<const ulonglong2*>(T + k + q * win);
+            acc[2 * q] = f2_fma(ww, E.x, acc[2 * q]);
+            acc[2 * q + 1] = f2_fma(ww, E.y, acc[2 * q + 1]);
+        }
     }
 }
 
 // Reference mode: weights of the K cells under the interval between the
 // detector coordinates t0, t1 (cell edges at integers), times `scale`.
-template <int K>
-__device__ __forceinline__ void add_interval(f32x2 (&acc)[2], const float4* T, int ilo, int imax, float t0, float t1,
-                                             float scale) {
+template <int K, int Q>
+__device__ __forceinline__ void add_interval(f32x2 (&acc)[2 * Q], const float4* T, int win, int ilo, int imax, float t0,
+                                             float t1, float scale) {
     const float lo = fminf(t0, t1), width = fabsf(t1 - t0);
     const float y = __fadd_rd(lo, 12582912.0f);
     const float f = lo - (y - 12582912.0f);
@@ -164,18 +169,19 @@ __device__ __forceinline__ void add_interval(f32x2 (&acc)[2], const float4* T, i
         w[k] = o * iw;
     }
     w[K - 1] = (rest - o) * iw;
-    add_cells<K>(acc, T + (i - ilo), w);
+    add_cells<K, Q>(acc, T + (i - ilo), win, w);
 }
 
-// kMode 0: reference mode with K cells; 3: pixel driven (K = 2).
-template <int kMode, int K>
+// kMode 0: reference mode with K cells; 3: pixel driven (K = 2).  Q quads of
+// slices.
+template <int kMode, int K, int Q>
 __global__ void __launch_bounds__(32 * kBgWarps, 3) fan_bp_group_kernel(GroupParams p) {
-    constexpr int kCols = kMode == 3 ? 32 : 31;
+    constexpr int kCols = kMode == 3 ? 32 : 31, kRows = bg_rows(Q), kTileY = bg_tile_y(Q);
     extern __shared__ __align__(128) unsigned char smem[];
     BgShared* sh = reinterpret_cast<BgShared*>(smem);
     const size_t off = (sizeof(BgShared) + 127) & ~size_t(127);
-    float4* const buf0 = reinterpret_cast<float4*>(smem + off);                   // [2][kBgViews][win]
-    float2* const geo0 = reinterpret_cast<float2*>(buf0 + 2 * kBgViews * p.win);  // likewise
+    float4* const buf0 = reinterpret_cast<float4*>(smem + off);                   // [2][kBgViews][Q][win]
+    float2* const geo0 = reinterpret_cast<float2*>(buf0 + 2 * kBgViews * Q * p.win);   // [2][kBgViews][win]
     const int tiles = p.tiles_x * p.tiles_y;
     const int part = blockIdx.x % p.nparts, bid = blockIdx.x / p.nparts;
     const int grp = bid / tiles, ti = bid - grp * tiles;
@@ -184,11 +190,13 @@ __global__ void __launch_bounds__(32 * kBgWarps, 3) fan_bp_group_kernel(GroupPar
     const int nch_all = (p.nview + kBgViews - 1) / kBgViews, cpp = (nch_all + p.nparts - 1) / p.nparts;
     const int vbeg = min(p.nview, part * cpp * kBgViews), nview = min(p.nview, (part + 1) * cpp * kBgViews) - vbeg;
     const ViewGeo* views = p.views + p.view_off + vbeg;
-    const float4* gval = p.vals + ((long long)grp * p.nview + vbeg) * p.tabn;
+    // the block's first quad, and the distance to the second (0 where there is none: staged again, not stored)
+    const float4* gval = p.vals + ((long long)grp * Q * p.nview + vbeg) * p.tabn;
+    const long long second = grp * Q + 1 < (p.ns + kBgSlices - 1) / kBgSlices ? (long long)p.nview * p.tabn : 0;
     const float2* ggeo = p.geo + (long long)vbeg * p.tabn;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int X0 = txi * kCols, Y0 = tyi * kBgTileY;
-    const int x0 = X0 + lane, y0 = Y0 + warp * kBgRows;
+    const int X0 = txi * kCols, Y0 = tyi * kTileY;
+    const int x0 = X0 + lane, y0 = Y0 + warp * kRows;
     const int win = p.win;   // even, and at most tabn, so that every window starts on an even entry
     if (tid == 0) {
         mbar_init(&sh->bars[0], 1);
@@ -197,18 +205,21 @@ __global__ void __launch_bounds__(32 * kBgWarps, 3) fan_bp_group_kernel(GroupPar
     }
     const int nchunks = (nview + kBgViews - 1) / kBgViews;
     auto prep = [&](int c, const ViewGeo* src) {
-        bp_prep<kBgViews, kCols, kBgTileY>(sh, src, c, nview, X0, Y0, p.tabn, win, kBgPad, 3);
+        bp_prep<kBgViews, kCols, kTileY>(sh, src, c, nview, X0, Y0, p.tabn, win, kBgPad, 3);
     };
     auto issue = [&](int c) {
         const int b = c & 1;
         const int vc = min(kBgViews, nview - c * kBgViews);
         const int vn = c + 1 < nchunks ? min(kBgViews, nview - (c + 1) * kBgViews) : 0;
-        const uint32_t entry = sizeof(float4) + (kMode == 3 ? sizeof(float2) : 0);
+        const uint32_t entry = Q * sizeof(float4) + (kMode == 3 ? sizeof(float2) : 0);
         fence_proxy_async();
         mbar_arrive_expect_tx(&sh->bars[b], (uint32_t)(vc * win * entry + vn * sizeof(ViewGeo)));
         for (int v = 0; v < vc; v++) {
             const long long row = (long long)(c * kBgViews + v) * p.tabn + (sh->elo[c % 3][v] & ~1);
-            bulk_g2s(buf0 + (b * kBgViews + v) * win, gval + row, (uint32_t)(win * sizeof(float4)), &sh->bars[b]);
+#pragma unroll
+            for (int q = 0; q < Q; q++)
+                bulk_g2s(buf0 + ((b * kBgViews + v) * Q + q) * win, gval + q * second + row,
+                         (uint32_t)(win * sizeof(float4)), &sh->bars[b]);
             if (kMode == 3)
                 bulk_g2s(geo0 + (b * kBgViews + v) * win, ggeo + row, (uint32_t)(win * sizeof(float2)), &sh->bars[b]);
         }
@@ -220,9 +231,11 @@ __global__ void __launch_bounds__(32 * kBgWarps, 3) fan_bp_group_kernel(GroupPar
         __syncthreads();
         if (tid == 0) issue(0);
     }
-    f32x2 acc[kBgRows][2];
+    f32x2 acc[kRows][2 * Q];
 #pragma unroll
-    for (int j = 0; j < kBgRows; j++) acc[j][0] = acc[j][1] = 0ull;
+    for (int j = 0; j < kRows; j++)
+#pragma unroll
+        for (int q = 0; q < 2 * Q; q++) acc[j][q] = 0ull;
     const float dso2 = p.d.dso * p.d.dso;
     // one barrier per chunk, as in fan_bp_kernel
     bool ok = true;
@@ -244,7 +257,7 @@ __global__ void __launch_bounds__(32 * kBgWarps, 3) fan_bp_group_kernel(GroupPar
         const int slot = c % 3, vc = min(kBgViews, nview - c * kBgViews);
         for (int v = 0; v < vc; v++) {
             const BpView vg = sh->vw[slot][v];
-            const float4* T = buf0 + (b * kBgViews + v) * win;
+            const float4* T = buf0 + (b * kBgViews + v) * Q * win;
             const float2* G = geo0 + (b * kBgViews + v) * win;
             const int ilo = sh->elo[slot][v] & ~1, imax = ilo + win - 1;
             const bool xc = vg.xcls;
@@ -252,29 +265,29 @@ __global__ void __launch_bounds__(32 * kBgWarps, 3) fan_bp_group_kernel(GroupPar
             if (kMode == 0) {
                 if (xc) {
                     const float A = (float)x0 - vg.par, aq = (A + 0.5f) * dq;
-                    const TCubic cu = t_cubic(vg, A * __fdividef(1.0f, (float)(y0 + kBgRows / 2) - vg.perp));
+                    const TCubic cu = t_cubic(vg, A * __fdividef(1.0f, (float)(y0 + kRows / 2) - vg.perp));
 #pragma unroll
-                    for (int j = 0; j < kBgRows; j++) {
+                    for (int j = 0; j < kRows; j++) {
                         const float D = (float)(y0 + j) + 0.5f - vg.perp;
                         const float h = A * __fdividef(1.0f, D) - cu.rt;
                         const float t = fmaf(h, fmaf(h, fmaf(h, cu.c3, cu.c2), cu.c1), cu.c0);
                         const float nt = __shfl_down_sync(0xffffffffu, t, 1);
                         const float bl = D * dl;
-                        add_interval<K>(acc[j], T, ilo, imax, t, nt,
+                        add_interval<K, Q>(acc[j], T, win, ilo, imax, t, nt,
                                         p.fbp ? __fdividef(dso2, fmaf(aq, aq, bl * bl)) : 1.0f);
                     }
                 } else {
                     const float D = (float)x0 + 0.5f - vg.perp, g = __fdividef(1.0f, D), bl = D * dl;
                     const float r0 = ((float)y0 - vg.par) * g;
-                    const TCubic cu = t_cubic(vg, fmaf((float)(kBgRows / 2), g, r0));
+                    const TCubic cu = t_cubic(vg, fmaf((float)(kRows / 2), g, r0));
                     float tp = 0.f;
 #pragma unroll
-                    for (int j = 0; j <= kBgRows; j++) {
+                    for (int j = 0; j <= kRows; j++) {
                         const float h = fmaf((float)j, g, r0) - cu.rt;
                         const float t = fmaf(h, fmaf(h, fmaf(h, cu.c3, cu.c2), cu.c1), cu.c0);
                         if (j > 0) {
                             const float a = ((float)(y0 + j) - 0.5f - vg.par) * dq;
-                            add_interval<K>(acc[j - 1], T, ilo, imax, tp, t,
+                            add_interval<K, Q>(acc[j - 1], T, win, ilo, imax, tp, t,
                                             p.fbp ? __fdividef(dso2, fmaf(a, a, bl * bl)) : 1.0f);
                         }
                         tp = t;
@@ -288,11 +301,11 @@ __global__ void __launch_bounds__(32 * kBgWarps, 3) fan_bp_group_kernel(GroupPar
                 split_hilo(vg.pard - ((double)q0 + 0.5), Ah, Al);
                 split_hilo(((double)l0 + 0.5) - vg.perpd, Dh, Dl);
                 const float A = q0 + 0.5f - vg.par, g = __fdividef(1.0f, l0 + 0.5f - vg.perp);
-                const TCubic cu = t_cubic(vg, xc ? A * __fdividef(1.0f, l0 + (float)(kBgRows / 2) - vg.perp)
-                                                 : fmaf((float)(kBgRows / 2) - 0.5f, g, A * g));
+                const TCubic cu = t_cubic(vg, xc ? A * __fdividef(1.0f, l0 + (float)(kRows / 2) - vg.perp)
+                                                 : fmaf((float)(kRows / 2) - 0.5f, g, A * g));
                 const float cfrac = -vg.tB * dq * dl;
 #pragma unroll
-                for (int j = 0; j < kBgRows; j++) {
+                for (int j = 0; j < kRows; j++) {
                     float a_h = Ah, a_l = Al, d_h = Dh, d_l = Dl, e, r;
                     if (xc) {
                         r = A * __fdividef(1.0f, l0 + (float)j + 0.5f - vg.perp);
@@ -317,7 +330,7 @@ __global__ void __launch_bounds__(32 * kBgWarps, 3) fan_bp_group_kernel(GroupPar
                     const float wgt = (i < kBgPad && frac < 0.f) ? 0.f : dso2 * il2;
                     const float w1 = frac * wgt;
                     const float w[2] = {wgt - w1, w1};
-                    add_cells<2>(acc[j], T + (i - ilo), w);
+                    add_cells<2, Q>(acc[j], T + (i - ilo), win, w);
                 }
             }
         }
@@ -327,12 +340,12 @@ __global__ void __launch_bounds__(32 * kBgWarps, 3) fan_bp_group_kernel(GroupPar
         float* base = p.nparts > 1 ? p.parts + part * p.part_stride : p.img;
         const bool add = p.nparts == 1 && p.accumulate;
 #pragma unroll
-        for (int s = 0; s < kBgSlices; s++) {
-            const int si = grp * kBgSlices + s;
+        for (int s = 0; s < Q * kBgSlices; s++) {
+            const int si = grp * Q * kBgSlices + s;
             if (si >= p.ns) break;
             float* out = base + p.bps[p.s_begin + si].img_off + (long long)x0 * p.d.isx;
 #pragma unroll
-            for (int j = 0; j < kBgRows; j++) {
+            for (int j = 0; j < kRows; j++) {
                 const int iy = y0 + j;
                 if (iy < p.d.ny) {
                     const float2 a = f2_unpack(acc[j][s / 2]);
@@ -350,12 +363,12 @@ __global__ void __launch_bounds__(32 * kBgWarps, 3) fan_bp_group_kernel(GroupPar
 // ---------------------------------------------------------------------------
 static int group_tabn(const rn_fan_plan* p) { return (p->dims.nu + 2 * kBgPad + 1) & ~1; }
 
-// Staged entries per view: the detector extent of a 32 x 64 tile at the point
+// Staged entries per view: the detector extent of a tile at the point
 // closest to the source, with the cells before and after it; 0 where the
 // window does not fit.
-static int group_window(const rn_fan_plan* p) {
+static int group_window(const rn_fan_plan* p, int quads) {
     const RnFanGeom& g = p->g;
-    const double tw = 32 * (double)g.dx, th = kBgTileY * (double)g.dy;
+    const double tw = 32 * (double)g.dx, th = bg_tile_y(quads) * (double)g.dy;
     const double hx = g.nx * (double)g.dx / 2 + std::fabs(g.cx), hy = g.ny * (double)g.dy / 2 + std::fabs(g.cy);
     const double dmin = g.dso - std::sqrt(hx * hx + hy * hy);
     if (!(dmin > 0)) return 0;
@@ -364,8 +377,18 @@ static int group_window(const rn_fan_plan* p) {
     return std::min(((int)std::ceil(w) + 7) & ~7, group_tabn(p));
 }
 
-static size_t group_smem(int win) {
-    return ((sizeof(BgShared) + 127) & ~size_t(127)) + 2 * (size_t)kBgViews * win * (sizeof(float4) + sizeof(float2));
+static size_t group_smem(int win, int quads) {
+    return ((sizeof(BgShared) + 127) & ~size_t(127)) +
+           2 * (size_t)kBgViews * win * (quads * sizeof(float4) + sizeof(float2));
+}
+
+// Quads per block: two (a pixel's cells and weights cost about 45 instructions, a
+// quad about 8) where their windows fit and the quads fill the blocks, or nearly:
+// 12 slices in two blocks of two quads take as long as in three of one.
+static int group_quads(const rn_fan_plan* p, int ns) {
+    const int win = group_window(p, 2);
+    const int groups = (ns + kBgSlices - 1) / kBgSlices;
+    return (groups % 2 == 0 || groups >= 5) && win >= 8 && group_smem(win, 2) <= (size_t)kBgSmem ? 2 : 1;
 }
 
 // Most cells a pixel's interval can span in reference mode.
@@ -382,8 +405,8 @@ static double group_width(const rn_fan_plan* p) {
 bool fan_group_ok(const rn_fan_plan* p, int type, int ns) {
     if (p->ragged || ns < 3) return false;
     if (type != RN_TYPE_ITERATIVE && type != RN_TYPE_FBP && type != RN_TYPE_PIXEL) return false;
-    const int win = group_window(p);
-    if (win < 8 || group_smem(win) > (size_t)kBgSmem) return false;
+    const int win = group_window(p, 1);
+    if (win < 8 || group_smem(win, 1) > (size_t)kBgSmem) return false;
     if (type != RN_TYPE_PIXEL && !(group_width(p) <= 2.99)) return false;
     const long long rows = (long long)p->total_views * group_tabn(p);
     const long long groups = (ns + kBgSlices - 1) / kBgSlices;
@@ -392,16 +415,19 @@ bool fan_group_ok(const rn_fan_plan* p, int type, int ns) {
 
 int fan_group_attributes() {
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_group_kernel<0, 3>, attr, kBgSmem));
-    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_group_kernel<0, 4>, attr, kBgSmem));
-    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_group_kernel<3, 2>, attr, kBgSmem));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_group_kernel<0, 3, 1>, attr, kBgSmem));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_group_kernel<0, 3, 2>, attr, kBgSmem));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_group_kernel<0, 4, 1>, attr, kBgSmem));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_group_kernel<0, 4, 2>, attr, kBgSmem));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_group_kernel<3, 2, 1>, attr, kBgSmem));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_group_kernel<3, 2, 2>, attr, kBgSmem));
     return RN_OK;
 }
 
 int fan_group_backproject(rn_fan_plan* p, float* d_img, const float* d_prj, int type, int accumulate, int s0, int ns,
                           int* nparts, cudaStream_t st) {
     const FanDims& d = p->dims;
-    const int nview = (int)p->total_views, tabn = group_tabn(p), win = group_window(p);
+    const int quads = group_quads(p, ns), nview = (int)p->total_views, tabn = group_tabn(p), win = group_window(p, quads);
     const bool pixel = type == RN_TYPE_PIXEL;
     const int groups = (ns + kBgSlices - 1) / kBgSlices;
     float4* vals = p->d_tab;
@@ -431,11 +457,11 @@ int fan_group_backproject(rn_fan_plan* p, float* d_img, const float* d_prj, int 
     g.fbp = type == RN_TYPE_FBP;
     const int cols = pixel ? 32 : 31;
     g.tiles_x = (d.nx + cols - 1) / cols;
-    g.tiles_y = (d.ny + kBgTileY - 1) / kBgTileY;
+    g.tiles_y = (d.ny + bg_tile_y(quads) - 1) / bg_tile_y(quads);
     g.spin = p->spin_limit;
     // too few blocks to fill the GPU: split each tile's views (tuned, or
     // towards six blocks per SM), as far as the plan's scratch goes
-    const long long ctas = (long long)g.tiles_x * g.tiles_y * groups;
+    const long long ctas = (long long)g.tiles_x * g.tiles_y * ((groups + quads - 1) / quads);
     const int nch = (nview + kBgViews - 1) / kBgViews;
     long long want = 1;
     if (ns == (int)p->h_bpr.size() && p->bp_parts_cap > 0) {
@@ -447,11 +473,12 @@ int fan_group_backproject(rn_fan_plan* p, float* d_img, const float* d_prj, int 
     g.parts = p->d_bp_parts;
     *nparts = g.nparts;
     const unsigned grid = (unsigned)(ctas * g.nparts);
-    const size_t smem = group_smem(win);
+    const size_t smem = group_smem(win, quads);
     LaunchScope ls(p, st, 3);
-    if (pixel) fan_bp_group_kernel<3, 2><<<grid, 32 * kBgWarps, smem, st>>>(g);
-    else if (group_width(p) <= 1.99) fan_bp_group_kernel<0, 3><<<grid, 32 * kBgWarps, smem, st>>>(g);
-    else fan_bp_group_kernel<0, 4><<<grid, 32 * kBgWarps, smem, st>>>(g);
+    auto launch = [&](auto kern) { kern<<<grid, 32 * kBgWarps, smem, st>>>(g); };
+    if (pixel) quads == 2 ? launch(fan_bp_group_kernel<3, 2, 2>) : launch(fan_bp_group_kernel<3, 2, 1>);
+    else if (group_width(p) <= 1.99) quads == 2 ? launch(fan_bp_group_kernel<0, 3, 2>) : launch(fan_bp_group_kernel<0, 3, 1>);
+    else quads == 2 ? launch(fan_bp_group_kernel<0, 4, 2>) : launch(fan_bp_group_kernel<0, 4, 1>);
     RN_CUDA_TRY(cudaGetLastError());
     return RN_OK;
 }
