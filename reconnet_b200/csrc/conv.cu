@@ -195,18 +195,21 @@ struct ConvArgs {
     int* err;
 };
 
-// Warp-specialised pipeline.  Warp 5 loads: it keeps kConvStages TMA boxes in
+// Warp-specialised pipeline.  Warp 9 loads: it keeps kConvStages TMA boxes in
 // flight, refilling a stage when its "empty" barrier says that the MMAs on it are
-// done.  Warp 4 issues each tile's MMA group (one elected lane) and commits it
+// done.  Warp 8 issues each tile's MMA group (one elected lane) and commits it
 // twice, to the box's "empty" barrier and to the accumulator's "full" barrier.
-// Warps 0-3 are the epilogue: thread t reads TMEM lane t (output pixel w0 + t
-// of the tile's row) from one of two accumulators of 32 columns, releases the
-// accumulator (one arrival per warp on its "empty" barrier) and stores.  So
+// Warps 0-3 and 4-7 are the epilogues of the even and the odd tiles: thread t
+// reads TMEM lane t (output pixel w0 + t of the tile's row) from its accumulator
+// of 32 columns, releases the accumulator (one arrival per warp on its "empty"
+// barrier) and stores.  So
 // the TMA copies, the MMAs of tile i and the epilogue of tile i - 1 overlap.
-// A tile's issue is one warp's serial instruction stream, which bounds the
-// kernel: the descriptors are a base and constants, stages and phases are
-// counted, and loading has its own warp.  8 images of 512 x 512, 32 to 32
-// channels: 128 us with one lane loading and issuing from 64-bit indices, now 82.
+// What bounded it were serial instruction streams: a lane that loaded and issued
+// from 64-bit indices, then one warpgroup's epilogues.  8 images of 512 x 512, 32
+// to 32 channels: 128 us with both, 82 us with loads in their own warp and
+// descriptors as a base and constants, 66 us with a warpgroup per accumulator; a
+// tile's 18 MMAs read 128 x 16 operands from shared memory for 720 of its 1130
+// cycles on the SM.
 //
 // Boxes: the tensor map views each image row as groups of PIX pixels (16 PIX
 // bytes; PIX = 8 when the width allows, else 2, else 1), so a TMA row is a
@@ -214,7 +217,8 @@ struct ConvArgs {
 // PIX - 1 pixels before the halo pixel w0 - 1 (128 + 2 PIX pixels) and the
 // operands start 16 (PIX - 1) bytes into each box row.
 constexpr int kConvStages = 3;
-constexpr int kConvWsThreads = kConvThreads + 64;
+constexpr int kConvEpilogues = 2;   // epilogue warpgroups, one per accumulator
+constexpr int kConvWsThreads = kConvEpilogues * kConvThreads + 64;
 
 template <int CH, int NPAD, int PIX>
 __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_constant__ CUtensorMap tm_in, ConvArgs a) {
@@ -266,7 +270,7 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
 
     TileWalk walk(blockIdx.x, gridDim.x, tiles_w, a.H);   // the next box, or the epilogue's next tile
 
-    if (warp == kConvThreads / 32 + 1) {
+    if (warp == kConvEpilogues * kConvThreads / 32 + 1) {
         // ---- loads ----
         const bool leader = elect_one();
         int s = 0, phase = 1, i = 0;   // stage, parity of its previous use
@@ -290,7 +294,7 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
             // the copies in flight, before the shared memory is released
             for (int k = max(0, i - S); k < i; k++) mbar_wait(&bar_full[k % S], (uint32_t)((k / S) & 1));
         }
-    } else if (warp == kConvThreads / 32) {
+    } else if (warp == kConvEpilogues * kConvThreads / 32) {
         // ---- MMAs ----
         const bool leader = elect_one();
         constexpr uint32_t idesc = umma_idesc(NPAD, false, false), hi = desc_hi(128);
@@ -339,10 +343,12 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
             if (j > 0) mbar_wait(&bar_empty[(j - 1) % S], (uint32_t)(((j - 1) / S) & 1));
         }
     } else {
-        // ---- epilogue: thread tid owns output pixel w0 + tid ----
-        for (int j = 0; j < nmine; j++) {
-            const int acc = j & 1;
-            const int n = walk.n, h = walk.h, w = walk.tw * kConvTile + tid;
+        // ---- epilogue: thread t of the warpgroup owns output pixel w0 + t ----
+        const int acc = warp >> 2;   // tiles acc, acc + 2, ..
+        if (acc) walk.next();
+        for (int j = acc; j < nmine; j += kConvEpilogues) {
+            const int n = walk.n, h = walk.h, w = walk.tw * kConvTile + (tid & (kConvThreads - 1));
+            walk.next();
             walk.next();
             // the aux input is on its way while the MMAs are
             uint4 act[NPAD / 8];
@@ -362,7 +368,7 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
             }
             tc_fence_after();
             float v[32];
-            tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(acc * 32), v);
+            tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(acc * 32), v);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar_acce[acc]);
