@@ -793,6 +793,9 @@ struct rn_cone_plan {
 
 namespace {
 
+// *out stays null where the device has no room (a tomosynthesis plan then takes
+// the general kernels; an upright plan's table is a quarter of the ray table that
+// the general backprojection keeps).
 int scratch_get(rn_cone_plan* p, size_t bytes, cudaStream_t st, void** out) {
     {
         std::lock_guard<std::mutex> lk(p->pool_mu);
@@ -807,7 +810,13 @@ int scratch_get(rn_cone_plan* p, size_t bytes, cudaStream_t st, void** out) {
             RN_CUDA_TRY(cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep));
         }
     }
-    RN_CUDA_TRY(cudaMallocFromPoolAsync(out, bytes, p->pool, st));
+    const cudaError_t e = cudaMallocFromPoolAsync(out, bytes, p->pool, st);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        *out = nullptr;
+        return RN_OK;
+    }
+    RN_CUDA_TRY(e);
     return RN_OK;
 }
 
@@ -1048,10 +1057,12 @@ int rn_cone_project(rn_cone_plan* p, float* d_prj, const float* d_img, void* str
         cudaStream_t st = (cudaStream_t)stream;
         void* vol = nullptr;
         RN_TRY(scratch_get(p, cone_tile_fp_bytes(cd), st, &vol));
-        p->launches += 2LL * cd.nb * cd.nc;
-        const int s = cone_tile_project(p->d_tile, cd, p->tp, static_cast<float*>(vol), d_prj, d_img, st);
-        cudaFreeAsync(vol, st);
-        return s;
+        if (vol) {
+            p->launches += 2LL * cd.nb * cd.nc;
+            const int s = cone_tile_project(p->d_tile, cd, p->tp, static_cast<float*>(vol), d_prj, d_img, st);
+            cudaFreeAsync(vol, st);
+            return s;
+        }
     }
     const int gx = p->lanes_v ? (cd.nu + 7) / 8 : (cd.nu + 31) / 32;
     const int gy = p->lanes_v ? (cd.nv + 31) / 32 : (cd.nv + 7) / 8;
@@ -1080,6 +1091,7 @@ int rn_cone_backproject(rn_cone_plan* p, float* d_img, const float* d_prj, int a
         cudaStream_t st = (cudaStream_t)stream;
         void* tab = nullptr;
         RN_TRY(scratch_get(p, cone_col_table_bytes(cd), st, &tab));
+        if (!tab) return set_cuda_error(cudaErrorMemoryAllocation, "cone backprojection: prefix table");
         p->launches += 2LL * slices;
         const int s = cone_col_backproject(p->d_col, cd, p->col_one, static_cast<double*>(tab), d_img, d_prj,
                                            accumulate, st);
@@ -1090,10 +1102,14 @@ int rn_cone_backproject(rn_cone_plan* p, float* d_img, const float* d_prj, int a
         cudaStream_t st = (cudaStream_t)stream;
         void* wp = nullptr;
         RN_TRY(scratch_get(p, cone_tile_bp_bytes(cd), st, &wp));
-        p->launches += 2LL * slices;
-        const int s = cone_tile_backproject(p->d_tile, cd, p->tp, static_cast<float*>(wp), d_img, d_prj, accumulate, st);
-        cudaFreeAsync(wp, st);
-        return s;
+        if (!wp && !p->bp_sep) return set_cuda_error(cudaErrorMemoryAllocation, "cone backprojection: scratch");
+        if (wp) {
+            p->launches += 2LL * slices;
+            const int s =
+                cone_tile_backproject(p->d_tile, cd, p->tp, static_cast<float*>(wp), d_img, d_prj, accumulate, st);
+            cudaFreeAsync(wp, st);
+            return s;
+        }
     }
     if (p->bp_sep) {
         // one warp per 2 (U) x 32 (V) voxels at one m
