@@ -4,6 +4,8 @@
 #include <string.h>
 
 #include <algorithm>
+#include <functional>
+#include <map>
 #include <cmath>
 #include <mutex>
 #include <string>
@@ -76,24 +78,63 @@ static void set_dims(rn_fan_plan* p, long long isx, long long isy) {
     d.isy = isy;
 }
 
+// Time of the forward projection with VT views per work item, up to a factor: one
+// CTA per SM takes items from a list sorted by cost, longest first.  An item's
+// cost per line is 20 plus its pairs of ray groups (measured on 512 x 512 and 256
+// x 256 images with 512 to 888 channels: 32 us + 1.6 us per pair and 512 lines).
+static double fp_makespan(const rn_fan_plan* p, int VT) {
+    const int pairs = ((p->g.nu + 30) / 31 + 1) / 2;
+    std::map<double, long long, std::greater<double>> items;   // cost -> how many
+    for (const FpSlice& f : p->h_fp) {
+        const GeoSet& gs = p->h_sets[f.set];
+        for (int y = 0; y < 2; y++) {
+            const int views = y ? gs.nview - gs.nxv : gs.nxv, lines = y ? p->g.nx : p->g.ny;
+            if (views / VT > 0) items[(20.0 + VT * pairs) * lines] += views / VT;
+            if (views % VT > 0) items[(20.0 + views % VT * pairs) * lines]++;
+        }
+    }
+    std::map<double, long long> load{{0.0, 148}};   // finish time -> SMs
+    for (const auto& item : items) {
+        long long left = item.second;
+        if (left > 148 * 32) {   // whole rounds at once
+            const long long rounds = left / 148 - 16;
+            std::map<double, long long> moved;
+            for (const auto& l : load) moved[l.first + rounds * item.first] += l.second;
+            load.swap(moved);
+            left -= rounds * 148;
+        }
+        while (left > 0) {
+            const double t = load.begin()->first;
+            const long long n = std::min(left, load.begin()->second);
+            if ((load.begin()->second -= n) == 0) load.erase(load.begin());
+            load[t + item.first] += n;
+            left -= n;
+        }
+    }
+    return load.rbegin()->first;
+}
+
 static void build_fp_work(rn_fan_plan* p) {
-    // views per work item: at most the kernel's table capacity, fewer when a
-    // small batch would leave SMs idle (one CTA per SM; aim for two waves),
-    // or the tuned count.  A ray's sum does not depend on which views share
-    // its CTA.
+    // views per work item: the count that the list schedule finishes first (more
+    // views share an item's fixed cost, fewer fill the SMs more evenly), or the
+    // tuned count.  A ray's sum does not depend on which views share its CTA.
+    // 16 slices x 36 views of 888 channels: 284 us with as few views as make two
+    // items per SM (one), 225 with four; one 256 x 256 slice x 360 views of 512
+    // channels: 100 us with one, 61 with three.
     const int vmax = fan_fp_views(p->g.nu);
     int VT = vmax;
-    auto items = [&](int vt) {
-        long long n = 0;
-        for (size_t s = 0; s < p->h_fp.size(); s++) {
-            const GeoSet& gs = p->h_sets[p->h_fp[s].set];
-            n += (gs.nxv + vt - 1) / vt + (gs.nview - gs.nxv + vt - 1) / vt;
+    if (p->fp_vt > 0) {
+        VT = std::min(p->fp_vt, vmax);
+    } else {
+        double best = fp_makespan(p, vmax);
+        for (int v = vmax - 1; v >= 1; v--) {
+            const double t = fp_makespan(p, v);
+            if (t < best) {
+                best = t;
+                VT = v;
+            }
         }
-        return n;
-    };
-    if (p->fp_vt > 0) VT = std::min(p->fp_vt, vmax);
-    else
-        while (VT > 1 && items(VT) < 2LL * 148) VT--;
+    }
     p->fp_vt_used = VT;
     p->h_fp_work.clear();
     for (size_t s = 0; s < p->h_fp.size(); s++) {
