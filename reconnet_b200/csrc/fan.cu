@@ -1243,7 +1243,7 @@ __global__ void __launch_bounds__(kBpThreads, kMode == 3 ? 0 : 3) fan_bp_kernel(
     const int nchunks = (gs.nview + kBpViews - 1) / kBpViews;
     auto prep = [&](int c, const ViewGeo* src) {
         // table index = edge / cell index + 1
-        bp_prep<kBpViews, kBmCols, kBmTileY, kMode == 2 ? 3 : 0>(sh, src, c, gs.nview, X0, Y0, tabn, p.win, 1, 2);
+        bp_prep<kBpViews, kBmCols, kBmTileY, kMode == 2 ? 3 : 0>(sh, src, c, gs.nview, X0, Y0, nx, ny, tabn, p.win, 1, 2);
     };
     // tid 0: stage chunk c's table windows into buffer c & 1 and the view
     // records of chunk c + 1 into record slot (c + 1) & 1, on barrier c & 1.
@@ -1462,8 +1462,8 @@ int fan_build_geometry(rn_fan_plan* p, const float* host_deg, FanGeoHost& gh) {
             int nl = xc ? g.ny : g.nx;
             double side = (nl / 2.0 - q.perp) > 0 ? 1.0 : -1.0;
             q.sigma = (float)((r1 > r0 ? 1.0 : -1.0) * side);
-            // Whether the polynomials that pick a lattice point's cell are good to
-            // a quarter of a cell for any lane of the image's tiles (the last ones
+            // Whether the polynomials that pick a lattice point's cell are good (to
+            // a quarter of a cell, the cubic, and 0.01, the quartic) for any lane of the image's tiles (the last ones
             // reach past the image): t_cubic over a lane's 17 points (atan's
             // fourth derivative is at most 4.7), and the matched
             // backprojection's quartic over 32 lines x 32 points (its fifth is at
@@ -1479,7 +1479,8 @@ int fan_build_geometry(rn_fan_plan* p, const float* host_deg, FanGeoHost& gh) {
             const double hc = xc ? reach(kBmCols, kBmTileY, 0, 9) : reach(kBmCols, kBmTileY, 9, 0);
             const double hm = reach(kMatchedTile, kMatchedTile, 17, 17);
             q.cubic = 4.7 / 24 * std::fabs(tB) * std::pow(hc, 4) < 0.25;
-            q.quartic = 24.0 / 120 * std::fabs(tB) * std::pow(hm, 5) < 0.25;
+            q.quartic = 24.0 / 120 * std::fabs(tB) * std::pow(hm, 5) < 0.01;
+            if (!q.quartic) p->matched_near = true;
             // adding and subtracting this rounds a coordinate relative to the
             // source to a multiple of 2^-22 of the largest (or more)
             const double far = std::max(std::fabs(q.par), std::fabs(q.perp)) + std::max(g.nx, g.ny) + 256.0;

@@ -15,6 +15,7 @@ struct BpView {
     double pard, perpd;   // source coordinates (Siddon band positions)
     float par, perp, kappa, tA, tB, sigma, round;
     int xcls;
+    int good;             // the polynomial is good over the whole tile
     int inside;           // the window holds every entry that the tile's edge-index cubics can select
 };
 
@@ -80,13 +81,18 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
 // count of the whole accumulation loop.
 template <int V, int kCols, int kRows, int kPoly = 0>
 __device__ __noinline__ void bp_prep(BpSharedT<V>* sh, const ViewGeo* src, int c, int nview, int X0, int Y0,
-                                     int tabn, int win, int pad, int back) {
+                                     int nx, int ny, int tabn, int win, int pad, int back) {
     const int lane = threadIdx.x & 31, v = lane >> 2, corner = lane & 3;
     const bool valid = v < V && c * V + v < nview;
     const ViewGeo& vg = src[valid ? v : 0];
     const int cx = corner & 1, cy = corner >> 1;
     const int xcls = vg.xcls;
-    const float X = (float)(X0 + cx * kCols), Y = (float)(Y0 + cy * kRows);
+    // the tile's corners; cut to the image unless the polynomial (and with it an
+    // unclamped index of a lane beyond the image) is good over the whole tile,
+    // which may reach past the source
+    const bool whole = kPoly && (kPoly == 4 ? vg.quartic : vg.cubic);
+    const float X = (float)(whole ? X0 + cx * kCols : min(X0 + cx * kCols, nx));
+    const float Y = (float)(whole ? Y0 + cy * kRows : min(Y0 + cy * kRows, ny));
     const float l = xcls ? Y : X, q = xcls ? X : Y;
     float t = matched_t(vg, (q - (float)vg.par) / (l - (float)vg.perp));
     float tmax = t;
@@ -102,8 +108,9 @@ __device__ __noinline__ void bp_prep(BpSharedT<V>* sh, const ViewGeo* src, int c
         sh->elo[slot][v] = max(0, min(lo, tabn - win));
         BpView& w = sh->vw[slot][v];
         // (an index may be a quarter of a cell off, hence one entry of room each side)
+        if (kPoly) w.good = whole;
         if (kPoly)
-            w.inside = (kPoly == 4 ? vg.quartic : vg.cubic) && back >= 1 && lo >= 0 && lo < tabn - win && tmax < 1e6f &&
+            w.inside = whole && back >= 1 && lo >= 0 && lo < tabn - win && tmax < 1e6f &&
                        (int)floorf(tmax) + pad + 1 < lo + win;
         w.pard = vg.par;
         w.perpd = vg.perp;

@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(32 * kBgWarps, 3) fan_bp_group_kernel(GroupPar
     }
     const int nchunks = (nview + kBgViews - 1) / kBgViews;
     auto prep = [&](int c, const ViewGeo* src) {
-        bp_prep<kBgViews, kCols, kTileY>(sh, src, c, nview, X0, Y0, p.tabn, win, kBgPad, 3);
+        bp_prep<kBgViews, kCols, kTileY>(sh, src, c, nview, X0, Y0, p.d.nx, p.d.ny, p.tabn, win, kBgPad, 3);
     };
     auto issue = [&](int c) {
         const int b = c & 1;

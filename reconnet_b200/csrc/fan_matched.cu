@@ -54,8 +54,8 @@ struct MtParams {
 
 // A view as a warp reads it: the quartic of the edge index t(r) = tA + tB
 // atan(kappa r) around the slope at the middle of the warp's 31 x 31 pixels
-// (ViewGeo::quartic says that it stays within a quarter of a cell; at usual
-// geometries it is good to 1e-4, and it only selects the cell), as pairs for
+// (ViewGeo::quartic says that it stays within 0.01 cells; it only selects the
+// cell), as pairs for
 // packed arithmetic.  Lane v works out view v of a chunk.
 struct alignas(16) MtView {
     f32x2 c0, c1, c2, c3, c4, nrt, npar;
@@ -109,6 +109,29 @@ __device__ __forceinline__ void mt_view(float (&line)[kMtBlock], const MtView& v
     }
 }
 
+// The same where the quartic is not good enough (tiles near or beyond the source):
+// a cubic per lane and 8 cells, clamped indices.
+__device__ __forceinline__ void mt_view_near(float (&line)[kMtBlock], const BpView& vg, const float4* T, float l, float q0,
+                                             int ilo, int imax) {
+    const float g = __fdividef(1.0f, l - vg.perp);
+    TCubic c;
+    float hp = 0.f, rp = 0.f;
+#pragma unroll
+    for (int j = 0; j <= kMtBlock; j++) {
+        if (j % 8 == 0) c = t_cubic(vg, ((q0 + (float)(j + 4)) - vg.par) * g);
+        const float a = (q0 + (float)j) - vg.par, h = fmaf(a, g, -c.rt);
+        const float t = fmaf(h, fmaf(h, fmaf(h, c.c3, c.c2), c.c1), c.c0);
+        const float4 E = T[min(max(floor_small(t) + 1, ilo), imax) - ilo];
+        const float r = fmaf(E.z, fmaf(a, g, -E.w), E.y);
+        if (j > 0) line[j - 1] += (E.x - hp) + (r - rp);
+        hp = E.x;
+        rp = r;
+    }
+}
+
+// kNear: some views of the plan are near ones (a kernel of its own: its third
+// form of the line costs the others 4%).
+template <bool kNear>
 __global__ void __launch_bounds__(32 * kMtWarps, 3) fan_bp_matched_kernel(MtParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     MtShared* sh = reinterpret_cast<MtShared*>(smem);
@@ -146,7 +169,7 @@ __global__ void __launch_bounds__(32 * kMtWarps, 3) fan_bp_matched_kernel(MtPara
     }
     const int nchunks = (gs.nview + kMtViews - 1) / kMtViews;
     auto prep = [&](int c, const ViewGeo* src) {
-        bp_prep<kMtViews, kMatchedTile, kMatchedTile, 4>(sh, src, c, gs.nview, X0, Y0, tabn, p.win, 1, 2);
+        bp_prep<kMtViews, kMatchedTile, kMatchedTile, 4>(sh, src, c, gs.nview, X0, Y0, nx, ny, tabn, p.win, 1, 2);
     };
     // tid 0: stage chunk c's table windows into buffer c & 1 and the view
     // records of chunk c + 1 into record slot (c + 1) & 1, on barrier c & 1
@@ -225,7 +248,9 @@ __global__ void __launch_bounds__(32 * kMtWarps, 3) fan_bp_matched_kernel(MtPara
                 mt_view<true>(line, rec[v], l, q0, 0, 0);
             } else {
                 const int ilo = sh->elo[slot][v];
-                mt_view<false>(line, rec[v], l, q0, ilo, ilo + cnt - 1);   // <= nu + 1
+                if (kNear && !sh->vw[slot][v].good)
+                    mt_view_near(line, sh->vw[slot][v], buf0 + (b * kMtViews + v) * p.win, l, q0, ilo, ilo + cnt - 1);
+                else mt_view<false>(line, rec[v], l, q0, ilo, ilo + cnt - 1);   // <= nu + 1
             }
         }
         __syncwarp();   // the records are rewritten for the next chunk
@@ -262,7 +287,8 @@ static size_t matched_smem(int win) {
 }
 
 int fan_matched_attributes() {
-    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_matched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_matched_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_matched_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     return RN_OK;
 }
 
@@ -288,7 +314,11 @@ int fan_matched_launch(rn_fan_plan* p, float* d_img, int accumulate, int s0, int
     m.spin = p->spin_limit;
     m.part_stride = p->img_elems;
     m.parts = p->d_bp_parts;
-    fan_bp_matched_kernel<<<(unsigned)(ns * m.tiles_x * m.tiles_y * nparts), 32 * kMtWarps, matched_smem(m.win), st>>>(m);
+    auto launch = [&](auto kern) {
+        kern<<<(unsigned)(ns * m.tiles_x * m.tiles_y * nparts), 32 * kMtWarps, matched_smem(m.win), st>>>(m);
+    };
+    if (p->matched_near) launch(fan_bp_matched_kernel<true>);
+    else launch(fan_bp_matched_kernel<false>);
     RN_CUDA_TRY(cudaGetLastError());
     return RN_OK;
 }

@@ -158,6 +158,7 @@ struct rn_fan_plan {
     float* d_la = nullptr;          // FP line values
     long long line_slot_elems = 0;  // per FP slice: ny*lpx + nx*lpy
     long long fp_slots = 0;         // FP slices whose lines fit in the scratch
+    bool matched_near = false;      // a view's quartic is not good over every tile (fan_matched.cu)
     int table_win_t = 0;            // the same for the matched backprojection's tiles
     int table_win_m = 0;            // staged table entries per view (BP tiles of 31 x 128 pixels)
     float4* d_tab = nullptr;        // BP edge tables

@@ -1,0 +1,58 @@
+"""The matched fan backprojection's blocks (csrc/fan_matched.cu) and the forward
+projection's pairs of ray groups (csrc/fan.cu) at the sizes where they can go wrong:
+images at and beside a block of 31 and a tile of 62 pixels, one block, views of one
+class only, view chunks of 8 and one more, tiles that reach past the source (indices
+clamped), wide pixels, channels at and beside groups of 31 in odd and even numbers,
+against the FP64 oracle and the adjoint identity.
+
+Tolerance: the fan pair's bar, relative L2 <= 1e-5; adjoint 1e-5."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2, small_fan, to_geometry
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+
+ALL = np.pi * 2
+# name: (geometry, views, range of the angles)
+CASES = {
+    "one_block": (dict(nx=31, ny=31), 9, ALL),
+    "block_and_one": (dict(nx=32, ny=30), 9, ALL),
+    "tile": (dict(nx=62, ny=62), 8, ALL),
+    "tile_and_one": (dict(nx=63, ny=125), 7, ALL),
+    "x_class_only": (dict(nx=40, ny=70), 9, 0.6),
+    "one_view": (dict(nx=33, ny=35), 1, 0.0),
+    "past_the_source": (dict(nx=64, ny=64, dx=2.0, dy=2.0, dso=220.0, dsd=400.0, da=0.012), 11, ALL),
+    "wide_pixels": (dict(nx=40, ny=33, dx=3.0, dy=3.0, da=0.0012, nu=140), 10, ALL),
+    "one_group": (dict(nu=30), 9, ALL),
+    "group": (dict(nu=31), 9, ALL),
+    "two_groups": (dict(nu=62), 6, ALL),
+    "three_groups": (dict(nu=63), 5, ALL),
+    "off_centre": (dict(nx=50, ny=45, nu=90, off_a=5.3), 17, ALL),
+}
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_matched_pair_matches_oracle(name, rng):
+    import torch
+    from oracle import oracle as O
+    from reconnet_b200.torch_ops import FanPlan
+    over, nview, span = CASES[name]
+    g = small_fan(**over)
+    ang = (np.arange(nview) * span / max(nview, 1) + 0.05).astype(np.float32)
+    plan = FanPlan(to_geometry(g), ang, nbatches=2)
+    x = rng.random(plan.img_shape).astype(np.float32)
+    y = rng.random(plan.sino_shape).astype(np.float32)
+    xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    ax, aty = plan.project(xd), plan.backproject(yd, 2)
+    plan.check()
+    assert rel_l2(ax.cpu().numpy(), O.fan_fp(x, ang, g, g.nu, g.nv)) <= TOL
+    assert rel_l2(aty.cpu().numpy(), O.fan_bp(y, ang, g, (g.nx, g.ny, g.nz), 2)) <= TOL
+    lhs, rhs = float((ax.double() * yd.double()).sum()), float((xd.double() * aty.double()).sum())
+    assert abs(lhs - rhs) <= 1e-5 * abs(lhs)
+    acc = plan.backproject(yd, 2, out=torch.full(plan.img_shape, 0.5, device="cuda"), accumulate=True)
+    assert torch.allclose(acc, aty + 0.5, rtol=1e-6, atol=1e-6)
+    plan.set_tuning(bp_parts=1)
+    assert rel_l2(plan.backproject(yd, 2).cpu().numpy(), aty.cpu().numpy()) <= 1e-6
