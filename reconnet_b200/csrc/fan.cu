@@ -1463,7 +1463,7 @@ int fan_build_geometry(rn_fan_plan* p, const float* host_deg, FanGeoHost& gh) {
             double side = (nl / 2.0 - q.perp) > 0 ? 1.0 : -1.0;
             q.sigma = (float)((r1 > r0 ? 1.0 : -1.0) * side);
             // Whether the polynomials that pick a lattice point's cell are good (to
-            // a quarter of a cell, the cubic, and 0.01, the quartic) for any lane of the image's tiles (the last ones
+            // a quarter of a cell, the cubic, and 0.05, the quartic) for any lane of the image's tiles (the last ones
             // reach past the image): t_cubic over a lane's 17 points (atan's
             // fourth derivative is at most 4.7), and the matched
             // backprojection's quartic over 32 lines x 32 points (its fifth is at
@@ -1477,9 +1477,11 @@ int fan_build_geometry(rn_fan_plan* p, const float* host_deg, FanGeoHost& gh) {
                 return D > 0 && std::isfinite(tB * q.par * h) ? h : 1e9;
             };
             const double hc = xc ? reach(kBmCols, kBmTileY, 0, 9) : reach(kBmCols, kBmTileY, 9, 0);
-            const double hm = reach(kMatchedTile, kMatchedTile, 17, 17);
+            // (atan's fifth derivative at u times (1 + u)^5 is at most 130: a warp's
+            // slopes differ by 17 (1 + u) / D from its middle one; twice that)
+            const double hm = reach(kMatchedTile, kMatchedTile, 17 * std::max(1.0, 1.0 / kap), 0);
             q.cubic = 4.7 / 24 * std::fabs(tB) * std::pow(hc, 4) < 0.25;
-            q.quartic = 24.0 / 120 * std::fabs(tB) * std::pow(hm, 5) < 0.01;
+            q.quartic = 2.2 * std::fabs(tB) * std::pow(hm, 5) < 0.05;
             if (!q.quartic) p->matched_near = true;
             // adding and subtracting this rounds a coordinate relative to the
             // source to a multiple of 2^-22 of the largest (or more)

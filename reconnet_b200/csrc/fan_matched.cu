@@ -54,7 +54,7 @@ struct MtParams {
 
 // A view as a warp reads it: the quartic of the edge index t(r) = tA + tB
 // atan(kappa r) around the slope at the middle of the warp's 31 x 31 pixels
-// (ViewGeo::quartic says that it stays within 0.01 cells; it only selects the
+// (ViewGeo::quartic says that it stays within 0.05 cells, usually 1e-3; it only selects the
 // cell), as pairs for
 // packed arithmetic.  Lane v works out view v of a chunk.
 struct alignas(16) MtView {
