@@ -4,7 +4,7 @@ limits beyond which a plan stays on the general kernels.
 
 Tolerance: the cone pair's bar, relative L2 <= 1e-5 (positions are good to
 2.4e-7 of a voxel or ray, which a crossing of a nearly level ray turns into a
-few 1e-6 of its length)."""
+few 1e-6 of its length); the adjoint identity 1e-5, as in the other pairs."""
 from types import SimpleNamespace as NS
 
 import numpy as np
@@ -49,6 +49,14 @@ CASES = {
     "many_rays_per_voxel": (_geom(nx=9, ny=8, nz=9, dz=2.0, nv=90, dv=0.45), dict(nview=5), 1, 1),
     "many_voxels_per_ray": (_geom(nx=9, ny=8, nz=40, dz=0.25, nv=9, dv=4.0), dict(nview=5), 1, 1),
     "steep": (_geom(nx=12, ny=13, nz=24, dz=1.0, nv=60, dv=3.2), dict(nview=6), 1, 1),
+    # level rays in a voxel face: the source's height on one, a detector row at that height
+    "level_row": (_geom(nz=16, dz=1.0, cz=0.0, nv=21, off_v=0.0), dict(nview=7), 1, 1),
+    "level_single_row": (_geom(nz=16, dz=1.0, cz=0.0, nv=1, off_v=0.0), dict(nview=7), 1, 1),
+    "level_row_downwards": (_geom(nz=16, dz=1.0, cz=0.0, nv=21, off_v=0.0), dict(nview=7, up=-1.0), 1, 1),
+    "level_row_higher": (_geom(nz=40, dz=1.0, cz=0.0, nv=21, off_v=0.0), dict(nview=7, height=5.0, det_height=5.0), 1, 1),
+    "level_row_top_face": (_geom(nz=16, dz=1.0, cz=0.0, nv=21, off_v=0.0), dict(nview=5, height=8.0, det_height=8.0), 1, 1),
+    "level_row_bottom_face": (_geom(nz=16, dz=1.0, cz=0.0, nv=21, off_v=0.0), dict(nview=5, height=-8.0, det_height=-8.0), 1, 1),
+    "level_row_chunk_edge": (_geom(nx=9, ny=8, nz=256, dz=1.0, cz=0.0, nv=33, dv=2.0, off_v=0.0), dict(nview=5), 1, 1),
     # outside the column kernels' limits: rays rising more than a voxel per step, a tilted detector axis
     "too_steep": (_geom(nx=12, ny=13, nz=40, dz=0.4, nv=60, dv=3.2), dict(nview=4), 1, 1),
     "tilted": (_geom(), dict(nview=5), 1, 1),
@@ -77,6 +85,23 @@ def test_column_pair_matches_oracle(name, rng):
     assert rel_l2(aty.cpu().numpy(), ref) <= TOL
     acc = plan.backproject(yd, out=torch.full(plan.img_shape, 0.5, device="cuda"), accumulate=True)
     assert torch.allclose(acc, aty + 0.5, rtol=1e-6, atol=1e-6)
+
+
+# in-plane rays that run exactly along a grid line (a column at the axis, views along the axes): which of the two
+# voxels such a ray meets is the sign of a rounding, but the pair has to agree on it
+@pytest.mark.parametrize("nview", [1, 4, 8])
+def test_rays_along_grid_lines_are_adjoint(nview, rng):
+    import torch
+    from reconnet_b200.torch_ops import ConeGeometry, ConePlan
+    g = _geom(nx=24, ny=20, nz=16, dy=1.0, dz=1.0, cx=0.0, cy=0.0, cz=0.0, nu=41, nv=21, off_u=0.0, off_v=0.0)
+    plan = ConePlan(ConeGeometry(**g), *_orbit(nview, start=0.0))
+    # the rays in question alone
+    y = torch.zeros(plan.prj_shape, device="cuda")
+    y[:, 20] = torch.from_numpy(rng.random(tuple(y[:, 20].shape)).astype(np.float32)).cuda()
+    x = torch.from_numpy(rng.random(plan.img_shape).astype(np.float32)).cuda()
+    lhs = float((plan.project(x).double() * y.double()).sum())
+    rhs = float((x.double() * plan.backproject(y).double()).sum())
+    assert abs(lhs - rhs) <= 1e-5 * abs(lhs)
 
 
 def test_column_backprojection_on_two_streams(rng):
