@@ -68,6 +68,7 @@ struct TileView {
     double su, sv, sm;             // source, voxels (x, y, z)
     double ru0, ru1, rv0, rv1;     // slopes ru0 + iu ru1 along x and rv0 + iv rv1 along y, per slab
     float gu_max, gv_max;          // widest ray spacing inside the grid, voxels
+    int vt;                        // the row whose rays are (the closest to) level along y
 };
 struct TilePlan {
     bool fp_narrow = false;        // rays under a voxel apart

@@ -20,7 +20,7 @@
 // that crosses gives its first part [0, ta] to the voxel it leaves and the rest
 // to the next.
 //
-// Positions are 64-bit fixed point (2^-32 or 2^-30 voxels).
+// Positions are 64-bit fixed point (2^-32 or 2^-40 voxels).
 //
 // Measured, 512x512x128 voxels, 736x736 cells, 25 views: forward 1.70 ms with
 // the plane-major copy (3.98 ms for cone_fp_staged_kernel, one thread per ray),
@@ -386,13 +386,17 @@ __global__ void __launch_bounds__(128, 3) cone_bp_tile_kernel(float* __restrict_
             const float ig0 = __fdividef(1.f, (float)gv0), ig1 = __fdividef(1.f, (float)gv1);
             const double bv0 = fma((double)vb, gv0, av0), bv1 = fma((double)vb, gv1, av1);   // ray vb at the two faces
             const float fb0 = (float)bv0, fb1 = (float)bv1;
-            const long long fx0 = to_fixed(bv0), fx1 = to_fixed(bv1), fg0 = to_fixed(gv0), fg1 = to_fixed(gv1);
-            // offsets from a voxel: 26 fractional bits, held to +-8 voxels
-            // (farther rays miss it either way)
-            constexpr int kBits = 26;
+            // 64-bit fixed point with 40 fractional bits; offsets from a voxel are
+            // rounded to 26 and held to +-8 voxels (farther rays miss it either way)
+            constexpr int kWide = 40, kBits = 26;
             constexpr float kUnit = 1.0f / (1 << kBits);
-            const int g0 = (int)(fg0 >> (32 - kBits)), g1 = (int)(fg1 >> (32 - kBits));
-            auto near = [](long long v) { return (int)(max(min(v, 8ll << 32), -(8ll << 32)) >> (32 - kBits)); };
+            auto wide = [](double v) { return llrint(v * (double)(1ll << kWide)); };
+            const long long fx0 = wide(bv0), fx1 = wide(bv1), fg0 = wide(gv0), fg1 = wide(gv1);
+            auto near = [](long long v) {
+                constexpr long long kFar = 8ll << kWide, kHalf = 1ll << (kWide - kBits - 1);
+                return (int)((max(min(v, kFar), -kFar) + kHalf) >> (kWide - kBits));
+            };
+            const int g0 = near(fg0), g1 = near(fg1), level = V.vt - vb;
             const float* col[2];
             f32x2 len[KV];
             float lo[2][KV], hi[2][KV];
@@ -402,8 +406,12 @@ __global__ void __launch_bounds__(128, 3) cone_bp_tile_kernel(float* __restrict_
                 const float e0 = ((float)pv - fb0) * ig0, e1 = ((float)pv - fb1) * ig1;
                 const int jl = min(max((int)ceilf(fminf(e0, e1) - 1e-3f), 0), cols - KV);
                 col[h] = pbase + jl;
-                const long long off = (long long)pv << 32;
-                const int x0i = near(fx0 + jl * fg0 - off), x1i = near(fx1 + jl * fg1 - off);
+                const long long off = (long long)pv << kWide;
+                // stepped from the level ray where the lane has it: in a voxel face it
+                // must come out exactly there (then it belongs to the voxel above, as in
+                // the forward projection)
+                const int jb = min(max(level, jl), jl + KV - 1);
+                const int x0i = near(fx0 + jb * fg0 - off) - (jb - jl) * g0, x1i = near(fx1 + jb * fg1 - off) - (jb - jl) * g1;
 #pragma unroll
                 for (int k = 0; k < KV; k++) {
                     // offsets at the two faces, the slope, and the times at 0 and 1
@@ -529,6 +537,7 @@ bool cone_tile_views(const std::vector<ConeView>& views, const ConeDims& cd, std
         q.ru1 = v.rho[1];
         q.rv0 = v.rho[3];
         q.rv1 = v.rho[5];
+        q.vt = (int)std::min(std::max(std::rint(-q.rv0 / q.rv1), -1e9), 1e9);
         const double e = q.sm + v.Dm0;
         if (!((q.sm < -0.5 && e >= nz) || (q.sm > nz + 0.5 && e <= 0.0))) return false;
         double glo[2] = {1e300, 1e300}, ghi[2] = {0, 0};

@@ -15,10 +15,10 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-5
 
 
-def _views(n, arc=15.0, dist=400.0, below=30.0, lift=6.0, flip=(1.0, 1.0), up=1.0):
+def _views(n, arc=15.0, dist=400.0, below=30.0, lift=6.0, flip=(1.0, 1.0), up=1.0, dcx=1.0, dcy=-0.5):
     a = np.radians(np.linspace(-arc, arc, n)) if n > 1 else np.zeros(1)
     src = np.stack([dist * np.sin(a), lift * np.ones(n), up * dist * np.cos(a)], 1).astype(np.float32)
-    return [np.tile(np.float32([1.0, -0.5, -up * below]), (n, 1)), np.tile(np.float32([flip[0], 0, 0]), (n, 1)),
+    return [np.tile(np.float32([dcx, dcy, -up * below]), (n, 1)), np.tile(np.float32([flip[0], 0, 0]), (n, 1)),
             np.tile(np.float32([0, flip[1], 0]), (n, 1)), src]
 
 
@@ -46,6 +46,12 @@ CASES = {
     "fine_cells": (_geom(nu=110, nv=112, du=0.52, dv=0.5), dict(n=3), 1, 1),
     # steep arcs: most columns cross a voxel line, in either direction
     "steep": (_geom(nz=14, dz=1.9), dict(n=4, arc=24.0, dist=160.0), 1, 1),
+    # level rays in a voxel face: a detector row at the source's y, on a grid line
+    "level_row": (_geom(nx=32, ny=32, dy=1.0, cx=0.0, cy=0.0, nu=40, nv=41, off_u=0.0, off_v=0.0), dict(n=4, lift=0.0, dcy=0.0), 1, 1),
+    "level_row_fine": (_geom(nx=34, ny=128, dy=1.0, cx=0.0, cy=0.0, nu=80, nv=161, du=0.6, dv=0.6, off_u=0.0, off_v=0.0),
+                       dict(n=4, lift=0.0, dcy=0.0), 1, 1),
+    "level_row_and_column": (_geom(nx=32, ny=64, dy=1.0, cx=0.0, cy=0.0, nu=41, nv=81, off_u=0.0, off_v=0.0),
+                             dict(n=1, lift=-7.0, dcx=0.0, dcy=-7.0), 1, 1),
     # outside the limits: a reversed axis, cells under 0.3 voxels, slopes over one
     "reversed_v": (_geom(), dict(n=3, flip=(1.0, -1.0)), 1, 1),
     "very_fine": (_geom(nu=90, nv=91, du=0.25, dv=0.25), dict(n=2), 1, 1),
