@@ -28,13 +28,12 @@
 
 namespace rn {
 
-constexpr int kMtViews = 8;                    // views per staged chunk
 constexpr int kMtBlock = 31;                   // pixels per block side: lanes 0..30, the last lane only supplies a line
 constexpr int kMtWarps = 4;                    // 2 x 2 blocks
 constexpr int kMtPitch = kMtBlock + 2;         // odd: rows and columns of the pixel store are free of bank conflicts
 constexpr int kMtStore = kMtBlock * kMtPitch;  // floats per warp
 static_assert(2 * kMtBlock == kMatchedTile, "the plan sizes windows and cubics for this tile");
-using MtShared = BpSharedT<kMtViews>;
+constexpr int kMtSmem = 113 * 1024;            // two blocks per SM
 
 struct MtParams {
     const ViewGeo* views;
@@ -62,6 +61,24 @@ struct alignas(16) MtView {
     float perp;
     uint32_t tbase;   // byte address of the entry of edge index 0 less the bias of the round-down add
 };
+
+// A block's shared memory with V views per staged chunk: the views' parameters,
+// the pixel store, the warps' view records, then two buffers of V table windows.
+// Windows widen with the pixels (in detector cells), so wide ones go with fewer
+// views per chunk: as many of 8, 4 and 2 as leave room for two blocks per SM, or
+// else two, which fit whatever window the plan's own limit lets through.  8 slices
+// of 576 to 720 views: 256 x 256 pixels of 1.65 mm (392 entries) 0.80 ms with eight
+// views (one block per SM), 0.53 with four; 128 x 128 pixels of 2.9 mm (656 entries)
+// 0.35 with eight, 0.27 with four (two blocks per SM), 0.28 with two (three); 316 x
+// 316 pixels of 1.2 mm (280 entries) 0.70 with eight (two blocks), 0.71 with four.
+template <int V>
+struct MtLayout {
+    static constexpr size_t kStore = (sizeof(BpSharedT<V>) + 127) & ~size_t(127);
+    static constexpr size_t kRec = (kStore + sizeof(float) * kMtWarps * kMtStore + 127) & ~size_t(127);
+    static constexpr size_t kBuf = (kRec + sizeof(MtView) * kMtWarps * V + 127) & ~size_t(127);
+    static size_t bytes(int win) { return kBuf + 2 * (size_t)V * win * sizeof(float4); }
+};
+
 __device__ __forceinline__ void mt_prepare(MtView& o, const BpView& vg, float lmid, float qmid, uint32_t T, int ilo) {
     const float rt = (qmid - vg.par) * __fdividef(1.0f, lmid - vg.perp), ut = vg.kappa * rt, u2 = ut * ut;
     const float iw = __fdividef(1.0f, 1.0f + u2), kw = vg.kappa * iw;
@@ -129,16 +146,14 @@ __device__ __forceinline__ void mt_view_near(float (&line)[kMtBlock], const BpVi
     }
 }
 
-// kNear: some views of the plan are near ones (a kernel of its own: its third
-// form of the line costs the others 4%).
-template <bool kNear>
+// V views per staged chunk.  kNear: some views of the plan are near ones (a
+// kernel of its own: its third form of the line costs the others 4%).
+template <int V, bool kNear>
 __global__ void __launch_bounds__(32 * kMtWarps, 3) fan_bp_matched_kernel(MtParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    MtShared* sh = reinterpret_cast<MtShared*>(smem);
-    constexpr size_t kStoreOff = (sizeof(MtShared) + 127) & ~size_t(127);
-    constexpr size_t kRecOff = (kStoreOff + sizeof(float) * kMtWarps * kMtStore + 127) & ~size_t(127);
-    constexpr size_t kBufOff = (kRecOff + sizeof(MtView) * kMtWarps * kMtViews + 127) & ~size_t(127);
-    float4* const buf0 = reinterpret_cast<float4*>(smem + kBufOff);   // buffer b at buf0 + b * kMtViews * win
+    using L = MtLayout<V>;
+    BpSharedT<V>* sh = reinterpret_cast<BpSharedT<V>*>(smem);
+    float4* const buf0 = reinterpret_cast<float4*>(smem + L::kBuf);   // buffer b at buf0 + b * V * win
 
     const int tiles = p.tiles_x * p.tiles_y;
     const int part = blockIdx.x % p.nparts, bid = blockIdx.x / p.nparts;
@@ -159,35 +174,37 @@ __global__ void __launch_bounds__(32 * kMtWarps, 3) fan_bp_matched_kernel(MtPara
     const int X0 = txi * kMatchedTile, Y0 = tyi * kMatchedTile;
     const int bx = X0 + (warp & 1) * kMtBlock, by = Y0 + (warp >> 1) * kMtBlock;
     const bool live = bx < nx && by < ny;   // the whole warp
-    MtView* const rec = reinterpret_cast<MtView*>(smem + kRecOff) + warp * kMtViews;
-    float* const store = reinterpret_cast<float*>(smem + kStoreOff) + warp * kMtStore;   // pixel (bx + a, by + b) at a kMtPitch + b
+    MtView* const rec = reinterpret_cast<MtView*>(smem + L::kRec) + warp * V;
+    float* const store = reinterpret_cast<float*>(smem + L::kStore) + warp * kMtStore;   // pixel (bx + a, by + b) at a kMtPitch + b
 
     if (tid == 0) {
         mbar_init(&sh->bars[0], 1);
         mbar_init(&sh->bars[1], 1);
         fence_mbar_init();
     }
-    const int nchunks = (gs.nview + kMtViews - 1) / kMtViews;
+    const int nchunks = (gs.nview + V - 1) / V;
     auto prep = [&](int c, const ViewGeo* src) {
-        bp_prep<kMtViews, kMatchedTile, kMatchedTile, 4>(sh, src, c, gs.nview, X0, Y0, nx, ny, tabn, p.win, 1, 2);
+        bp_prep<V, kMatchedTile, kMatchedTile, 4>(sh, src, c, gs.nview, X0, Y0, nx, ny, tabn, p.win, 1, 2);
     };
     // tid 0: stage chunk c's table windows into buffer c & 1 and the view
     // records of chunk c + 1 into record slot (c + 1) & 1, on barrier c & 1
     auto issue = [&](int c) {
-        const int b = c & 1, vc = min(kMtViews, gs.nview - c * kMtViews), cnt = min(p.win, tabn);
-        const int vn = c + 1 < nchunks ? min(kMtViews, gs.nview - (c + 1) * kMtViews) : 0;
+        const int b = c & 1, vc = min(V, gs.nview - c * V), cnt = min(p.win, tabn);
+        const int vn = c + 1 < nchunks ? min(V, gs.nview - (c + 1) * V) : 0;
         fence_proxy_async();
         mbar_arrive_expect_tx(&sh->bars[b], (uint32_t)(vc * cnt * sizeof(float4) + vn * sizeof(ViewGeo)));
         for (int v = 0; v < vc; v++)
-            bulk_g2s(buf0 + (b * kMtViews + v) * p.win, gtab + (long long)(c * kMtViews + v) * tabn + sh->elo[c % 3][v],
+            bulk_g2s(buf0 + (b * V + v) * p.win, gtab + (long long)(c * V + v) * tabn + sh->elo[c % 3][v],
                      (uint32_t)(cnt * sizeof(float4)), &sh->bars[b]);
         if (vn > 0)
-            bulk_g2s(sh->rec[(c + 1) & 1], p.views + gs.view_off + (c + 1) * kMtViews, (uint32_t)(vn * sizeof(ViewGeo)),
+            bulk_g2s(sh->rec[(c + 1) & 1], p.views + gs.view_off + (c + 1) * V, (uint32_t)(vn * sizeof(ViewGeo)),
                      &sh->bars[b]);
     };
-    if (tid < 32) prep(0, p.views + gs.view_off);
-    __syncthreads();
-    if (tid == 0) issue(0);
+    if (nchunks > 0) {
+        if (tid < 32) prep(0, p.views + gs.view_off);
+        __syncthreads();
+        if (tid == 0) issue(0);
+    }
 
     float line[kMtBlock];
 #pragma unroll
@@ -226,14 +243,14 @@ __global__ void __launch_bounds__(32 * kMtWarps, 3) fan_bp_matched_kernel(MtPara
         }
         if (tid == 0 && c + 1 < nchunks) issue(c + 1);
         if (!live) continue;
-        const int slot = c % 3, vc = min(kMtViews, gs.nview - c * kMtViews), cnt = min(p.win, tabn);
+        const int slot = c % 3, vc = min(V, gs.nview - c * V), cnt = min(p.win, tabn);
         bool xv = false, in = false;
         if (lane < vc) {
             const BpView& vg = sh->vw[slot][lane];
             xv = vg.xcls != 0;
             in = vg.inside != 0;
             mt_prepare(rec[lane], vg, (float)(xv ? by : bx) + 0.5f * kMtBlock, (float)(xv ? bx : by) + 0.5f * kMtBlock,
-                       smem_u32(buf0 + (b * kMtViews + lane) * p.win), sh->elo[slot][lane]);
+                       smem_u32(buf0 + (b * V + lane) * p.win), sh->elo[slot][lane]);
         }
         const unsigned xmask = __ballot_sync(0xffffffffu, xv), inside = __ballot_sync(0xffffffffu, in);
         __syncwarp();
@@ -249,7 +266,7 @@ __global__ void __launch_bounds__(32 * kMtWarps, 3) fan_bp_matched_kernel(MtPara
             } else {
                 const int ilo = sh->elo[slot][v];
                 if (kNear && !sh->vw[slot][v].good)
-                    mt_view_near(line, sh->vw[slot][v], buf0 + (b * kMtViews + v) * p.win, l, q0, ilo, ilo + cnt - 1);
+                    mt_view_near(line, sh->vw[slot][v], buf0 + (b * V + v) * p.win, l, q0, ilo, ilo + cnt - 1);
                 else mt_view<false>(line, rec[v], l, q0, ilo, ilo + cnt - 1);   // <= nu + 1
             }
         }
@@ -279,16 +296,23 @@ __global__ void __launch_bounds__(32 * kMtWarps, 3) fan_bp_matched_kernel(MtPara
     }
 }
 
-static size_t matched_smem(int win) {
-    const size_t store = (sizeof(MtShared) + 127) & ~size_t(127);
-    const size_t rec = (store + sizeof(float) * kMtWarps * kMtStore + 127) & ~size_t(127);
-    const size_t buf = (rec + sizeof(MtView) * kMtWarps * kMtViews + 127) & ~size_t(127);
-    return buf + 2 * (size_t)kMtViews * win * sizeof(float4);
+// Views per staged chunk for windows of `win` entries; 0 where not even two fit.
+static int matched_views(int win) {
+    if (MtLayout<8>::bytes(win) <= kMtSmem) return 8;
+    if (MtLayout<4>::bytes(win) <= kMtSmem) return 4;
+    return MtLayout<2>::bytes(win) <= 227 * 1024 ? 2 : 0;
 }
 
+bool fan_matched_fits(int win) { return matched_views(win) > 0; }
+
 int fan_matched_attributes() {
-    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_matched_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_matched_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_matched_kernel<8, false>, attr, kMtSmem));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_matched_kernel<8, true>, attr, kMtSmem));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_matched_kernel<4, false>, attr, kMtSmem));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_matched_kernel<4, true>, attr, kMtSmem));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_matched_kernel<2, false>, attr, 227 * 1024));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_matched_kernel<2, true>, attr, 227 * 1024));
     return RN_OK;
 }
 
@@ -314,11 +338,20 @@ int fan_matched_launch(rn_fan_plan* p, float* d_img, int accumulate, int s0, int
     m.spin = p->spin_limit;
     m.part_stride = p->img_elems;
     m.parts = p->d_bp_parts;
-    auto launch = [&](auto kern) {
-        kern<<<(unsigned)(ns * m.tiles_x * m.tiles_y * nparts), 32 * kMtWarps, matched_smem(m.win), st>>>(m);
+    auto launch = [&](auto kern, size_t smem) {
+        kern<<<(unsigned)(ns * m.tiles_x * m.tiles_y * nparts), 32 * kMtWarps, smem, st>>>(m);
     };
-    if (p->matched_near) launch(fan_bp_matched_kernel<true>);
-    else launch(fan_bp_matched_kernel<false>);
+    const bool near = p->matched_near;
+    switch (matched_views(m.win)) {
+        case 8:
+            launch(near ? fan_bp_matched_kernel<8, true> : fan_bp_matched_kernel<8, false>, MtLayout<8>::bytes(m.win));
+            break;
+        case 4:
+            launch(near ? fan_bp_matched_kernel<4, true> : fan_bp_matched_kernel<4, false>, MtLayout<4>::bytes(m.win));
+            break;
+        default:
+            launch(near ? fan_bp_matched_kernel<2, true> : fan_bp_matched_kernel<2, false>, MtLayout<2>::bytes(m.win));
+    }
     RN_CUDA_TRY(cudaGetLastError());
     return RN_OK;
 }

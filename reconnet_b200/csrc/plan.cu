@@ -256,7 +256,10 @@ static int finish_plan(rn_fan_plan* p, const float* host_deg, cudaStream_t st) {
     if (win_m < 0) return set_error(RN_ERR_ARG, "fan geometry: the image reaches the source");
     if (win_m > 800) return set_error(RN_ERR_ARG, "fan geometry: backprojection tile window too large");
     p->table_win_m = win_m;
+    // (at most twice as wide: 2 win_m + 16 entries, which always fit)
     p->table_win_t = table_window(g, kMatchedTile, kMatchedTile);
+    if (!fan_matched_fits(p->table_win_t))
+        return set_error(RN_ERR_ARG, "fan geometry: matched backprojection tile window too large");
     RN_TRY(fan_kernel_attributes());
     FanGeoHost gh;
     RN_TRY(fan_build_geometry(p, host_deg, gh));

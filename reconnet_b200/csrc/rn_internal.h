@@ -240,6 +240,8 @@ int fan_slope_tables(rn_fan_plan* p, const double2* d_vcs, const int* d_vx, cons
 // it does not split), and the number of slices in its first launch.
 int fan_bp_split(const rn_fan_plan* p, int type, int* first_wave_slices);
 // Matched backprojection of slices whose tables are built (fan_matched.cu).
+// whether its staged windows of `win` table entries fit in shared memory
+bool fan_matched_fits(int win);
 int fan_matched_attributes();
 int fan_matched_launch(rn_fan_plan* p, float* d_img, int accumulate, int s0, int ns, long long table_base, int nparts,
                        cudaStream_t st);

@@ -26,6 +26,10 @@ CASES = {
     "one_view": (dict(nx=33, ny=35), 1, 0.0),
     "past_the_source": (dict(nx=64, ny=64, dx=2.0, dy=2.0, dso=220.0, dsd=400.0, da=0.012), 11, ALL),
     "wide_pixels": (dict(nx=40, ny=33, dx=3.0, dy=3.0, da=0.0012, nu=140), 10, ALL),
+    # table windows of 232 entries (eight views per chunk), 472 (four), 832 (two)
+    "window_232": (dict(nx=70, ny=75, dx=1.2, dy=1.2, nu=300, da=0.0009), 17, ALL),
+    "window_472": (dict(nx=70, ny=75, dx=1.2, dy=1.2, nu=600, da=0.00043), 17, ALL),
+    "window_832": (dict(nx=200, ny=800, dx=2.0, dy=0.5, nu=2000, da=0.0005), 9, ALL),
     "one_group": (dict(nu=30), 9, ALL),
     "group": (dict(nu=31), 9, ALL),
     "two_groups": (dict(nu=62), 6, ALL),
