@@ -43,6 +43,10 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <atomic>
+#include <condition_variable>
+#include <deque>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -766,6 +770,188 @@ __global__ void __launch_bounds__(256) cone_bp_kernel(float* __restrict__ img, c
 
 using namespace rn;
 
+namespace {
+
+// Calls that allocate or ask about events stay legal while another thread captures.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Scratch of a plan's calls, in a few buffers that live as long as the plan.  A
+// call holds one from `get` to `put` and leaves an event behind it; the next call to
+// get the buffer waits for that event on its own stream, so calls on several streams
+// and threads never share one at a time: they have a buffer each, up to kBuffers, then
+// they queue.  A call under stream capture takes a buffer that belongs to the graph
+// (one per capture and stream, whose calls are ordered) until the graph and
+// everything instantiated from it are gone; so captured calls add kernel nodes
+// only, and the graph can be cloned, or be a child of another.
+class ConeScratch {
+public:
+    struct Buffer {
+        void* ptr;
+        size_t bytes;
+        cudaEvent_t done;
+        cudaStream_t stream;
+        bool held;
+    };
+    struct Hold {
+        void* ptr = nullptr;   // null: no room on the device
+        Buffer* buffer = nullptr;
+    };
+
+    // The size that serves every call of the plan; a buffer of it now (best effort),
+    // so that the first call need not allocate.
+    void reserve(size_t bytes) {
+        std::lock_guard<std::mutex> lk(mu_);
+        full_ = bytes;
+        if (bytes > 0) grow(bytes);
+    }
+
+    int get(size_t bytes, cudaStream_t st, Hold* out) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        unsigned long long id = 0;
+        cudaGraph_t graph = nullptr;
+        RN_CUDA_TRY(cudaStreamGetCaptureInfo_v2(st, &status, &id, &graph, nullptr, nullptr));
+        if (status == cudaStreamCaptureStatusActive) return get_captured(bytes, st, id, graph, out);
+        std::unique_lock<std::mutex> lk(mu_);
+        for (;;) {
+            Buffer* pick = nullptr;
+            bool idle = false, held = false;
+            for (Buffer& b : buffers_) {
+                if (b.bytes < bytes) continue;
+                held = held || b.held;
+                if (b.held) continue;
+                RelaxedCapture relaxed;
+                idle = b.stream == st || cudaEventQuery(b.done) == cudaSuccess;
+                if (idle || !pick) pick = &b;
+                if (idle) break;
+            }
+            if (!idle && buffers_.size() < kBuffers && grow(bytes)) pick = &buffers_.back();
+            if (pick) {
+                RN_CUDA_TRY(cudaStreamWaitEvent(st, pick->done, 0));
+                pick->held = true;
+                pick->stream = st;
+                out->ptr = pick->ptr;
+                out->buffer = pick;
+                return RN_OK;
+            }
+            if (!held) return RN_OK;   // no room
+            cv_.wait(lk);
+        }
+    }
+
+    // the launches that use the buffer are on `st`
+    int put(const Hold& h, cudaStream_t st) {
+        if (!h.buffer) return RN_OK;
+        const cudaError_t e = cudaEventRecord(h.buffer->done, st);
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            h.buffer->held = false;
+        }
+        cv_.notify_one();
+        RN_CUDA_TRY(e);
+        return RN_OK;
+    }
+
+    ~ConeScratch() {
+        for (Buffer& b : buffers_) {
+            cudaFree(b.ptr);
+            cudaEventDestroy(b.done);
+        }
+        for (Captured& c : captured_) cudaFree(c.ptr);
+    }
+
+private:
+    static constexpr size_t kBuffers = 4;
+    struct Captured {
+        void* ptr;
+        size_t bytes;
+        unsigned long long id;
+        cudaStream_t stream;
+        std::shared_ptr<std::atomic<bool>> live;   // shared with the graph, which clears it
+    };
+
+    static void* allocate(size_t bytes) {
+        RelaxedCapture relaxed;
+        void* ptr = nullptr;
+        if (cudaMalloc(&ptr, bytes) == cudaSuccess) return ptr;
+        cudaGetLastError();
+        return nullptr;
+    }
+
+    bool grow(size_t bytes) {
+        Buffer b{allocate(std::max(bytes, full_)), std::max(bytes, full_), nullptr, nullptr, false};
+        if (!b.ptr && bytes < full_) {
+            b.ptr = allocate(bytes);
+            b.bytes = bytes;
+        }
+        if (!b.ptr) return false;
+        if (cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFree(b.ptr);
+            return false;
+        }
+        buffers_.push_back(b);
+        return true;
+    }
+
+    int get_captured(size_t bytes, cudaStream_t st, unsigned long long id, cudaGraph_t graph, Hold* out) {
+        std::lock_guard<std::mutex> lk(mu_);
+        Captured* free = nullptr;
+        for (Captured& c : captured_) {
+            if (c.bytes < bytes) continue;
+            if (!c.live->load()) {
+                free = &c;
+            } else if (c.id == id && c.stream == st) {
+                out->ptr = c.ptr;
+                return RN_OK;
+            }
+        }
+        if (!free) {
+            size_t size = std::max(bytes, full_);
+            void* ptr = allocate(size);
+            if (!ptr && bytes < size) ptr = allocate(size = bytes);
+            if (!ptr) return RN_OK;
+            captured_.push_back(Captured{ptr, size, 0, nullptr, std::make_shared<std::atomic<bool>>(false)});
+            free = &captured_.back();
+        }
+        auto* token = new std::shared_ptr<std::atomic<bool>>(free->live);
+        cudaUserObject_t object = nullptr;
+        cudaError_t e = cudaUserObjectCreate(
+            &object, token,
+            [](void* t) {
+                auto* live = static_cast<std::shared_ptr<std::atomic<bool>>*>(t);
+                (*live)->store(false);
+                delete live;
+            },
+            1, cudaUserObjectNoDestructorSync);
+        if (e != cudaSuccess) {
+            delete token;
+            return set_cuda_error(e, "cone scratch");
+        }
+        free->live->store(true);
+        e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+        if (e != cudaSuccess) {
+            cudaUserObjectRelease(object, 1);   // clears `live` again
+            return set_cuda_error(e, "cone scratch");
+        }
+        free->id = id;
+        free->stream = st;
+        out->ptr = free->ptr;
+        return RN_OK;
+    }
+
+    std::mutex mu_;
+    std::condition_variable cv_;
+    size_t full_ = 0;
+    std::deque<Buffer> buffers_;   // (a deque: entries that calls hold do not move)
+    std::vector<Captured> captured_;
+};
+
+}  // namespace
+
 struct rn_cone_plan {
     ConeDims cd;
     int device = 0;
@@ -782,43 +968,11 @@ struct rn_cone_plan {
     bool tile = false;         // tomosynthesis: the kernels of cone_tile.cu
     TilePlan tp;
     TileView* d_tile = nullptr;
-    // scratch of one call: taken from and given back to the plan's own pool in
-    // stream order, so calls on several streams or threads each have theirs;
-    // the pool keeps the memory for the next call until the plan goes
-    std::mutex pool_mu;
-    cudaMemPool_t pool = nullptr;
-    float* d_prjw = nullptr;   // separable backprojection: projections times segment lengths (lazily allocated)
+    std::unique_ptr<ConeScratch> scratch{new ConeScratch};
     long long launches = 0;
 };
 
 namespace {
-
-// *out stays null where the device has no room (a tomosynthesis plan then takes
-// the general kernels; an upright plan's table is a quarter of the ray table that
-// the general backprojection keeps).
-int scratch_get(rn_cone_plan* p, size_t bytes, cudaStream_t st, void** out) {
-    {
-        std::lock_guard<std::mutex> lk(p->pool_mu);
-        if (!p->pool) {
-            cudaMemPoolProps props;
-            memset(&props, 0, sizeof(props));
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = p->device;
-            RN_CUDA_TRY(cudaMemPoolCreate(&p->pool, &props));
-            uint64_t keep = UINT64_MAX;
-            RN_CUDA_TRY(cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep));
-        }
-    }
-    const cudaError_t e = cudaMallocFromPoolAsync(out, bytes, p->pool, st);
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        *out = nullptr;
-        return RN_OK;
-    }
-    RN_CUDA_TRY(e);
-    return RN_OK;
-}
 
 int cone_views(rn_cone_plan* p, const RnConeGeom& g, const float* dc, const float* du_, const float* dv_,
                const float* src, std::vector<ConeView>& out, double& max_slope) {
@@ -935,6 +1089,31 @@ int cone_views(rn_cone_plan* p, const RnConeGeom& g, const float* dc, const floa
     return RN_OK;
 }
 
+size_t cone_bp_scratch_bytes(const rn_cone_plan* p) {
+    if (p->col) return cone_col_table_bytes(p->cd);
+    if (p->tile) return cone_tile_bp_bytes(p->cd);
+    return p->bp_sep ? sizeof(float) * p->cd.nb * p->cd.prj_b : 0;
+}
+
+// cone_bp_sep_kernel on the projections times the segment lengths (prjw).
+int cone_sep_backproject(rn_cone_plan* p, float* prjw, float* d_img, const float* d_prj, int accumulate,
+                         cudaStream_t st) {
+    const ConeDims& cd = p->cd;
+    cone_prj_seg_kernel<<<dim3((unsigned)((cd.nv * cd.nc + 255) / 256), (unsigned)cd.nview, (unsigned)cd.nu), 256, 0,
+                          st>>>(prjw, d_prj, p->d_views, cd);
+    RN_CUDA_TRY(cudaGetLastError());
+    // one warp per 2 (U) x 32 (V) voxels at one m
+    const ConeView& v0 = p->h_view0;
+    const int ax_u = v0.affine == 1 ? v0.a : v0.b;
+    const long long warps = (long long)((cd.n[ax_u] + 1) / 2) * cd.n[v0.m];
+    const dim3 grid((unsigned)((warps + kSepWarps - 1) / kSepWarps), (unsigned)((cd.n[p->bp_fast] + 31) / 32),
+                    (unsigned)(cd.nb * cd.nc));
+    cone_bp_sep_kernel<<<grid, 32 * kSepWarps, 0, st>>>(d_img, prjw, p->d_views, cd, accumulate);
+    RN_CUDA_TRY(cudaGetLastError());
+    p->launches += 2;
+    return RN_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1022,6 +1201,8 @@ int rn_cone_plan_create(rn_cone_plan** out, const RnConeGeom* g, const float* ho
         cone_ray_kernel<<<(unsigned)((nrays + 255) / 256), 256, 0, st>>>(p->d_rays, p->d_views, cd);
         e = cudaGetLastError();
     }
+    if (p->col || p->tile)
+        p->scratch->reserve(std::max(cone_bp_scratch_bytes(p), p->tile ? cone_tile_fp_bytes(cd) : 0));
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // the host copies go out of scope
     if (e != cudaSuccess) {
         rn_cone_plan_destroy(p);
@@ -1035,10 +1216,8 @@ int rn_cone_plan_destroy(rn_cone_plan* p) {
     if (!p) return RN_OK;
     cudaFree(p->d_views);
     cudaFree(p->d_rays);
-    cudaFree(p->d_prjw);
     cudaFree(p->d_col);
     cudaFree(p->d_tile);
-    if (p->pool) cudaMemPoolDestroy(p->pool);
     delete p;
     return RN_OK;
 }
@@ -1055,14 +1234,15 @@ int rn_cone_project(rn_cone_plan* p, float* d_prj, const float* d_img, void* str
     }
     if (p->tile) {
         cudaStream_t st = (cudaStream_t)stream;
-        void* vol = nullptr;
-        RN_TRY(scratch_get(p, cone_tile_fp_bytes(cd), st, &vol));
-        if (vol) {
+        ConeScratch::Hold vol;
+        RN_TRY(p->scratch->get(cone_tile_fp_bytes(cd), st, &vol));
+        if (vol.ptr) {
             p->launches += 2LL * cd.nb * cd.nc;
-            const int s = cone_tile_project(p->d_tile, cd, p->tp, static_cast<float*>(vol), d_prj, d_img, st);
-            cudaFreeAsync(vol, st);
+            const int s = cone_tile_project(p->d_tile, cd, p->tp, static_cast<float*>(vol.ptr), d_prj, d_img, st);
+            RN_TRY(p->scratch->put(vol, st));
             return s;
         }
+        // no room for the plane-major copy: the general kernel needs none
     }
     const int gx = p->lanes_v ? (cd.nu + 7) / 8 : (cd.nu + 31) / 32;
     const int gy = p->lanes_v ? (cd.nv + 31) / 32 : (cd.nv + 7) / 8;
@@ -1087,51 +1267,29 @@ int rn_cone_backproject(rn_cone_plan* p, float* d_img, const float* d_prj, int a
     const long long nvox = (long long)cd.n[0] * cd.n[1] * cd.n[2];
     const int slices = cd.nb * cd.nc;
     if (slices > 65535) return set_error(RN_ERR_ARG, "cone backprojection: too many batches x channels");
-    if (p->col) {
+    if (p->col || p->tile || p->bp_sep) {
         cudaStream_t st = (cudaStream_t)stream;
-        void* tab = nullptr;
-        RN_TRY(scratch_get(p, cone_col_table_bytes(cd), st, &tab));
-        if (!tab) return set_cuda_error(cudaErrorMemoryAllocation, "cone backprojection: prefix table");
-        p->launches += 2LL * slices;
-        const int s = cone_col_backproject(p->d_col, cd, p->col_one, static_cast<double*>(tab), d_img, d_prj,
-                                           accumulate, st);
-        cudaFreeAsync(tab, st);
+        if (p->bp_sep && !p->tile && (cd.nu > 65535 || cd.nview > 65535))
+            return set_error(RN_ERR_ARG, "cone backprojection: more than 65535 detector columns or views");
+        ConeScratch::Hold h;
+        RN_TRY(p->scratch->get(cone_bp_scratch_bytes(p), st, &h));
+        if (!h.ptr) return set_cuda_error(cudaErrorMemoryAllocation, "cone backprojection: scratch");
+        int s = RN_OK;
+        if (p->col) {
+            p->launches += 2LL * slices;
+            s = cone_col_backproject(p->d_col, cd, p->col_one, static_cast<double*>(h.ptr), d_img, d_prj, accumulate, st);
+        } else if (p->tile) {
+            p->launches += 2LL * slices;
+            s = cone_tile_backproject(p->d_tile, cd, p->tp, static_cast<float*>(h.ptr), d_img, d_prj, accumulate, st);
+        } else {
+            s = cone_sep_backproject(p, static_cast<float*>(h.ptr), d_img, d_prj, accumulate, st);
+        }
+        RN_TRY(p->scratch->put(h, st));
         return s;
     }
-    if (p->tile) {
-        cudaStream_t st = (cudaStream_t)stream;
-        void* wp = nullptr;
-        RN_TRY(scratch_get(p, cone_tile_bp_bytes(cd), st, &wp));
-        if (!wp && !p->bp_sep) return set_cuda_error(cudaErrorMemoryAllocation, "cone backprojection: scratch");
-        if (wp) {
-            p->launches += 2LL * slices;
-            const int s =
-                cone_tile_backproject(p->d_tile, cd, p->tp, static_cast<float*>(wp), d_img, d_prj, accumulate, st);
-            cudaFreeAsync(wp, st);
-            return s;
-        }
-    }
-    if (p->bp_sep) {
-        // one warp per 2 (U) x 32 (V) voxels at one m
-        const ConeView& v0 = p->h_view0;
-        const int ax_u = v0.affine == 1 ? v0.a : v0.b;
-        const int nv_axis = cd.n[p->bp_fast];
-        const long long warps = (long long)((cd.n[ax_u] + 1) / 2) * cd.n[v0.m];
-        if (!p->d_prjw) RN_CUDA_TRY(cudaMalloc(&p->d_prjw, sizeof(float) * cd.nb * cd.prj_b));
-        if (cd.nu > 65535 || cd.nview > 65535)
-            return set_error(RN_ERR_ARG, "cone backprojection: more than 65535 detector columns or views");
-        cone_prj_seg_kernel<<<dim3((unsigned)((cd.nv * cd.nc + 255) / 256), (unsigned)cd.nview, (unsigned)cd.nu), 256,
-                              0, (cudaStream_t)stream>>>(p->d_prjw, d_prj, p->d_views, cd);
-        RN_CUDA_TRY(cudaGetLastError());
-        p->launches++;
-        dim3 grid((unsigned)((warps + kSepWarps - 1) / kSepWarps), (unsigned)((nv_axis + 31) / 32), slices);
-        cone_bp_sep_kernel<<<grid, 32 * kSepWarps, 0, (cudaStream_t)stream>>>(d_img, p->d_prjw, p->d_views, cd,
-                                                                             accumulate);
-    } else {
-        dim3 grid((unsigned)((nvox + 255) / 256), slices);
-        cone_bp_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(d_img, d_prj, p->d_rays, p->d_views, cd, accumulate,
-                                                                p->bp_fast);
-    }
+    dim3 grid((unsigned)((nvox + 255) / 256), slices);
+    cone_bp_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(d_img, d_prj, p->d_rays, p->d_views, cd, accumulate,
+                                                            p->bp_fast);
     p->launches++;
     RN_CUDA_TRY(cudaGetLastError());
     return RN_OK;
