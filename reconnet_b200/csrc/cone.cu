@@ -56,6 +56,21 @@
 
 namespace rn {
 
+// Rays whose slope is under this are level: the forward projection's fixed-point
+// positions (2^-32) do not move along them.  A level ray in a voxel face belongs to
+// the voxel above it there, so the backprojections keep its position exact: slopes
+// under kLevel count as 0, positions within 2 kLevel of a face as in the face, and
+// FP32 steps along the detector start from the level ray.
+constexpr float kLevel = 1.1641532e-10f;   // 2^-33
+
+__device__ __forceinline__ float level_inverse(float r) { return fabsf(r) > kLevel ? __fdividef(1.f, r) : 1e30f; }
+__device__ __forceinline__ float snap_face(float x) { return fabsf(x) < 2.f * kLevel ? 0.f : x; }
+// index in [i0, i1] nearest to that of the level ray, slopes r0 + i r1
+__device__ __forceinline__ int level_index(double r0, double r1, int i0, int i1) {
+    const float q = __fdividef((float)-r0, (float)r1);
+    return min(max((int)rintf(fminf(fmaxf(q, -1e9f), 1e9f)), i0), i1);
+}
+
 // Per ray (view, iv, iu) geometry for the backprojection:
 // {r_a hi, r_a lo, r_b hi, r_b lo}, {1 / r_a, 1 / r_b, seg, E_m}.
 __global__ void cone_ray_kernel(float4* __restrict__ rays, const ConeView* __restrict__ views, ConeDims cd) {
@@ -69,7 +84,10 @@ __global__ void cone_ray_kernel(float4* __restrict__ rays, const ConeView* __res
     double D[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) D[k] = V.C[k] + iu * V.Eu[k] + iv * V.Ev[k] - V.S[k];
-    const double Dm = D[V.m], ra = D[V.a] / Dm, rb = D[V.b] / Dm;
+    const double Dm = D[V.m];
+    double ra = D[V.a] / Dm, rb = D[V.b] / Dm;
+    if (fabs(ra) < kLevel) ra = 0.0;
+    if (fabs(rb) < kLevel) rb = 0.0;
     const double dm = cd.d[V.m], da = cd.d[V.a], db = cd.d[V.b];
     const double seg = sqrt(dm * dm + ra * ra * da * da + rb * rb * db * db);
     const float rah = (float)ra, rbh = (float)rb;
@@ -498,11 +516,12 @@ __device__ __forceinline__ bool bp_separable(float& acc, const ConeView& V, int 
     range(XB0, GB, rs_b, nj, j0, j1);
     if (i1 < i0 || j1 < j0) return true;
     if (i1 - i0 >= kSepMax || j1 - j0 >= kSepMax) return false;
-    // the first candidate's offsets in FP64, then steps in FP32
-    const float xa0 = (float)fma((double)i0, GA, XA0), xb0 = (float)fma((double)j0, GB, XB0);
+    // one candidate's offsets in FP64 (the level ray's, or the nearest to it), then steps in FP32
+    const int il = level_index(ra0, ra1, i0, i1), jl = level_index(rb0, rb1, j0, j1);
+    const float xa0 = snap_face((float)fma((double)il, GA, XA0)), xb0 = snap_face((float)fma((double)jl, GB, XB0));
     const float ga = (float)GA, gb = (float)GB;
     const float ra1f = (float)ra1, rb1f = (float)rb1;
-    const float rai_f = (float)(ra0 + i0 * ra1), rbj_f = (float)(rb0 + j0 * rb1);
+    const float rai_f = (float)(ra0 + il * ra1), rbj_f = (float)(rb0 + jl * rb1);
     // the segment's ends along m, relative to the voxel's low face
     const float e0 = (float)(-M), e1 = (float)(-M + V.Dm0);
     const float clo = fmaxf(0.f, fminf(e0, e1)), chi = fminf(1.f, fmaxf(e0, e1));
@@ -513,17 +532,17 @@ __device__ __forceinline__ bool bp_separable(float& acc, const ConeView& V, int 
     const int su = cd.nview * cd.nv * cd.nc, sv = cd.nc;
     const float* pview = pb + (long long)view * cd.nv * cd.nc;
     for (int j = j0; j <= j1; j++) {
-        const float kj = (float)(j - j0);
+        const float kj = (float)(j - jl);
         const float xb = fmaf(kj, gb, xb0), rb = fmaf(kj, rb1f, rbj_f);
-        const float ib = fabsf(rb) > 1e-30f ? __fdividef(1.f, rb) : 1e30f;
+        const float ib = level_inverse(rb);
         const float tb0 = -xb * ib, tb1 = (1.f - xb) * ib;
         const float lb = fmaxf(clo, fminf(tb0, tb1)), hb = fminf(chi, fmaxf(tb0, tb1));
         if (!(hb > lb)) continue;
         const float qb = fmaf(rb * rb, db2, dm2);
         for (int i = i0; i <= i1; i++) {
-            const float ki = (float)(i - i0);
+            const float ki = (float)(i - il);
             const float xa = fmaf(ki, ga, xa0), ra = fmaf(ki, ra1f, rai_f);
-            const float ia = fabsf(ra) > 1e-30f ? __fdividef(1.f, ra) : 1e30f;
+            const float ia = level_inverse(ra);
             const float ta0 = -xa * ia, ta1 = (1.f - xa) * ia;
             const float tl = fmaxf(lb, fminf(ta0, ta1)), th = fminf(hb, fmaxf(ta0, ta1));
             if (th > tl) {
@@ -629,29 +648,28 @@ __global__ void __launch_bounds__(256) cone_bp_sep_kernel(float* __restrict__ im
                   i1);
         sep_range(XV0, GV, -fmaxf(rv_s, 0.f) - 0.02f, 1.f - fminf(rv_s, 0.f) + 0.02f, cd.nv, j0, j1);
         if (!live) j1 = j0 - 1;
-        // this lane's V candidates: offsets from FP64 for the first, then
-        // FP32 steps
-        const float xv0 = (float)fma((double)j0, GV, XV0), gv = (float)GV;
-        const float rvj = (float)(rV0 + j0 * rV1), rv1f = (float)rV1;
+        // this lane's V candidates: offsets from FP64 for one (the level ray, or
+        // the nearest to it), then FP32 steps
+        const int jl = level_index(rV0, rV1, j0, j1);
+        const float xv0 = snap_face((float)fma((double)jl, GV, XV0)), gv = (float)GV;
+        const float rvj = (float)(rV0 + jl * rV1), rv1f = (float)rV1;
         const float* pview = pb + (long long)view * cd.nv * cd.nc;
         for (int base = i0; base <= i1; base += 32) {
             const int nk = min(32, i1 - base + 1);
             __syncwarp();
             if (lane < nk) {
                 const int i = base + lane;
-                const float xu = (float)fma((double)i, GU, XU0);
-                const float ru = (float)fma((double)i, rU1, rU0);
-                const float iru = fabsf(ru) > 1e-30f ? __fdividef(1.f, ru) : 1e30f;
+                const float xu = snap_face((float)fma((double)i, GU, XU0));
+                const float iru = level_inverse((float)fma((double)i, rU1, rU0));
                 const float t0 = -xu * iru, t1 = (1.f - xu) * iru, t2 = (2.f - xu) * iru;
                 s_t[warp][lane] = make_float4(fmaxf(clo, fminf(t0, t1)), fminf(chi, fmaxf(t0, t1)),
                                               fmaxf(clo, fminf(t1, t2)), fminf(chi, fmaxf(t1, t2)));
                 s_i[warp][lane] = i;
             }
             __syncwarp();
-            float kj = 0.f;
+            float kj = (float)(j0 - jl);
             for (int j = j0; j <= j1; j++, kj += 1.f) {
-                const float xv = fmaf(kj, gv, xv0), rv = fmaf(kj, rv1f, rvj);
-                const float irv = fabsf(rv) > 1e-30f ? __fdividef(1.f, rv) : 1e30f;
+                const float xv = fmaf(kj, gv, xv0), irv = level_inverse(fmaf(kj, rv1f, rvj));
                 const float tv0 = -xv * irv, tv1 = (1.f - xv) * irv;
                 const float lv = fminf(tv0, tv1), hv = fmaxf(tv0, tv1);
                 const float* pcol = pview + j * sv;
@@ -990,8 +1008,9 @@ int cone_views(rn_cone_plan* p, const RnConeGeom& g, const float* dc, const floa
             V.Ev[k] = (double)dv_[3 * iv + k] * g.dv / d[k];
             V.C[k] = ((double)dc[3 * iv + k] - u0 * g.du * du_[3 * iv + k] - v0 * g.dv * dv_[3 * iv + k] - cen[k]) / d[k] +
                      n[k] / 2.0;
-            V.Sh[k] = (float)V.S[k];
-            V.Sl[k] = (float)(V.S[k] - (double)V.Sh[k]);
+            const double fixed = std::rint(V.S[k] * 4294967296.0) / 4294967296.0;   // (kLevel)
+            V.Sh[k] = (float)fixed;
+            V.Sl[k] = (float)(fixed - (double)V.Sh[k]);
         }
         // main axis: the largest advance of the central ray, in voxels
         double Dc[3];

@@ -52,6 +52,8 @@ CASES = {
                        dict(n=4, lift=0.0, dcy=0.0), 1, 1),
     "level_row_and_column": (_geom(nx=32, ny=64, dy=1.0, cx=0.0, cy=0.0, nu=41, nv=81, off_u=0.0, off_v=0.0),
                              dict(n=1, lift=-7.0, dcx=0.0, dcy=-7.0), 1, 1),
+    "level_row_reversed_v": (_geom(nx=32, ny=32, dy=1.0, cx=0.0, cy=0.0, nu=41, nv=41, off_u=0.0, off_v=0.0),
+                             dict(n=1, lift=0.0, dcx=0.0, dcy=0.0, flip=(1.0, -1.0)), 1, 1),
     # outside the limits: a reversed axis, cells under 0.3 voxels, slopes over one
     "reversed_v": (_geom(), dict(n=3, flip=(1.0, -1.0)), 1, 1),
     "very_fine": (_geom(nu=90, nv=91, du=0.25, dv=0.25), dict(n=2), 1, 1),
