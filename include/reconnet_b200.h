@@ -315,6 +315,10 @@ int rn_cone_plan_destroy(rn_cone_plan* plan);
  * 0 overwrites img, 1 adds to it), device pointers, on `stream`. */
 int rn_cone_project(rn_cone_plan* plan, float* d_prj, const float* d_img, void* stream);
 int rn_cone_backproject(rn_cone_plan* plan, float* d_img, const float* d_prj, int accumulate, void* stream);
+/* Which kernels a plan uses, forward and back: 0 the plan's own choice (as made), 1
+ * the general ones, 2 those of its geometry's family (upright or tomosynthesis;
+ * RN_ERR_ARG where it has none).  Between calls only. */
+int rn_cone_plan_set_route(rn_cone_plan* plan, int fp, int bp, void* stream);
 long long rn_cone_plan_launches(const rn_cone_plan* plan);
 
 /* replaces ReconNet4D/SiddonCone.cu:126-201 (host pointers; prj overwritten) */

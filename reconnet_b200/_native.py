@@ -92,6 +92,7 @@ SIGNATURES = {
     "rn_cone_plan_destroy": (_i, [_vp]),
     "rn_cone_project": (_i, [_vp, _vp, _vp, _vp]),
     "rn_cone_backproject": (_i, [_vp, _vp, _vp, _i, _vp]),
+    "rn_cone_plan_set_route": (_i, [_vp, _i, _i, _vp]),
     "rn_cone_plan_launches": (ctypes.c_longlong, [_vp]),
     "cSiddonConeProjectionAbitrary": (None, [_fp] * 6 + _TOMO),
     "cSiddonConeBackprojectionAbitrary": (None, [_fp] * 6 + _TOMO),

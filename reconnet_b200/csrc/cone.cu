@@ -980,12 +980,14 @@ struct rn_cone_plan {
     bool bp_sep = false;       // every view separable the same way (cone_bp_sep_kernel)
     ConeView h_view0;          // host copy of view 0 (axes of a separable plan)
     bool unit = true;          // every ray's lateral slopes are at most 1
-    bool col = false;          // upright detectors: the kernels of cone_col.cu
+    bool col = false;          // upright detectors: the kernels of cone_col.cu can take the plan
     bool col_one = false;      // (their single-crossing form)
     ColView* d_col = nullptr;
-    bool tile = false;         // tomosynthesis: the kernels of cone_tile.cu
+    bool tile = false;         // tomosynthesis: the kernels of cone_tile.cu can
     TilePlan tp;
     TileView* d_tile = nullptr;
+    bool own_fp = false, own_bp = false;         // whether they do
+    bool choice_fp = false, choice_bp = false;   // the rule's answers (cone_routes)
     std::unique_ptr<ConeScratch> scratch{new ConeScratch};
     long long launches = 0;
 };
@@ -1109,9 +1111,71 @@ int cone_views(rn_cone_plan* p, const RnConeGeom& g, const float* dc, const floa
 }
 
 size_t cone_bp_scratch_bytes(const rn_cone_plan* p) {
-    if (p->col) return cone_col_table_bytes(p->cd);
-    if (p->tile) return cone_tile_bp_bytes(p->cd);
+    if (p->col && p->own_bp) return cone_col_table_bytes(p->cd);
+    if (p->tile && p->own_bp) return cone_tile_bp_bytes(p->cd);
     return p->bp_sep ? sizeof(float) * p->cd.nb * p->cd.prj_b : 0;
+}
+
+// Whether a plan that cone_tile.cu's or cone_col.cu's kernels can take goes to them:
+// by estimates of both sides' times (us), fitted to measurements.  The general
+// kernels work per ray or voxel and fill the GPU early; the others share work
+// within blocks of rays or voxels that walk the planes or the views one after
+// another, which pays where there are enough of them (or, with many planes and few
+// views, long enough runs).
+void cone_routes(rn_cone_plan* p, const ConeView& v0, const std::vector<ColView>& col) {
+    const ConeDims& cd = p->cd;
+    const double slices = (double)cd.nb * cd.nc, nx = cd.n[0], ny = cd.n[1], nz = cd.n[2], V = cd.nview;
+    auto blocks = [](int n, int t) { return (double)((n + t - 1) / t); };
+    if (p->tile) {
+        // Forward: 203 grids of 32^2 to 512^2 x 1 to 48 voxels, 3 to 200 views of 8^2 to
+        // 500^2 cells: the better side to 0.5% on average, 27% off at worst, where the
+        // tiles alone take up to 5.3 times as long as the better side.
+        const double rays = (double)cd.nu * cd.nv * V;
+        const double met = std::min<double>(cd.nu, nx / p->tp.gu) * std::min<double>(cd.nv, ny / p->tp.gv) * V;
+        const double general = 9 + slices * (25e-6 * rays + met * (15e-6 + 1.75e-6 * nz));
+        double wave = 1.6 * blocks(cd.nu, 32) * blocks(cd.nv, 64) * V / 444;
+        if (cone_tile_big(cd, p->tp)) wave = 3.1 * blocks(cd.nu, 64) * blocks(cd.nv, 128) * V / 444;
+        p->choice_fp = slices * (12 + nz * std::max(1.05, wave)) < general;
+        // Back: a tile and view take 9 to 13 us whatever the tiles' number, up to three per
+        // SM; the same grids: the better side within 5% from half of that on, the tiles
+        // up to 6 times as slow below.
+        p->choice_bp = blocks(cd.n[0], 32) * blocks(cd.n[1], 64) * blocks(cd.n[2], 4) >= 222;
+    } else if (p->col) {
+        // ray and row spacing at the grid's centre, voxels
+        const ColView& q = col[0];
+        const int m = v0.m;
+        const double share = std::fabs((cd.n[m] / 2.0 - q.S[m]) / (q.D[m] + (cd.nu - 1) / 2.0 * q.E[m]));
+        const double gu = std::max(share * std::hypot(q.E[0], q.E[1]), 1e-3), gv = share * std::fabs(q.ez);
+        // Forward: warps of 32 rays of a column.  504 grids of 32^2 to 256^2 x 1 to 64
+        // voxels, 6 and 60 views of 64 x 1 to 300 x 64 cells: the better side to 1.2% on
+        // average, never slower than the general kernel, up to 35% slower than the columns
+        // (general up to 2.1 times as fast where it is taken, columns up to 3.3 times).
+        const double warps = slices * V * cd.nu * blocks(cd.nv, 32);
+        p->choice_fp = warps >= 4500 || (nz >= 32 && cd.nv >= 32);
+        // Back: a voxel's candidates against a pixel's, whose lateral work goes 32 views at
+        // a time.  The same grids: 1.2% on average, 40% at worst (general up to 6
+        // times as fast where it is taken, columns up to 6 times).
+        const double cells = 1 + 1.27 / gu, pixels = nx * ny, cover = std::min(1.0, cd.nu * gu / std::max(nx, ny));
+        const double rows = std::min(1.0, cd.nv * gv / nz), chunk = nz <= 32 ? 1 : nz <= 64 ? 1.4 : 1.9 * blocks(cd.n[2], 128);
+        const double own = 15 + pixels * chunk * cells *
+                                    (blocks(cd.nview, 32) * 2e-4 + V * 27e-6 * (0.3 + 0.7 * std::sqrt(cover)));
+        const double general = 9 + V * std::max(1.3, slices * pixels * nz * (4.5e-6 + 8e-6 * cells * cover * rows));
+        p->choice_bp = slices * own < general;
+    }
+    p->own_fp = p->choice_fp;
+    p->own_bp = p->choice_bp;
+}
+
+// What the plan's routes need on the device; rays: the general backprojection's table.
+cudaError_t cone_route_memory(rn_cone_plan* p, cudaStream_t st) {
+    const ConeDims& cd = p->cd;
+    p->scratch->reserve(std::max(p->own_bp ? cone_bp_scratch_bytes(p) : 0, p->tile && p->own_fp ? cone_tile_fp_bytes(cd) : 0));
+    if (p->d_rays || p->own_bp || p->tile) return cudaSuccess;
+    const long long nrays = (long long)cd.nview * cd.nv * cd.nu;
+    const cudaError_t e = cudaMalloc(&p->d_rays, sizeof(float4) * 2 * nrays);
+    if (e != cudaSuccess) return e;
+    cone_ray_kernel<<<(unsigned)((nrays + 255) / 256), 256, 0, st>>>(p->d_rays, p->d_views, cd);
+    return cudaGetLastError();
 }
 
 // cone_bp_sep_kernel on the projections times the segment lengths (prjw).
@@ -1192,7 +1256,6 @@ int rn_cone_plan_create(rn_cone_plan** out, const RnConeGeom* g, const float* ho
         p->h_view0 = views[0];
     }
     cudaStream_t st = (cudaStream_t)stream;
-    const long long nrays = (long long)g->nview * g->nv * g->nu;
     std::vector<ColView> col;
     std::vector<TileView> tiles;
     p->col = cone_col_views(views, cd, col, p->col_one);
@@ -1213,15 +1276,9 @@ int rn_cone_plan_create(rn_cone_plan** out, const RnConeGeom* g, const float* ho
         if (e == cudaSuccess) e = cudaMalloc(&p->d_tile, sizeof(TileView) * tiles.size());
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(p->d_tile, tiles.data(), sizeof(TileView) * tiles.size(), cudaMemcpyHostToDevice, st);
-    } else if (e == cudaSuccess) {
-        e = cudaMalloc(&p->d_rays, sizeof(float4) * 2 * nrays);
     }
-    if (e == cudaSuccess && p->d_rays) {
-        cone_ray_kernel<<<(unsigned)((nrays + 255) / 256), 256, 0, st>>>(p->d_rays, p->d_views, cd);
-        e = cudaGetLastError();
-    }
-    if (p->col || p->tile)
-        p->scratch->reserve(std::max(cone_bp_scratch_bytes(p), p->tile ? cone_tile_fp_bytes(cd) : 0));
+    cone_routes(p, views[0], col);
+    if (e == cudaSuccess) e = cone_route_memory(p, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // the host copies go out of scope
     if (e != cudaSuccess) {
         rn_cone_plan_destroy(p);
@@ -1247,11 +1304,11 @@ int rn_cone_project(rn_cone_plan* p, float* d_prj, const float* d_img, void* str
     const ConeDims& cd = p->cd;
     const long long nz = (long long)cd.nb * cd.nview * cd.nc;
     if (nz > 65535) return set_error(RN_ERR_ARG, "cone projection: more than 65535 views x batches x channels");
-    if (p->col) {
+    if (p->col && p->own_fp) {
         p->launches++;
         return cone_col_project(p->d_col, cd, d_prj, d_img, (cudaStream_t)stream);
     }
-    if (p->tile) {
+    if (p->tile && p->own_fp) {
         cudaStream_t st = (cudaStream_t)stream;
         ConeScratch::Hold vol;
         RN_TRY(p->scratch->get(cone_tile_fp_bytes(cd), st, &vol));
@@ -1286,18 +1343,18 @@ int rn_cone_backproject(rn_cone_plan* p, float* d_img, const float* d_prj, int a
     const long long nvox = (long long)cd.n[0] * cd.n[1] * cd.n[2];
     const int slices = cd.nb * cd.nc;
     if (slices > 65535) return set_error(RN_ERR_ARG, "cone backprojection: too many batches x channels");
-    if (p->col || p->tile || p->bp_sep) {
+    if (p->own_bp || p->bp_sep) {
         cudaStream_t st = (cudaStream_t)stream;
-        if (p->bp_sep && !p->tile && (cd.nu > 65535 || cd.nview > 65535))
+        if (!p->own_bp && (cd.nu > 65535 || cd.nview > 65535))
             return set_error(RN_ERR_ARG, "cone backprojection: more than 65535 detector columns or views");
         ConeScratch::Hold h;
         RN_TRY(p->scratch->get(cone_bp_scratch_bytes(p), st, &h));
         if (!h.ptr) return set_cuda_error(cudaErrorMemoryAllocation, "cone backprojection: scratch");
         int s = RN_OK;
-        if (p->col) {
+        if (p->own_bp && p->col) {
             p->launches += 2LL * slices;
             s = cone_col_backproject(p->d_col, cd, p->col_one, static_cast<double*>(h.ptr), d_img, d_prj, accumulate, st);
-        } else if (p->tile) {
+        } else if (p->own_bp) {
             p->launches += 2LL * slices;
             s = cone_tile_backproject(p->d_tile, cd, p->tp, static_cast<float*>(h.ptr), d_img, d_prj, accumulate, st);
         } else {
@@ -1312,6 +1369,19 @@ int rn_cone_backproject(rn_cone_plan* p, float* d_img, const float* d_prj, int a
     p->launches++;
     RN_CUDA_TRY(cudaGetLastError());
     return RN_OK;
+}
+
+int rn_cone_plan_set_route(rn_cone_plan* p, int fp, int bp, void* stream) {
+    clear_error();
+    if (!p || fp < 0 || fp > 2 || bp < 0 || bp > 2) return set_error(RN_ERR_ARG, "cone route: 0, 1 or 2");
+    if ((fp == 2 || bp == 2) && !p->col && !p->tile)
+        return set_error(RN_ERR_ARG, "cone route: the geometry has only the general kernels");
+    p->own_fp = fp == 0 ? p->choice_fp : fp == 2;
+    p->own_bp = bp == 0 ? p->choice_bp : bp == 2;
+    const cudaError_t e = cone_route_memory(p, (cudaStream_t)stream);
+    if (e == cudaSuccess) return RN_OK;
+    p->own_bp = true;   // (no room for the general backprojection's table)
+    return set_cuda_error(e, "rn_cone_plan_set_route");
 }
 
 long long rn_cone_plan_launches(const rn_cone_plan* p) { return p ? p->launches : 0; }

@@ -72,11 +72,14 @@ struct TileView {
 };
 struct TilePlan {
     bool fp_narrow = false;        // rays under a voxel apart
+    double gu = 1, gv = 1;         // widest ray spacing, voxels
     int kv = 0;                    // rows of rays that can meet one voxel
     int bp_patch = 0, bp_smem = 0; // floats of a backprojection patch, shared memory of a block
 };
 // Fills `out` and `tp` where the tile kernels can take the plan (false otherwise).
 bool cone_tile_views(const std::vector<ConeView>& views, const ConeDims& cd, std::vector<TileView>& out, TilePlan& tp);
+// whether the forward projection goes in tiles of 64 x 128 rays (else 32 x 64)
+bool cone_tile_big(const ConeDims& cd, const TilePlan& tp);
 int cone_tile_attributes();
 size_t cone_tile_fp_bytes(const ConeDims& cd);
 size_t cone_tile_bp_bytes(const ConeDims& cd);

@@ -586,6 +586,8 @@ bool cone_tile_views(const std::vector<ConeView>& views, const ConeDims& cd, std
     if (8LL * tp.bp_patch > kBpTileSmemWide) return false;
     tp.bp_smem = 8 * tp.bp_patch > kBpTileSmem ? kBpTileSmemWide : kBpTileSmem;
     tp.fp_narrow = gu_hi <= kTileNarrow && gv_hi <= kTileNarrow;
+    tp.gu = gu_hi;
+    tp.gv = gv_hi;
     return true;
 }
 
@@ -613,13 +615,15 @@ size_t cone_tile_bp_bytes(const ConeDims& cd) {
     return sizeof(float) * (size_t)cd.nview * cd.nu * ((cd.nv + 3) & ~3);
 }
 
+// Tiles of 64 x 128 rays for rays under a voxel apart where they fill the GPU.
+bool cone_tile_big(const ConeDims& cd, const TilePlan& tp) {
+    return tp.fp_narrow && (long long)((cd.nu + 63) / 64) * ((cd.nv + 127) / 128) * cd.nview >= 3 * 148;
+}
+
 int cone_tile_project(const TileView* d_views, const ConeDims& cd, const TilePlan& tp, float* d_vol, float* d_prj,
                       const float* d_img, cudaStream_t st) {
     const int pitch = (cd.n[1] + 3) & ~3;
-    // 64 x 128-ray tiles for rays under a voxel apart where they fill the GPU,
-    // else 32 x 64
-    const bool big = tp.fp_narrow &&
-                     (long long)((cd.nu + 63) / 64) * ((cd.nv + 127) / 128) * cd.nview >= 3 * 148;
+    const bool big = cone_tile_big(cd, tp);
     for (int b = 0; b < cd.nb; b++)
         for (int c = 0; c < cd.nc; c++) {
             cone_planes_kernel<<<dim3((pitch + 31) / 32, (cd.n[2] + 31) / 32, std::min(cd.n[0], 64)), dim3(32, 8), 0,

@@ -402,6 +402,12 @@ class ConePlan:
                                           _stream_ptr(prj.device)))
         return out
 
+    def set_route(self, fp: str = "auto", bp: str = "auto") -> None:
+        """Kernels of the forward and back projection: "auto" the plan's own choice, "general", or "own", those of
+        its geometry's family (upright detectors, tomosynthesis)."""
+        ways = ("auto", "general", "own")
+        N.check(N.lib.rn_cone_plan_set_route(self._plan, ways.index(fp), ways.index(bp), _stream_ptr(self.device)))
+
     def launches(self) -> int:
         return int(N.lib.rn_cone_plan_launches(self._plan))
 
