@@ -396,6 +396,7 @@ bool cone_col_views(const std::vector<ConeView>& views, const ConeDims& cd, std:
     one = true;
     const double nx = cd.n[0], ny = cd.n[1], nz = cd.n[2];
     if ((long long)cd.nview * cd.nu > 0x7fffffff || (long long)cd.nview * cd.nb * cd.nc > 65535) return false;
+    if (cd.n[1] > 2 * 65535 || cd.n[2] > 32 * 65535) return false;   // the grid's y and z
     for (const ConeView& v : views) {
         if (v.m == 2 || v.Ev[0] != 0.0 || v.Ev[1] != 0.0 || v.Eu[2] != 0.0 || v.Ev[2] == 0.0) return false;
         ColView q;

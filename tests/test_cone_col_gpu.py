@@ -122,3 +122,17 @@ def test_column_backprojection_on_two_streams(rng):
     torch.cuda.synchronize()
     for k in range(2):
         assert all(torch.equal(o, want[k]) for o in outs[k])
+
+
+def test_more_rows_of_pixels_than_a_grid_holds(rng):
+    """131072 pixels along y are more blocks than a launch takes along one axis."""
+    import torch
+    from oracle import oracle as O
+    from reconnet_b200.torch_ops import ConeGeometry, ConePlan
+    g = _geom(nx=2, ny=131072, nz=1, dx=1e-3, dy=1e-3, dz=1e-3, cx=0.0, cy=0.0, cz=0.0, nu=140, nv=1, du=1.3, dv=1.2,
+              off_u=0.0, off_v=0.0)
+    geo = _orbit(1, start=0.0)
+    plan = ConePlan(ConeGeometry(**g), *geo)
+    y = rng.random(plan.prj_shape).astype(np.float32)
+    got = plan.backproject(torch.from_numpy(y).cuda()).cpu().numpy()
+    assert rel_l2(got, O.cone_bp(y, *geo, NS(**g), (2, 131072, 1))) <= TOL
