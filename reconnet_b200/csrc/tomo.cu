@@ -96,13 +96,24 @@ __device__ __forceinline__ int tomo_fp_class(const TomoDims& d, const float* dc,
     return hi <= kTomoNarrow ? 2 : 3;
 }
 
-// Whether some view of the call has one of the classes in `mask` (bit k: class
-// k).  All threads of the block take part.
-__device__ __forceinline__ bool tomo_fp_any(const TomoDims& d, const float* dc, const float* sp, int mask) {
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x, n = blockDim.x * blockDim.y;
-    int hit = 0;
-    for (int v = tid; v < d.nview; v += n) hit |= (mask >> tomo_fp_class(d, dc + 3 * v, sp + 3 * v)) & 1;
-    return __syncthreads_or(hit) != 0;
+// Which kernels a call needs, decided once per call by a kernel of its own (in the
+// others the test costs 2 to 4 us each, and registers) and kept in the scratch's first double.  That entry of the tables
+// is zero, so the word keeps its meaning while they are built:
+//   forward: 4 and / or 8 where every view has class 2 or 3 (the tile kernels), 0 where
+//     every view has class 0 (the tables), -0.0 where only some have (both);
+//   back: the call's class and patch, or 0 (the tables).
+constexpr unsigned long long kTomoMixed = 1ull << 63;
+__device__ __forceinline__ unsigned long long tomo_word(const double* sat) {
+    return *reinterpret_cast<const volatile unsigned long long*>(sat);
+}
+
+__global__ void __launch_bounds__(128) tomo_fp_decide(double* sat, const float* __restrict__ detCenter,
+                                                      const float* __restrict__ src, TomoDims d) {
+    int found = 0;
+    for (int v = threadIdx.x; v < d.nview; v += 128) found |= 1 << tomo_fp_class(d, detCenter + 3 * v, src + 3 * v);
+    const bool c0 = __syncthreads_or(found & 1), c2 = __syncthreads_or(found & 4), c3 = __syncthreads_or(found & 8);
+    if (threadIdx.x == 0)
+        *reinterpret_cast<unsigned long long*>(sat) = c0 ? (c2 || c3 ? kTomoMixed : 0ull) : (c2 ? 4ull : 0ull) | (c3 ? 8ull : 0ull);
 }
 
 // Overlaps of an interval that starts a fraction f into a unit cell and is
@@ -207,10 +218,8 @@ __device__ __forceinline__ double tomo_len_weight(const float* dc, const float* 
 // y fastest, pitch = ny rounded up to 4, the padding zero.  32 x 32 (y, z)
 // tiles through shared memory.  Block (32, 8): blockIdx = (y tile, z tile, x).
 __global__ void __launch_bounds__(256) tomo_planes_kernel(float* __restrict__ vol, const float* __restrict__ img,
-                                                          const float* __restrict__ detCenter,
-                                                          const float* __restrict__ src, TomoDims d, int pitch, int b,
-                                                          int c) {
-    if (!tomo_fp_any(d, detCenter, src, 12)) return;   // no view for the tile kernels
+                                                          const double* sat, TomoDims d, int pitch, int b, int c) {
+    if (tomo_word(sat) == 0) return;   // no view for the tile kernels
     __shared__ float tile[32][33];
     const int y0 = blockIdx.x * 32, z0 = blockIdx.y * 32;
     const int lane = threadIdx.x, w = threadIdx.y;
@@ -251,8 +260,9 @@ constexpr int kTomoTileSmem = 70 * 1024;   // with the static tables, three bloc
 
 template <int K, int UPW, int NP>
 __global__ void __launch_bounds__(128, 3)
-    tomo_fp_tile_kernel(float* __restrict__ prj, const float* __restrict__ vol, const float* __restrict__ detCenter,
-                        const float* __restrict__ src, TomoDims d, int pitch, int b, int c, int all) {
+    tomo_fp_tile_kernel(float* __restrict__ prj, const float* __restrict__ vol, const double* sat,
+                        const float* __restrict__ detCenter, const float* __restrict__ src, TomoDims d, int pitch, int b,
+                        int c, int all) {
     constexpr int TU = 4 * UPW, TV = 64 * NP;
     constexpr double kWidest = K == 2 ? kTomoNarrow : kTomoWide;
     constexpr int kMaxRows = (int)(TU * kWidest) + K + 2, kMaxPitch = ((int)(TV * kWidest) + K + 2 + 6) & ~3;
@@ -262,7 +272,8 @@ __global__ void __launch_bounds__(128, 3)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int u0 = blockIdx.y * TU, v0 = blockIdx.x * TV;
     const int uw = u0 + warp * UPW;
-    if (!all && !tomo_fp_any(d, detCenter, src, 1 << K)) return;
+    const unsigned long long word = tomo_word(sat);
+    if (word == 0 || (!all && word != kTomoMixed && !((word >> K) & 1))) return;
     for (int view = blockIdx.z; view < d.nview; view += gridDim.z) {
         const float* dc = detCenter + 3 * view;
         const float* sp = src + 3 * view;
@@ -443,8 +454,9 @@ __device__ __forceinline__ int2 tomo_bp_patch(const TomoDims& d, const TomoBpGeo
 }
 
 // How many cells a voxel's footprint can touch per axis in this view: 3 (at
-// most 2 cells wide), 4 (at most 3), or 0 where the tile kernel does not apply.
-__device__ __forceinline__ int tomo_bp_class(const TomoDims& d, const float* dc, const float* sp, int2& patch) {
+// most 2 cells wide), 4 (at most 3), or 0 where the tile kernel does not apply;
+// its patch, in floats, for either kernel's tile.
+__device__ __forceinline__ int tomo_bp_class(const TomoDims& d, const float* dc, const float* sp, int& patch3, int& patch4) {
     const TomoBpGeo g = tomo_bp_geo(d, dc, sp);
     const double r0 = tomo_bp_r(d, g, 0), r1 = tomo_bp_r(d, g, d.nz - 1);
     const double rlo = fmin(r0, r1), rhi = fmax(r0, r1);
@@ -457,44 +469,32 @@ __device__ __forceinline__ int tomo_bp_class(const TomoDims& d, const float* dc,
     if (!(ue < 1e6 && ve < 1e6)) return 0;
     const double step = d.nz < 2 ? 0.0
                                  : fmax(fabs(tomo_bp_r(d, g, 1) - r0), fabs(r1 - tomo_bp_r(d, g, d.nz - 2)));
-    patch = hi <= 2.0 ? tomo_bp_patch<3>(d, g, rhi, step) : tomo_bp_patch<4>(d, g, rhi, step);
-    if ((long long)patch.x * patch.y * 8 > kTomoBpSmem) return 0;
+    const int2 p3 = tomo_bp_patch<3>(d, g, rhi, step), p4 = tomo_bp_patch<4>(d, g, rhi, step);
+    patch3 = p3.x * p3.y;
+    patch4 = p4.x * p4.y;
     return hi <= 2.0 ? 3 : 4;
 }
 
-// The class of the whole call: 0 if some view has class 0, else the largest
-// (a class's kernel also serves the narrower footprints of its own tile, so
-// every view's patch is taken for that tile); `patch` = the largest patch in
-// floats.  All threads of the block take part.
-__device__ __forceinline__ int tomo_bp_call_class(const TomoDims& d, const float* dc, const float* sp, int& patch) {
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x, n = blockDim.x * blockDim.y;
-    int any0 = 0, any4 = 0;
-    for (int v = tid; v < d.nview; v += n) {
-        int2 p;
-        const int k = tomo_bp_class(d, dc + 3 * v, sp + 3 * v, p);
-        any0 |= k == 0;
-        any4 |= k == 4;
+// The class of the whole call: 0 if some view has class 0 or a patch that does not
+// fit twice, else the largest (a class's kernel also serves the narrower footprints,
+// on its own tile), in the word's low byte; above it the largest patch in floats.
+__global__ void __launch_bounds__(128) tomo_bp_decide(double* sat, const float* __restrict__ detCenter,
+                                                      const float* __restrict__ src, TomoDims d) {
+    __shared__ int s_patch[2];
+    if (threadIdx.x < 2) s_patch[threadIdx.x] = 0;
+    __syncthreads();
+    int found = 0;   // bit k: a view of class k
+    for (int v = threadIdx.x; v < d.nview; v += 128) {
+        int p3 = 0, p4 = 0;
+        found |= 1 << tomo_bp_class(d, detCenter + 3 * v, src + 3 * v, p3, p4);
+        atomicMax(&s_patch[0], p3);
+        atomicMax(&s_patch[1], p4);
     }
-    if (__syncthreads_or(any0)) return 0;
-    const bool four = __syncthreads_or(any4) != 0;
-    __shared__ int s_patch;
-    if (tid == 0) s_patch = 0;
-    __syncthreads();
-    int most = 0;
-    for (int v = tid; v < d.nview; v += n) {
-        const TomoBpGeo g = tomo_bp_geo(d, dc + 3 * v, sp + 3 * v);
-        const double r0 = tomo_bp_r(d, g, 0), r1 = tomo_bp_r(d, g, d.nz - 1);
-        const double step = d.nz < 2 ? 0.0
-                                     : fmax(fabs(tomo_bp_r(d, g, 1) - r0), fabs(r1 - tomo_bp_r(d, g, d.nz - 2)));
-        const int2 p = four ? tomo_bp_patch<4>(d, g, fmax(r0, r1), step) : tomo_bp_patch<3>(d, g, fmax(r0, r1), step);
-        most = max(most, p.x * p.y);
-    }
-    atomicMax(&s_patch, most);
-    __syncthreads();
-    patch = s_patch;
-    __syncthreads();
-    if ((long long)patch * 8 > kTomoBpSmem) return 0;
-    return four ? 4 : 3;
+    const bool any0 = __syncthreads_or(found & 1) != 0, four = __syncthreads_or(found & 16) != 0;
+    const long long patch = s_patch[four];
+    if (threadIdx.x == 0)
+        *reinterpret_cast<unsigned long long*>(sat) =
+            any0 || patch * 8 > kTomoBpSmem ? 0ull : (unsigned long long)(patch << 8 | (four ? 4 : 3));
 }
 
 // Length-weighted projections of one (b, c) in rows of v, wp[view][u][pitch]
@@ -504,10 +504,12 @@ __device__ __forceinline__ int tomo_bp_call_class(const TomoDims& d, const float
 // along v; blockIdx = (v, u / kTomoWeightRows, view).
 constexpr int kTomoWeightRows = 8;
 __global__ void __launch_bounds__(256) tomo_weight_kernel(float* __restrict__ wp, double* __restrict__ rt,
-                                                          double* __restrict__ geo, const float* __restrict__ prj,
+                                                          double* __restrict__ geo, const double* sat,
+                                                          const float* __restrict__ prj,
                                                           const float* __restrict__ detCenter,
                                                           const float* __restrict__ src, TomoDims d, int pitch, int b,
                                                           int c, int weight_all) {
+    if (tomo_word(sat) == 0) return;
     const int view = blockIdx.z, u0 = blockIdx.y * kTomoWeightRows, iv = blockIdx.x * 256 + threadIdx.x;
     const float* dc = detCenter + 3 * view;
     const float* sp = src + 3 * view;
@@ -561,15 +563,15 @@ __global__ void __launch_bounds__(256) tomo_weight_kernel(float* __restrict__ wp
 template <int K>
 __global__ void __launch_bounds__(128, 3)
     tomo_bp_tile_kernel(float* __restrict__ img, const float* __restrict__ wp, const double* __restrict__ rt,
-                        const double* __restrict__ geo, const float* __restrict__ detCenter,
-                        const float* __restrict__ src, TomoDims d, int pitch, int b, int c) {
+                        const double* __restrict__ geo, const double* sat, TomoDims d, int pitch, int b, int c) {
     constexpr int XPW = TomoBpTile<K>::xpw, NP = TomoBpTile<K>::ypl / 2, TZ = TomoBpTile<K>::tz;
     constexpr int TX = 4 * XPW, TY = 64 * NP;
     extern __shared__ __align__(16) float smem[];
     __shared__ __align__(16) WalkTaps<K> s_ut[4][XPW * TZ];   // per warp; rewritten after the next barrier
     __shared__ int4 s_win[4];   // per slot: first u, first v (a multiple of 4), columns (a multiple of 4)
-    int patch;
-    if (tomo_bp_call_class(d, detCenter, src, patch) != K) return;
+    const unsigned long long word = tomo_word(sat);
+    if ((word & 255) != K) return;
+    const int patch = (int)(word >> 8);
     const int S = min(4, kTomoBpSmem / (4 * patch));   // >= 2
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ntx = (d.nx + TX - 1) / TX, nty = (d.ny + TY - 1) / TY, ntz = (d.nz + TZ - 1) / TZ;
@@ -710,6 +712,15 @@ __global__ void __launch_bounds__(128, 3)
 }
 
 // ---------------------------------------------------------------------------
+// Table kernels: the calls and views that the tiles leave out.  Whether a call needs
+// them they read in its word, so their grids are no larger than the GPU holds and
+// walk their work.  (Blocks per SM are bounded from below because the compiler
+// otherwise trades them for registers: with two instead of four the backprojection
+// of 300 x 300 x 64 voxels from 25 views took 527 us, 457 now, 436 with a block per
+// tile and no word to read; the forward projection of 25 views of 400 x 400 cells takes
+// 1065 with eight, and took 774 with a block per 31 x 4 cells and neither word nor
+// classes to read, which as many blocks cost every other call.)
+//
 // Tables (FP64).  FP: per z plane, row prefixes along x of image row y,
 // layout [z][y + 1][x] (x fastest, x in [0, nx]); a rectangle integral is the
 // sum over the rows it overlaps (rows_integral), which equals the reference's
@@ -725,12 +736,10 @@ __global__ void __launch_bounds__(128, 3)
 
 // Row prefixes R[z][y + 1][x + 1] = sum_{x' <= x} img[x'][y][z].  Block
 // (32, 8): blockIdx.x = y, blockIdx.y = a tile of 32 planes.
-// `mask`: build only if some view has one of these classes (the views that
-// tomo_fp_kernel projects).
-__global__ void __launch_bounds__(256) tomo_sat_x(double* __restrict__ sat, const float* __restrict__ img,
-                                                  const float* __restrict__ detCenter, const float* __restrict__ src,
-                                                  TomoDims d, int mask, int b, int c) {
-    if (!tomo_fp_any(d, detCenter, src, mask)) return;
+// `tiled`: only if the call's word (left as it is, a zero) asks for the tables.
+__global__ void __launch_bounds__(256) tomo_sat_x(double* __restrict__ sat, const float* __restrict__ img, TomoDims d,
+                                                  int tiled, int b, int c) {
+    if (tiled && (tomo_word(sat) & ~kTomoMixed)) return;
     __shared__ float tile[32][33];
     const int y = blockIdx.x, z0 = blockIdx.y * 32;
     const int lane = threadIdx.x, w = threadIdx.y;
@@ -760,7 +769,8 @@ __global__ void __launch_bounds__(256) tomo_sat_x(double* __restrict__ sat, cons
     if (w == 0 && z < d.nz) sat[z * plane + (y + 1) * row] = 0.0;
     if (y == 0)
         for (int zz = w; zz < 32 && z0 + zz < d.nz; zz += 8)
-            for (int x = lane; x <= d.nx; x += 32) sat[(z0 + zz) * plane + x] = 0.0;
+            for (int x = lane; x <= d.nx; x += 32)
+                if (!tiled || z0 + zz > 0 || x > 0) sat[(z0 + zz) * plane + x] = 0.0;
 }
 
 // Weighted row prefixes R[view][v + 1][u + 1] = sum_{u' <= u} w p(u', v).
@@ -772,8 +782,7 @@ __global__ void __launch_bounds__(256) tomo_bp_sat_u(double* __restrict__ sat, c
                                                      const float* __restrict__ detCenter,
                                                      const float* __restrict__ src, TomoDims d, int b, int c,
                                                      int weight_all, int tiled) {
-    int unused;
-    if (tiled && tomo_bp_call_class(d, detCenter, src, unused) != 0) return;
+    if (tiled && tomo_word(sat)) return;
     __shared__ double tile[32][33];
     const int v0 = blockIdx.x * 32, view = blockIdx.y;
     const int lane = threadIdx.x, w = threadIdx.y;
@@ -824,10 +833,8 @@ __global__ void __launch_bounds__(256) tomo_bp_sat_u(double* __restrict__ sat, c
 // this one only serves the calls whose class they leave out (likewise
 // tomo_bp_sat_u and tomo_bp_kernel).  Block (32, 4): blockIdx.x * 4 + warp = a
 // strip of 32 columns, blockIdx.y = view.
-__global__ void __launch_bounds__(128) tomo_bp_sat_v(double* __restrict__ sat, const float* __restrict__ detCenter,
-                                                     const float* __restrict__ src, TomoDims d, int tiled) {
-    int unused;
-    if (tiled && tomo_bp_call_class(d, detCenter, src, unused) != 0) return;
+__global__ void __launch_bounds__(128) tomo_bp_sat_v(double* __restrict__ sat, TomoDims d, int tiled) {
+    if (tiled && tomo_word(sat)) return;
     const int u = (blockIdx.x * 4 + threadIdx.y) * 32 + threadIdx.x;
     // the two pad entries after the last view's table (read with weight 0
     // by the backprojection's u + 1 neighbour at u = nu)
@@ -900,50 +907,49 @@ __device__ __forceinline__ double rows_integral(const double* __restrict__ R, co
 // overlaps, so the rectangle integral of a cell is D(next lane) - D(this
 // lane): two reads per overlapped row instead of the reference's 16 corner
 // reads.  The rectangle's area is (x_{e+1} - x_e)(y2 - y1) = drx dry
-// (z - sz)^2, exact for the straight edge rays.  Takes the views whose class
-// is in `mask`; a warp loops over them view by view.
-__global__ void __launch_bounds__(128) tomo_fp_kernel(float* __restrict__ prj, const double* __restrict__ sat,
+// (z - sz)^2, exact for the straight edge rays.
+__global__ void __launch_bounds__(128, 8) tomo_fp_kernel(float* __restrict__ prj, const double* __restrict__ sat,
                                                       const float* __restrict__ detCenter,
-                                                      const float* __restrict__ src, TomoDims d, int mask, int b,
+                                                      const float* __restrict__ src, TomoDims d, int tiled, int b,
                                                       int c) {
-    if (!tomo_fp_any(d, detCenter, src, mask)) return;
+    const unsigned long long word = tiled ? tomo_word(sat) : 0ull;
+    if (word & ~kTomoMixed) return;
     const int lane = threadIdx.x;
     const int nut = (d.nu + 30) / 31, nvt = (d.nv + blockDim.y - 1) / blockDim.y;
-    for (int iview = 0; iview < d.nview; iview++) {
+    for (long long job = blockIdx.x; job < (long long)nut * nvt * d.nview; job += gridDim.x) {
+        const int iview = (int)(job / (nut * nvt)), item = (int)(job - (long long)iview * (nut * nvt));
         const float* dc = detCenter + 3 * iview;
         const float* sp = src + 3 * iview;
-        if (!((mask >> tomo_fp_class(d, dc, sp)) & 1)) continue;
-        for (int item = blockIdx.x; item < nut * nvt; item += gridDim.x) {
-            const int iu = (item % nut) * 31 + lane;
-            const int iv = (item / nut) * blockDim.y + threadIdx.y;
-            if (iv >= d.nv) continue;   // warp-uniform
-            const float u = (iu - d.off_u - (d.nu - 1) / 2.0f) * d.du;
-            const float v = (iv - d.off_v - (d.nv - 1) / 2.0f) * d.dv;
-            auto img_x = [&](float px) { return (px - d.cx) / d.dx + d.nx / 2.0f; };
-            auto img_y = [&](float py) { return (py - d.cy) / d.dy + d.ny / 2.0f; };
-            auto img_z = [&](float pz) { return (pz - d.cz) / d.dz + d.nz / 2.0f; };
-            const float sx = img_x(sp[0]), sy = img_y(sp[1]), sz = img_z(sp[2]);
-            const float zd = img_z(dc[2]);
-            const float xe = img_x(dc[0] + u - d.du / 2);
-            const float ya = img_y(dc[1] + v - d.dv / 2), yb = img_y(dc[1] + v + d.dv / 2);
-            const float rxe = (xe - sx) / (zd - sz);
-            const float rya = (ya - sy) / (zd - sz), ryb = (yb - sy) / (zd - sz);
-            const float drx = __shfl_down_sync(0xffffffffu, rxe, 1) - rxe;   // signed, as are D and dry
-            const float k = 1.0f / (drx * (ryb - rya));
-            const long long plane = (long long)(d.nx + 1) * (d.ny + 1), row = d.nx + 1;
-            float val = 0.f;
-            for (int iz = 0; iz < d.nz; iz++) {
-                const float t = (float)iz - sz;
-                const Lerp lx = lerp_at(sx + rxe * t, d.nx + 1);
-                const double D = rows_integral(sat + iz * plane, lx, sy + rya * t, sy + ryb * t, d.ny, row);
-                const double q = __shfl_down_sync(0xffffffffu, D, 1) - D;
-                val = fmaf((float)q, __fdividef(k, t * t), val);
-            }
-            if (lane < 31 && iu < d.nu) {
-                val *= (float)tomo_len_weight(dc, sp, u, v, d.dz);
-                prj[(long long)b * d.nu * d.nview * d.nv * d.nc + ((long long)iu * d.nview + iview) * d.nv * d.nc +
-                    (long long)iv * d.nc + c] = val;
-            }
+        if (word && tomo_fp_class(d, dc, sp) != 0) continue;   // a call that has tiled views too
+        const int iu = (item % nut) * 31 + lane;
+        const int iv = (item / nut) * blockDim.y + threadIdx.y;
+        if (iv >= d.nv) continue;   // warp-uniform
+        const float u = (iu - d.off_u - (d.nu - 1) / 2.0f) * d.du;
+        const float v = (iv - d.off_v - (d.nv - 1) / 2.0f) * d.dv;
+        auto img_x = [&](float px) { return (px - d.cx) / d.dx + d.nx / 2.0f; };
+        auto img_y = [&](float py) { return (py - d.cy) / d.dy + d.ny / 2.0f; };
+        auto img_z = [&](float pz) { return (pz - d.cz) / d.dz + d.nz / 2.0f; };
+        const float sx = img_x(sp[0]), sy = img_y(sp[1]), sz = img_z(sp[2]);
+        const float zd = img_z(dc[2]);
+        const float xe = img_x(dc[0] + u - d.du / 2);
+        const float ya = img_y(dc[1] + v - d.dv / 2), yb = img_y(dc[1] + v + d.dv / 2);
+        const float rxe = (xe - sx) / (zd - sz);
+        const float rya = (ya - sy) / (zd - sz), ryb = (yb - sy) / (zd - sz);
+        const float drx = __shfl_down_sync(0xffffffffu, rxe, 1) - rxe;   // signed, as are D and dry
+        const float k = 1.0f / (drx * (ryb - rya));
+        const long long plane = (long long)(d.nx + 1) * (d.ny + 1), row = d.nx + 1;
+        float val = 0.f;
+        for (int iz = 0; iz < d.nz; iz++) {
+            const float t = (float)iz - sz;
+            const Lerp lx = lerp_at(sx + rxe * t, d.nx + 1);
+            const double D = rows_integral(sat + iz * plane, lx, sy + rya * t, sy + ryb * t, d.ny, row);
+            const double q = __shfl_down_sync(0xffffffffu, D, 1) - D;
+            val = fmaf((float)q, __fdividef(k, t * t), val);
+        }
+        if (lane < 31 && iu < d.nu) {
+            val *= (float)tomo_len_weight(dc, sp, u, v, d.dz);
+            prj[(long long)b * d.nu * d.nview * d.nv * d.nc + ((long long)iu * d.nview + iview) * d.nv * d.nc +
+                (long long)iv * d.nc + c] = val;
         }
     }
 }
@@ -963,12 +969,11 @@ __global__ void __launch_bounds__(128) tomo_fp_kernel(float* __restrict__ prj, c
 // voxel and view, all independent of one another.
 constexpr int kTomoBpRows = 8;
 
-__global__ void __launch_bounds__(256) tomo_bp_kernel(float* __restrict__ img, const double* __restrict__ sat,
+__global__ void __launch_bounds__(256, 4) tomo_bp_kernel(float* __restrict__ img, const double* __restrict__ sat,
                                                       const float* __restrict__ detCenter,
                                                       const float* __restrict__ src, TomoDims d, int b, int c,
                                                       int tiled) {
-    int unused;
-    if (tiled && tomo_bp_call_class(d, detCenter, src, unused) != 0) return;
+    if (tiled && tomo_word(sat)) return;
     // z runs fastest over the grid, so the CTAs resident at a time cover few
     // (x, y) columns and their detector footprints in all views stay in L2
     const int lane = threadIdx.x;
@@ -990,6 +995,7 @@ __global__ void __launch_bounds__(256) tomo_bp_kernel(float* __restrict__ img, c
         float acc[kTomoBpRows];
     #pragma unroll
         for (int j = 0; j < kTomoBpRows; j++) acc[j] = 0.f;
+#pragma unroll 2
         for (int view = 0; view < d.nview; view++) {
             const float* dc = detCenter + 3 * view;
             const float* sp = src + 3 * view;
@@ -1080,31 +1086,43 @@ int tomo_project(float* d_prj, const float* d_img, const float* d_dc, const floa
                  double* d_sat, cudaStream_t st) {
     RN_TRY(tomo_validate(d));
     RN_TRY(tomo_kernel_attributes());
-    // The plane-major copy lives where the prefix tables of the other views
-    // are built afterwards: nz nx pitch floats and 16 bytes of alignment fit
-    // in nz (nx + 1) (ny + 1) doubles.
-    float* vol = reinterpret_cast<float*>(align16(d_sat));
+    // After the call's word the plane-major copy, where the prefix tables of the other
+    // views are built afterwards (a volume of a few voxels has no room for it)
+    float* vol = reinterpret_cast<float*>(align16(d_sat + 1));
     const int pitch = (d.ny + 3) & ~3;
+    const int tiled = 24 + 4 * (size_t)d.nz * d.nx * pitch <= 8 * (size_t)d.nz * (d.nx + 1) * (d.ny + 1);
     // 64 x 128-cell tiles for footprints up to a voxel where they fill the
-    // GPU, else 32 x 64-cell tiles for all of them; a view loop in every
-    // kernel, so that those with nothing to do cost a small grid
+    // GPU, else 32 x 64-cell tiles for all of them.  What the classes leave to the
+    // kernels after the first is not known here: each gets blocks enough to fill the
+    // GPU, and its blocks walk the rest of the views, so that one with nothing to do
+    // costs little and one with all views is not held up.  (With each cell's views one
+    // after another, 60 views of 400 x 400 cells with footprints over a voxel took 2.60
+    // ms forward; 0.97 now.)
     const long long big = (long long)((d.nu + 63) / 64) * ((d.nv + 127) / 128) * d.nview;
     const bool use_big = big >= 3 * 148;
     const int views = std::min(d.nview, 65535);
+    const long long small = (long long)((d.nu + 31) / 32) * ((d.nv + 63) / 64);
+    const long long items = (long long)((d.nu + 30) / 31) * ((d.nv + 3) / 4);
+    // grid z: blocks of a view times this are about `want`
+    auto fill = [&](long long per_view, long long want) {
+        return (unsigned)std::min<long long>(views, (want + per_view - 1) / per_view);
+    };
+    if (tiled) tomo_fp_decide<<<1, 128, 0, st>>>(d_sat, d_dc, d_src, d);
     for (int b = 0; b < d.nb; b++)
         for (int c = 0; c < d.nc; c++) {
-            tomo_planes_kernel<<<dim3((pitch + 31) / 32, (d.nz + 31) / 32, std::min(d.nx, 16)), dim3(32, 8), 0, st>>>(
-                vol, d_img, d_dc, d_src, d, pitch, b, c);
-            if (use_big)
-                tomo_fp_tile_kernel<2, 16, 2><<<dim3((d.nv + 127) / 128, (d.nu + 63) / 64, views), 128,
-                                                      kTomoTileSmem, st>>>(d_prj, vol, d_dc, d_src, d, pitch, b, c, 0);
-            tomo_fp_tile_kernel<3, 8, 1><<<dim3((d.nv + 63) / 64, (d.nu + 31) / 32, use_big ? 1 : views), 128,
-                                                  kTomoTileSmem, st>>>(d_prj, vol, d_dc, d_src, d, pitch, b, c,
-                                                                       use_big ? 0 : 1);
-            tomo_sat_x<<<dim3(d.ny, (d.nz + 31) / 32), dim3(32, 8), 0, st>>>(d_sat, d_img, d_dc, d_src, d, 1, b, c);
-            const long long items = (long long)((d.nu + 30) / 31) * ((d.nv + 3) / 4);
-            tomo_fp_kernel<<<(unsigned)std::min<long long>(items, 148 * 16), dim3(32, 4), 0, st>>>(
-                d_prj, d_sat, d_dc, d_src, d, 1, b, c);
+            if (tiled) {
+                tomo_planes_kernel<<<dim3((pitch + 31) / 32, (d.nz + 31) / 32, std::min(d.nx, 16)), dim3(32, 8), 0, st>>>(
+                    vol, d_img, d_sat, d, pitch, b, c);
+                if (use_big)
+                    tomo_fp_tile_kernel<2, 16, 2><<<dim3((d.nv + 127) / 128, (d.nu + 63) / 64, views), 128, kTomoTileSmem,
+                                                    st>>>(d_prj, vol, d_sat, d_dc, d_src, d, pitch, b, c, 0);
+                tomo_fp_tile_kernel<3, 8, 1>
+                    <<<dim3((d.nv + 63) / 64, (d.nu + 31) / 32, use_big ? fill(small, 2 * 3 * 148) : views), 128,
+                       kTomoTileSmem, st>>>(d_prj, vol, d_sat, d_dc, d_src, d, pitch, b, c, use_big ? 0 : 1);
+            }
+            tomo_sat_x<<<dim3(d.ny, (d.nz + 31) / 32), dim3(32, 8), 0, st>>>(d_sat, d_img, d, tiled, b, c);
+            const unsigned grid = (unsigned)std::min<long long>(items * d.nview, 148 * 16);
+            tomo_fp_kernel<<<grid, dim3(32, 4), 0, st>>>(d_prj, d_sat, d_dc, d_src, d, tiled, b, c);
         }
     RN_CUDA_TRY(cudaGetLastError());
     return RN_OK;
@@ -1114,35 +1132,36 @@ int tomo_backproject(float* d_img, const float* d_prj, const float* d_dc, const 
                      double* d_sat, int weight_all, cudaStream_t st) {
     RN_TRY(tomo_validate(d));
     RN_TRY(tomo_kernel_attributes());
-    // weighted projections, then the magnifications, in the scratch of the
-    // summed-area tables (too small for them only where a detector of a few
-    // cells meets many planes)
+    // after the call's word the weighted projections, then the magnifications, in the
+    // scratch of the summed-area tables (too small for them only where a detector of a
+    // few cells meets many planes)
     const int pitch = (d.nv + 3) & ~3;
-    float* wp = reinterpret_cast<float*>(align16(d_sat));
+    float* wp = reinterpret_cast<float*>(align16(d_sat + 1));
     const size_t wp_bytes = (size_t)d.nview * d.nu * pitch * sizeof(float);
     double* rt = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(wp) + wp_bytes);
     double* geo = rt + (size_t)d.nview * d.nz;
     const size_t have = ((size_t)d.nview * (d.nu + 1) * (d.nv + 1) + 2) * 8;
-    const bool tiled = 16 + wp_bytes + (size_t)d.nview * (d.nz + 4) * 8 <= have && d.nview <= 65535 && d.nu <= 65535;
+    const bool tiled = 24 + wp_bytes + (size_t)d.nview * (d.nz + 4) * 8 <= have && d.nview <= 65535 && d.nu <= 65535;
     auto tiles = [&](int tx, int ty, int tz) {
         const long long n =
             (long long)((d.nx + tx - 1) / tx) * ((d.ny + ty - 1) / ty) * ((d.nz + tz - 1) / tz);
         return (unsigned)std::min<long long>(n, 0x7fffffff);
     };
+    if (tiled) tomo_bp_decide<<<1, 128, 0, st>>>(d_sat, d_dc, d_src, d);
     for (int b = 0; b < d.nb; b++)
         for (int c = 0; c < d.nc; c++) {
             if (tiled) {
                 tomo_weight_kernel<<<dim3((pitch + 255) / 256, (d.nu + kTomoWeightRows - 1) / kTomoWeightRows, d.nview), 256, 0,
                                      st>>>(
-                    wp, rt, geo, d_prj, d_dc, d_src, d, pitch, b, c, weight_all);
-                tomo_bp_tile_kernel<3><<<tiles(32, 64, 4), 128, kTomoBpSmem, st>>>(d_img, wp, rt, geo, d_dc, d_src, d,
-                                                                                  pitch, b, c);
+                    wp, rt, geo, d_sat, d_prj, d_dc, d_src, d, pitch, b, c, weight_all);
+                tomo_bp_tile_kernel<3><<<tiles(32, 64, 4), 128, kTomoBpSmem, st>>>(d_img, wp, rt, geo, d_sat, d, pitch, b,
+                                                                                  c);
                 tomo_bp_tile_kernel<4><<<std::min(tiles(16, 64, 4), 148u * 3), 128, kTomoBpSmem, st>>>(
-                    d_img, wp, rt, geo, d_dc, d_src, d, pitch, b, c);
+                    d_img, wp, rt, geo, d_sat, d, pitch, b, c);
             }
             tomo_bp_sat_u<<<dim3((d.nv + 31) / 32, d.nview), dim3(32, 8), 0, st>>>(d_sat, d_prj, d_dc, d_src, d, b,
                                                                                     c, weight_all, tiled);
-            tomo_bp_sat_v<<<dim3((d.nu + 1 + 127) / 128, d.nview), dim3(32, 4), 0, st>>>(d_sat, d_dc, d_src, d, tiled);
+            tomo_bp_sat_v<<<dim3((d.nu + 1 + 127) / 128, d.nview), dim3(32, 4), 0, st>>>(d_sat, d, tiled);
             tomo_bp_kernel<<<std::min(tiles(31, 8 * kTomoBpRows, 1), 148u * 8), dim3(32, 8), 0, st>>>(
                 d_img, d_sat, d_dc, d_src, d, b, c, tiled);
         }

@@ -97,3 +97,24 @@ def test_views_outside_the_limits(rng):
         fp, bp = _pair(img, prj, dc, src, g, 30, 36)
         assert rel_l2(fp, O.tomo_fp(img, dc, src, g, 30, 36)) <= 1e-5, over
         assert rel_l2(bp, O.tomo_bp(prj, dc, src, g, (21, 35, 6), 1)) <= 1e-5, over
+
+
+@pytest.mark.parametrize("over,near,tol", [(dict(du=1.1, dv=1.0), False, 1e-6), ({}, True, 1e-5),
+                                           (dict(du=2.6, dv=2.7), False, 1e-5)],
+                         ids=["all_three_taps", "mixed", "tables"])
+def test_other_classes_beside_wide_blocks(over, near, tol, rng):
+    """Calls large enough for the wide blocks whose views need the others' kernels: footprints over one voxel in every
+    view; narrow ones in most views and none for the tiles in some; the tables for all, in two batches."""
+    from oracle import oracle as O
+    dc, src = _views(50)
+    if near:
+        src[::7, 2] = 50.0    # magnified footprints, down to nothing for the tiles
+        src[3::7, 2] = -2.0   # the source between the planes
+    g = _grid(**over)
+    img = rng.random((2, 40, 45, 6, 1)).astype(np.float32)
+    prj = rng.random((2, 130, 50, 260, 1)).astype(np.float32)
+    fp, bp = _pair(img, prj, dc, src, g, 130, 260)
+    keep = np.arange(50) % 7 != 3   # a source between the planes is compared nowhere else either
+    assert rel_l2(fp[:, :, keep], O.tomo_fp(img, dc, src, g, 130, 260)[:, :, keep]) <= tol
+    if not near:
+        assert rel_l2(bp, O.tomo_bp(prj, dc, src, g, (40, 45, 6), 1)) <= tol
