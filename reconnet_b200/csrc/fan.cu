@@ -320,9 +320,13 @@ __device__ __forceinline__ int fp_ray_range(double ra, double rb, double par, do
     return (le > lb) ? (((int)lb << 16) | (int)le) : 0;
 }
 
-template <bool kSiddon>
+//
+// kSingle: every group of a work item has a warp of its own and stays alone (17
+// groups as 9 pairs on the 24 warps took 31 us for two slices of 256 x 256 and 31
+// views, 22 alone).
+template <bool kSiddon, bool kSingle = false>
 __global__ void __launch_bounds__(FpCfg<kSiddon>::threads, 1) fan_fp_kernel(FpParams p) {
-    constexpr int kFpThreads = FpCfg<kSiddon>::threads, kFpGroups = FpCfg<kSiddon>::groups;
+    constexpr int kFpThreads = FpCfg<kSiddon>::threads, kFpGroups = kSingle ? 2 : FpCfg<kSiddon>::groups;
     constexpr int kFpWarps = FpCfg<kSiddon>::warps;
     extern __shared__ __align__(128) unsigned char smem[];
     const int4 w = p.work[blockIdx.x];
@@ -394,12 +398,13 @@ __global__ void __launch_bounds__(FpCfg<kSiddon>::threads, 1) fan_fp_kernel(FpPa
     // view and first ray of slot k (warp-uniform but for the lane); view -1
     // where the slot is empty
     auto slot_view = [&](int k) {
-        if (kSiddon) return warp + k * kFpWarps < vcount * ngpv ? (warp + k * kFpWarps) / ngpv : -1;
+        if (kSingle && k > 0) return -1;
+        if (kSiddon || kSingle) return warp + k * kFpWarps < vcount * ngpv ? (warp + k * kFpWarps) / ngpv : -1;
         const int pair = warp + (k >> 1) * kFpWarps, v = pair / npv;
         return v < vcount && 2 * (pair - v * npv) + (k & 1) < ngpv ? v : -1;
     };
     auto slot_ray = [&](int k) {
-        if (kSiddon) return (warp + k * kFpWarps) % ngpv * kFpGroupRays + lane;
+        if (kSiddon || kSingle) return (warp + k * kFpWarps) % ngpv * kFpGroupRays + lane;
         return (2 * ((warp + (k >> 1) * kFpWarps) % npv) + (k & 1)) * kFpGroupRays + lane;
     };
     // per group: line range (lb << 16 | le) and this lane's edge-table slot
@@ -558,7 +563,7 @@ __global__ void __launch_bounds__(FpCfg<kSiddon>::threads, 1) fan_fp_kernel(FpPa
         for (int k = 0; k < kFpGroups; k += 2) {
             const int J0a = max((urng[k] >> 16) - l0, 0), J1a = min((urng[k] & 0xffff) - l0, rc);
             const int J0b = max((urng[k + 1] >> 16) - l0, 0), J1b = min((urng[k + 1] & 0xffff) - l0, rc);
-            if (J0a < J1a && J0b < J1b) {   // warp-uniform
+            if (!kSingle && J0a < J1a && J0b < J1b) {   // warp-uniform
                 int Xia, Xib;
                 float Xfa, Xfb, ra, rb;
                 const float* ga;   // the view's line factors, the same for both groups
@@ -601,7 +606,7 @@ __global__ void __launch_bounds__(FpCfg<kSiddon>::threads, 1) fan_fp_kernel(FpPa
                 acc[k + 1] = ab;
             } else if (J0a < J1a) {
                 single(k, J0a, J1a);
-            } else if (J0b < J1b) {
+            } else if (!kSingle && J0b < J1b) {
                 single(k + 1, J0b, J1b);
             }
         }
@@ -1345,6 +1350,9 @@ int fan_fp_views(int nu) {
     return std::min(kFpViews, slots / ngpv);
 }
 
+// Whether each group of a DD work item of vt views has a warp of its own.
+static bool fp_single(int nu, int vt) { return vt * ((nu + kFpGroupRays - 1) / kFpGroupRays) <= FpCfg<false>::warps; }
+
 // DD lines are packed (P, a) float2 entries; Siddon lines add a value array
 static size_t fp_smem_bytes(int nu, int sp, int R, bool siddon) {
     size_t off = kFpHeader + sizeof(float4) * (size_t)fan_fp_views(nu) * (nu + 1);
@@ -1379,6 +1387,7 @@ int fan_kernel_attributes() {
     if ((int)g_attr_done.size() <= dev) g_attr_done.resize(dev + 1, 0);
     if (g_attr_done[dev]) return RN_OK;
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_fp_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
+    RN_CUDA_TRY(cudaFuncSetAttribute(fan_fp_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_fp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
     RN_CUDA_TRY(cudaFuncSetAttribute(fan_bp_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget));
@@ -1591,6 +1600,7 @@ int fan_project(rn_fan_plan* p, float* d_prj, const float* d_img, cudaStream_t s
             fp.spin = p->spin_limit;
             LaunchScope ls1(p, st, 1);
             if (siddon) fan_fp_kernel<true><<<wend - wbeg, FpCfg<true>::threads, smem, st>>>(fp);
+            else if (fp_single(d.nu, p->fp_vt_used)) fan_fp_kernel<false, true><<<wend - wbeg, FpCfg<false>::threads, smem, st>>>(fp);
             else fan_fp_kernel<false><<<wend - wbeg, FpCfg<false>::threads, smem, st>>>(fp);
             RN_CUDA_TRY(cudaGetLastError());
         }
@@ -1969,7 +1979,8 @@ extern "C" int rn_fan_project_noalloc(float* d_prj, const float* d_img, const fl
     fp.R = R;
     fp.vt = VT;
     fp.spin = kSpinLimit;
-    fan_fp_kernel<false><<<nwork, FpCfg<false>::threads, smem, st>>>(fp);
+    if (fp_single(d.nu, VT)) fan_fp_kernel<false, true><<<nwork, FpCfg<false>::threads, smem, st>>>(fp);
+    else fan_fp_kernel<false><<<nwork, FpCfg<false>::threads, smem, st>>>(fp);
     RN_CUDA_TRY(cudaGetLastError());
     int herr = 0;
     RN_CUDA_TRY(cudaMemcpyAsync(&herr, base + o_err, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -60,3 +60,22 @@ def test_matched_pair_matches_oracle(name, rng):
     assert torch.allclose(acc, aty + 0.5, rtol=1e-6, atol=1e-6)
     plan.set_tuning(bp_parts=1)
     assert rel_l2(plan.backproject(yd, 2).cpu().numpy(), aty.cpu().numpy()) <= 1e-6
+
+
+@pytest.mark.parametrize("nu,fp_views", [(217, 4), (248, 4), (249, 3), (249, 2), (744, 1), (745, 1), (775, 2)])
+def test_pairs_and_single_ray_groups(nu, fp_views, rng):
+    """Work items with more groups of rays than warps go in pairs (odd and even numbers of groups, a last group of one
+    ray), others one group per warp; on either side of that line."""
+    import torch
+    from oracle import oracle as O
+    from reconnet_b200.torch_ops import FanPlan
+    g = small_fan(nu=nu, da=0.16 / nu)
+    ang = (np.arange(11) * ALL / 11 + 0.05).astype(np.float32)
+    plan = FanPlan(to_geometry(g), ang, nbatches=2)
+    x = rng.random(plan.img_shape).astype(np.float32)
+    ref = O.fan_fp(x, ang, g, g.nu, g.nv)
+    xd = torch.from_numpy(x).cuda()
+    assert rel_l2(plan.project(xd).cpu().numpy(), ref) <= TOL
+    plan.set_tuning(fp_views=fp_views)
+    assert rel_l2(plan.project(xd).cpu().numpy(), ref) <= TOL
+    plan.check()
