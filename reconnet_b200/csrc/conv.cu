@@ -362,7 +362,8 @@ __global__ void __launch_bounds__(kConvWsThreads) conv3x3_kernel(const __grid_co
             }
             if (w < a.W && a.mode == 1)
                 res = reinterpret_cast<const float*>(a.aux)[((long long)n * a.H + h) * a.W + w];
-            if (!mbar_wait(&bar_accf[acc], (uint32_t)((j >> 1) & 1))) {
+            // (agreed on by the warp: the TMEM load below takes all of it)
+            if (!__all_sync(0xffffffffu, mbar_wait(&bar_accf[acc], (uint32_t)((j >> 1) & 1)))) {
                 s_fail = 1;
                 break;
             }
