@@ -735,7 +735,9 @@ __global__ void __launch_bounds__(256) fan_table_kernel(const float* __restrict_
         }
         const float4 q = *reinterpret_cast<const float4*>(w + u0 + 4 * lane);
         const double p1 = (double)q.x, p2 = p1 + (double)q.y, p3 = p2 + (double)q.z, p4 = p3 + (double)q.w;
-        const double incl = warp_incl_scan(p4), pre = carry + (incl - p4);
+        const double incl = warp_incl_scan(p4);
+        // (from the lanes before alone: a value that is not finite reaches no channel before it)
+        const double before = __shfl_up_sync(0xffffffffu, incl, 1), pre = lane ? carry + before : carry;
         reinterpret_cast<double2*>(sp)[2 * lane] = make_double2(pre, pre + p1);
         reinterpret_cast<double2*>(sp)[2 * lane + 1] = make_double2(pre + p2, pre + p3);
         __syncwarp();
