@@ -887,10 +887,10 @@ struct TvTerms {
 
 // 1 / sqrt(a) to about one rounding: the hardware's estimate and a Newton step
 // (a correctly rounded root and reciprocal take four times the instructions
-// and are two roundings).
+// and are two roundings).  0 for infinity, where the step would be inf x 0.
 __device__ __forceinline__ float inv_sqrt(float a) {
     const float r = rsqrtf(a);
-    return fmaf(0.5f * r, fmaf(-a * r, r, 1.0f), r);
+    return r > 0.0f ? fmaf(0.5f * r, fmaf(-a * r, r, 1.0f), r) : r;
 }
 template <bool kVar>
 __device__ __forceinline__ TvTerms tv_terms(const float* __restrict__ img, int ix, int iy, int nx, int ny,
