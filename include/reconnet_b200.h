@@ -306,7 +306,7 @@ typedef struct rn_cone_plan rn_cone_plan;
  * at most 16 B per ray or 4 B per voxel (with y rounded up to 4), by the geometry.
  * The geometry arrays are host pointers.  Calls on several streams or threads at a
  * time have a scratch each (up to four, then they wait for one another); calls
- * captured in a graph have one of that graph's own, and capture as kernel nodes only.
+ * captured in a graph have one of that graph's own, and add no allocation nodes.
  * The plan has to outlive its graphs' launches. */
 int rn_cone_plan_create(rn_cone_plan** plan, const RnConeGeom* g, const float* detCenter, const float* detU,
                         const float* detV, const float* src, void* stream);

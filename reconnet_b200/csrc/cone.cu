@@ -803,8 +803,8 @@ struct RelaxedCapture {
 // and threads never share one at a time: they have a buffer each, up to kBuffers, then
 // they queue.  A call under stream capture takes a buffer that belongs to the graph
 // (one per capture and stream, whose calls are ordered) until the graph and
-// everything instantiated from it are gone; so captured calls add kernel nodes
-// only, and the graph can be cloned, or be a child of another.
+// everything instantiated from it are gone; so captured calls add no
+// allocation nodes, and the graph can be cloned, or be a child of another.
 class ConeScratch {
 public:
     struct Buffer {
@@ -1352,10 +1352,10 @@ int rn_cone_backproject(rn_cone_plan* p, float* d_img, const float* d_prj, int a
         if (!h.ptr) return set_cuda_error(cudaErrorMemoryAllocation, "cone backprojection: scratch");
         int s = RN_OK;
         if (p->own_bp && p->col) {
-            p->launches += 2LL * slices;
+            p->launches += 3LL * slices;
             s = cone_col_backproject(p->d_col, cd, p->col_one, static_cast<double*>(h.ptr), d_img, d_prj, accumulate, st);
         } else if (p->own_bp) {
-            p->launches += 2LL * slices;
+            p->launches += 3LL * slices;
             s = cone_tile_backproject(p->d_tile, cd, p->tp, static_cast<float*>(h.ptr), d_img, d_prj, accumulate, st);
         } else {
             s = cone_sep_backproject(p, static_cast<float*>(h.ptr), d_img, d_prj, accumulate, st);

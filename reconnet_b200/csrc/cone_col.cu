@@ -181,8 +181,10 @@ __global__ void __launch_bounds__(32 * kColWarps) cone_fp_col_kernel(float* __re
 
 // C(k), k = 0 .. nv, of every (view, iu) for one (b, c): FP64 prefix sums over
 // the rays in the order of increasing height of the sinogram value times the
-// ray's length (mm) per slab of the view's main axis.  One warp per (view, iu).
-__global__ void __launch_bounds__(256) cone_col_table_kernel(double* __restrict__ tab, const float* __restrict__ prj,
+// ray's length (mm) per slab of the view's main axis; *bad set where they are not
+// finite.  One warp per (view, iu).
+__global__ void __launch_bounds__(256) cone_col_table_kernel(double* __restrict__ tab, int* __restrict__ bad,
+                                                             const float* __restrict__ prj,
                                                              const ColView* __restrict__ views, ConeDims cd, int bt,
                                                              int c) {
     const int lane = threadIdx.x & 31;
@@ -211,6 +213,7 @@ __global__ void __launch_bounds__(256) cone_col_table_kernel(double* __restrict_
         if (k < cd.nv) t[k + 1] = incl;
         carry = __shfl_sync(0xffffffffu, incl, 31);
     }
+    if (lane == 0 && !isfinite(carry)) atomicOr(bad, 1);   // (one value of a sum is enough)
 }
 
 constexpr int kColFrac = 28;   // fractional bits of kappa
@@ -258,15 +261,89 @@ __device__ __forceinline__ void col_below(double& sum, float& part, const longlo
     }
 }
 
+// One voxel by itself, from the projections: what the prefix sums cannot give where a
+// value among them is not finite, since C(k) is then lost for every face above that
+// ray.  Only the rays that meet the voxel count, each by its length in it.
+__device__ double col_direct(const float* __restrict__ prj, const ColView* __restrict__ views,
+                                          const ConeDims& cd, int x, int y, int z) {
+    double acc = 0.0;
+    for (int view = 0; view < cd.nview; view++) {
+        const ColView& V = views[view];
+        const int m = V.m;
+        const double M = (m ? y : x) - V.S[m], A = V.S[1 - m] - (m ? x : y);
+        double lo = 1e300, hi = -1e300;
+        for (int k = 0; k < 4; k++) {   // as cone_bp_col_kernel finds the columns
+            const double wm = M + (k & 1), wa = (k >> 1) - A;
+            const double q = (V.D[1 - m] * wm - V.D[m] * wa) / (V.E[m] * wa - V.E[1 - m] * wm);
+            lo = fmin(lo, q);
+            hi = fmax(hi, q);
+        }
+        const int u0 = max(0, (int)ceil(fmax(lo - 2e-3, -1.0))), u1 = min(cd.nu - 1, (int)floor(fmin(hi + 2e-3, (double)cd.nu)));
+        for (int iu = u0; iu <= u1; iu++) {
+            const double Dm = fma((double)iu, V.E[m], V.D[m]), ra = fma((double)iu, V.E[1 - m], V.D[1 - m]) / Dm;
+            const double xa = fma(ra, M, A);
+            double ta = 0.0, tb = 1.0;
+            if (fabs(ra) > 1e-12) {
+                const double p = -xa / ra, q = (1.0 - xa) / ra;
+                ta = fmax(0.0, fmin(p, q));
+                tb = fmin(1.0, fmax(p, q));
+            } else {
+                const double xf = rint(xa * 4294967296.0);
+                if (!(xf >= 0.0 && xf < 4294967296.0)) tb = -1.0;
+            }
+            if (!(tb - ta > 1e-12)) continue;
+            // rays between the lowest and highest that reach the voxel over the pixel
+            const double ga = Dm / ((M + ta) * V.ez), gb = Dm / ((M + tb) * V.ez), q0 = z - V.Sz, q1 = q0 + 1.0, c = V.dz0 / V.ez;
+            const double vlo = fmin(fmin(q0 * ga, q1 * ga), fmin(q0 * gb, q1 * gb)) - c;
+            const double vhi = fmax(fmax(q0 * ga, q1 * ga), fmax(q0 * gb, q1 * gb)) - c;
+            const int v0 = max(0, (int)ceil(fmax(vlo - 1e-6, -1.0))), v1 = min(cd.nv - 1, (int)floor(fmin(vhi + 1e-6, (double)cd.nv)));
+            const double dm = m ? cd.d[1] : cd.d[0], da = m ? cd.d[0] : cd.d[1], dz = cd.d[2];
+            for (int iv = v0; iv <= v1; iv++) {
+                const double rise = fma((double)iv, V.ez, V.dz0) / Dm, h = fma(rise, M, -q0);   // height over the voxel's face at t = 0
+                double t0 = ta, t1 = tb;
+                if (fabs(rise) > 1e-12) {
+                    const double p = -h / rise, q = (1.0 - h) / rise;
+                    t0 = fmax(t0, fmin(p, q));
+                    t1 = fmin(t1, fmax(p, q));
+                } else {
+                    const double hf = rint(h * 4294967296.0);
+                    if (!(hf >= 0.0 && hf < 4294967296.0)) continue;
+                }
+                if (t1 - t0 > 1e-9)
+                    acc += (double)__ldg(prj + (((long long)iu * cd.nview + view) * cd.nv + iv) * cd.nc) * (t1 - t0) *
+                           sqrt(dm * dm + ra * ra * da * da + rise * rise * dz * dz);
+            }
+        }
+    }
+    return acc;
+}
+
+// The slice whose projections hold a value that is not finite (*bad), a voxel per
+// thread; cone_bp_col_kernel leaves it alone.
+__global__ void __launch_bounds__(256) cone_bp_col_direct_kernel(float* __restrict__ img, const float* __restrict__ prj,
+                                                                 const int* __restrict__ bad,
+                                                                 const ColView* __restrict__ views, ConeDims cd, int bt,
+                                                                 int c, int accumulate) {
+    if (*bad == 0) return;
+    const long long n = (long long)cd.n[0] * cd.n[1] * cd.n[2];
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+        const int z = (int)(i % cd.n[2]), y = (int)(i / cd.n[2] % cd.n[1]), x = (int)(i / cd.n[2] / cd.n[1]);
+        const float v = (float)col_direct(prj + bt * cd.prj_b + c, views, cd, x, y, z);
+        float* o = img + bt * cd.img_b + (long long)x * cd.st[0] + (long long)y * cd.st[1] + (long long)z * cd.nc + c;
+        *o = accumulate ? *o + v : v;
+    }
+}
+
 template <int R, bool kOne>
 __global__ void __launch_bounds__(32 * kColWarps, 3) cone_bp_col_kernel(float* __restrict__ img, const double* __restrict__ tab,
+                                                                      const int* __restrict__ bad,
                                                                       const ColView* __restrict__ views, ConeDims cd,
                                                                       int bt, int c, int accumulate) {
     __shared__ ColTask s_task[kColWarps][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // 4 x 2 neighbouring pixels per block: they read neighbouring rows of the table
     const int x = blockIdx.x * 4 + (warp & 3), y = blockIdx.y * 2 + (warp >> 2);
-    if (x >= cd.n[0] || y >= cd.n[1]) return;   // the whole warp
+    if (x >= cd.n[0] || y >= cd.n[1] || *bad) return;   // the whole warp
     const int nz = cd.n[2], z0 = blockIdx.z * 32 * R;
     const int top = min(nz - z0, 32 * R);   // the chunk's upper face, evaluated by the lanes' own views
     double acc[R], acct = 0.0;
@@ -467,29 +544,33 @@ int cone_col_project(const ColView* d_views, const ConeDims& cd, float* d_prj, c
     return RN_OK;
 }
 
-size_t cone_col_table_bytes(const ConeDims& cd) { return sizeof(double) * (size_t)cd.nview * cd.nu * (cd.nv + 1); }
+static size_t col_table_entries(const ConeDims& cd) { return (size_t)cd.nview * cd.nu * (cd.nv + 1); }
+size_t cone_col_table_bytes(const ConeDims& cd) { return sizeof(double) * (col_table_entries(cd) + 1); }   // and the flag
 
 template <int R>
 static void launch_bp_col(const dim3& grid, const ColView* d_views, const ConeDims& cd, bool one, const double* d_tab,
-                          float* d_img, int accumulate, int b, int c, cudaStream_t st) {
+                          const int* d_bad, float* d_img, int accumulate, int b, int c, cudaStream_t st) {
     if (one)
-        cone_bp_col_kernel<R, true><<<grid, 32 * kColWarps, 0, st>>>(d_img, d_tab, d_views, cd, b, c, accumulate);
+        cone_bp_col_kernel<R, true><<<grid, 32 * kColWarps, 0, st>>>(d_img, d_tab, d_bad, d_views, cd, b, c, accumulate);
     else
-        cone_bp_col_kernel<R, false><<<grid, 32 * kColWarps, 0, st>>>(d_img, d_tab, d_views, cd, b, c, accumulate);
+        cone_bp_col_kernel<R, false><<<grid, 32 * kColWarps, 0, st>>>(d_img, d_tab, d_bad, d_views, cd, b, c, accumulate);
 }
 
 int cone_col_backproject(const ColView* d_views, const ConeDims& cd, bool one, double* d_tab, float* d_img,
                          const float* d_prj, int accumulate, cudaStream_t st) {
     const long long rows = (long long)cd.nview * cd.nu;
+    int* d_bad = reinterpret_cast<int*>(d_tab + col_table_entries(cd));
     const int R = cd.n[2] > 64 ? 4 : cd.n[2] > 32 ? 2 : 1;
     const dim3 grid((unsigned)((cd.n[0] + 3) / 4), (unsigned)((cd.n[1] + 1) / 2),
                     (unsigned)((cd.n[2] + 32 * R - 1) / (32 * R)));
     for (int b = 0; b < cd.nb; b++)
         for (int c = 0; c < cd.nc; c++) {
-            cone_col_table_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(d_tab, d_prj, d_views, cd, b, c);
-            if (R == 4) launch_bp_col<4>(grid, d_views, cd, one, d_tab, d_img, accumulate, b, c, st);
-            else if (R == 2) launch_bp_col<2>(grid, d_views, cd, one, d_tab, d_img, accumulate, b, c, st);
-            else launch_bp_col<1>(grid, d_views, cd, one, d_tab, d_img, accumulate, b, c, st);
+            RN_CUDA_TRY(cudaMemsetAsync(d_bad, 0, sizeof(int), st));
+            cone_col_table_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(d_tab, d_bad, d_prj, d_views, cd, b, c);
+            if (R == 4) launch_bp_col<4>(grid, d_views, cd, one, d_tab, d_bad, d_img, accumulate, b, c, st);
+            else if (R == 2) launch_bp_col<2>(grid, d_views, cd, one, d_tab, d_bad, d_img, accumulate, b, c, st);
+            else launch_bp_col<1>(grid, d_views, cd, one, d_tab, d_bad, d_img, accumulate, b, c, st);
+            cone_bp_col_direct_kernel<<<148 * 8, 256, 0, st>>>(d_img, d_prj, d_bad, d_views, cd, b, c, accumulate);
         }
     RN_CUDA_TRY(cudaGetLastError());
     return RN_OK;

@@ -266,9 +266,10 @@ __global__ void __launch_bounds__(128, 3) cone_fp_tile_kernel(float* __restrict_
 // Backprojection.
 // ---------------------------------------------------------------------------
 // Projections of one (b, c) times the rays' lengths per slab, in rows of v:
-// wp[view][u][pitch] (pitch = nv rounded up to 4, the padding zero).  Block 256
-// along v; blockIdx = (v, u, view).
-__global__ void __launch_bounds__(256) cone_tile_weight_kernel(float* __restrict__ wp, const float* __restrict__ prj,
+// wp[view][u][pitch] (pitch = nv rounded up to 4, the padding zero); *bad set where
+// one is not finite.  Block 256 along v; blockIdx = (v, u, view).
+__global__ void __launch_bounds__(256) cone_tile_weight_kernel(float* __restrict__ wp, int* __restrict__ bad,
+                                                               const float* __restrict__ prj,
                                                                const TileView* __restrict__ views, ConeDims cd,
                                                                int pitch, int bt, int c) {
     const int view = blockIdx.z, iu = blockIdx.y, iv = blockIdx.x * 256 + threadIdx.x;
@@ -282,6 +283,7 @@ __global__ void __launch_bounds__(256) cone_tile_weight_kernel(float* __restrict
         val = prj[bt * cd.prj_b + (((long long)iu * cd.nview + view) * cd.nv + iv) * cd.nc + c] * seg;
     }
     wp[((long long)view * cd.nu + iu) * pitch + iv] = val;
+    if (!isfinite(val)) atomicOr(bad, 1);
 }
 
 constexpr int kBpXpw = 8, kBpTz = 4;                  // columns of voxels per warp, planes per block
@@ -290,12 +292,14 @@ constexpr int kBpTx = 4 * kBpXpw, kBpTy = 64;
 // KV: rows iv that can meet one voxel (the host's bound).
 template <int KV>
 __global__ void __launch_bounds__(128, 3) cone_bp_tile_kernel(float* __restrict__ img, const float* __restrict__ wp,
+                                                               const int* __restrict__ bad,
                                                                const TileView* __restrict__ views, ConeDims cd,
                                                                int pitch, int patch, int smem_bytes, int bt, int c,
                                                                int accumulate) {
     extern __shared__ __align__(16) float smem[];
     __shared__ float4 s_ray[4][32];   // per warp: crossing time, patch row offset, voxel | flags
     __shared__ int4 s_win[4];         // per slot: first u, first v (a multiple of 4), columns (a multiple of 4)
+    if (*bad) return;   // cone_bp_tile_direct_kernel's
     const int S = min(4, smem_bytes / (4 * patch));   // >= 2
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nx = cd.n[0], ny = cd.n[1], nz = cd.n[2];
@@ -513,6 +517,58 @@ __global__ void __launch_bounds__(128, 3) cone_bp_tile_kernel(float* __restrict_
         }
 }
 
+// The slice whose projections hold a value that is not finite, a voxel per thread.
+// The tiles add rows of rays that miss a voxel with a length of 0, which would make NaN
+// of it; here only the rays that meet a voxel count, each by its length.
+__device__ __forceinline__ bool direct_interval(double a0, double a1, double& t0, double& t1) {
+    // positions at the two faces, as the forward projection rounds them
+    a0 = rint(a0 * 4294967296.0) / 4294967296.0;
+    a1 = rint(a1 * 4294967296.0) / 4294967296.0;
+    t0 = 0.0;
+    t1 = 1.0;
+    if (a0 == a1) return a0 >= 0.0 && a0 < 1.0;
+    const double p = -a0 / (a1 - a0), q = (1.0 - a0) / (a1 - a0);
+    t0 = fmax(t0, fmin(p, q));
+    t1 = fmin(t1, fmax(p, q));
+    return t1 > t0;
+}
+
+__global__ void __launch_bounds__(256) cone_bp_tile_direct_kernel(float* __restrict__ img, const float* __restrict__ wp,
+                                                                  const int* __restrict__ bad,
+                                                                  const TileView* __restrict__ views, ConeDims cd,
+                                                                  int pitch, int bt, int c, int accumulate) {
+    if (*bad == 0) return;
+    const long long n = (long long)cd.n[0] * cd.n[1] * cd.n[2];
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+        const int z = (int)(i % cd.n[2]), y = (int)(i / cd.n[2] % cd.n[1]), x = (int)(i / cd.n[2] / cd.n[1]);
+        float acc = 0.f;
+        for (int view = 0; view < cd.nview; view++) {
+            const TileView& V = views[view];
+            // ray i lies at a + i g on the voxel's two faces (relative to it)
+            const double M0 = z - V.sm, M1 = M0 + 1.0;
+            const double au0 = fma(M0, V.ru0, V.su) - x, au1 = fma(M1, V.ru0, V.su) - x, gu0 = M0 * V.ru1, gu1 = M1 * V.ru1;
+            const double av0 = fma(M0, V.rv0, V.sv) - y, av1 = fma(M1, V.rv0, V.sv) - y, gv0 = M0 * V.rv1, gv1 = M1 * V.rv1;
+            const int i0 = max(0, (int)floor(fmin(-au0 / gu0, -au1 / gu1)) - 1);
+            const int i1 = min(cd.nu - 1, (int)ceil(fmax((1.0 - au0) / gu0, (1.0 - au1) / gu1)) + 1);
+            const int j0 = max(0, (int)floor(fmin(-av0 / gv0, -av1 / gv1)) - 1);
+            const int j1 = min(cd.nv - 1, (int)ceil(fmax((1.0 - av0) / gv0, (1.0 - av1) / gv1)) + 1);
+            for (int iu = i0; iu <= i1; iu++) {
+                double t0, t1;
+                if (!direct_interval(fma((double)iu, gu0, au0), fma((double)iu, gu1, au1), t0, t1)) continue;
+                const float* row = wp + ((long long)view * cd.nu + iu) * pitch;
+                for (int iv = j0; iv <= j1; iv++) {
+                    double s0, s1;
+                    if (!direct_interval(fma((double)iv, gv0, av0), fma((double)iv, gv1, av1), s0, s1)) continue;
+                    const double len = fmin(t1, s1) - fmax(t0, s0);
+                    if (len > 1e-9) acc = fmaf((float)len, row[iv], acc);
+                }
+            }
+        }
+        float* o = img + bt * cd.img_b + (long long)x * cd.st[0] + (long long)y * cd.st[1] + (long long)z * cd.nc + c;
+        *o = accumulate ? *o + acc : acc;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Host side.
 // ---------------------------------------------------------------------------
@@ -611,9 +667,8 @@ int cone_tile_attributes() {
 size_t cone_tile_fp_bytes(const ConeDims& cd) {
     return sizeof(float) * (size_t)cd.n[2] * cd.n[0] * ((cd.n[1] + 3) & ~3);
 }
-size_t cone_tile_bp_bytes(const ConeDims& cd) {
-    return sizeof(float) * (size_t)cd.nview * cd.nu * ((cd.nv + 3) & ~3);
-}
+static size_t tile_bp_floats(const ConeDims& cd) { return (size_t)cd.nview * cd.nu * ((cd.nv + 3) & ~3); }
+size_t cone_tile_bp_bytes(const ConeDims& cd) { return sizeof(float) * (tile_bp_floats(cd) + 1); }   // and the flag
 
 // Tiles of 64 x 128 rays for rays under a voxel apart where they fill the GPU.
 bool cone_tile_big(const ConeDims& cd, const TilePlan& tp) {
@@ -642,18 +697,21 @@ int cone_tile_project(const TileView* d_views, const ConeDims& cd, const TilePla
 int cone_tile_backproject(const TileView* d_views, const ConeDims& cd, const TilePlan& tp, float* d_wp, float* d_img,
                           const float* d_prj, int accumulate, cudaStream_t st) {
     const int pitch = (cd.nv + 3) & ~3;
+    int* d_bad = reinterpret_cast<int*>(d_wp + tile_bp_floats(cd));
     const dim3 grid((unsigned)((cd.n[2] + kBpTz - 1) / kBpTz), (unsigned)((cd.n[0] + kBpTx - 1) / kBpTx),
                     (unsigned)((cd.n[1] + kBpTy - 1) / kBpTy));
     for (int b = 0; b < cd.nb; b++)
         for (int c = 0; c < cd.nc; c++) {
-            cone_tile_weight_kernel<<<dim3((pitch + 255) / 256, cd.nu, cd.nview), 256, 0, st>>>(d_wp, d_prj, d_views, cd,
-                                                                                                pitch, b, c);
+            RN_CUDA_TRY(cudaMemsetAsync(d_bad, 0, sizeof(int), st));
+            cone_tile_weight_kernel<<<dim3((pitch + 255) / 256, cd.nu, cd.nview), 256, 0, st>>>(d_wp, d_bad, d_prj, d_views,
+                                                                                                cd, pitch, b, c);
             if (tp.kv <= 3)
-                cone_bp_tile_kernel<3><<<grid, 128, tp.bp_smem, st>>>(d_img, d_wp, d_views, cd, pitch, tp.bp_patch,
+                cone_bp_tile_kernel<3><<<grid, 128, tp.bp_smem, st>>>(d_img, d_wp, d_bad, d_views, cd, pitch, tp.bp_patch,
                                                                       tp.bp_smem, b, c, accumulate);
             else
-                cone_bp_tile_kernel<4><<<grid, 128, tp.bp_smem, st>>>(d_img, d_wp, d_views, cd, pitch, tp.bp_patch,
+                cone_bp_tile_kernel<4><<<grid, 128, tp.bp_smem, st>>>(d_img, d_wp, d_bad, d_views, cd, pitch, tp.bp_patch,
                                                                       tp.bp_smem, b, c, accumulate);
+            cone_bp_tile_direct_kernel<<<148 * 8, 256, 0, st>>>(d_img, d_wp, d_bad, d_views, cd, pitch, b, c, accumulate);
         }
     RN_CUDA_TRY(cudaGetLastError());
     return RN_OK;

@@ -71,7 +71,7 @@ def test_captured_and_concurrent_calls(kind):
 
 @pytest.mark.parametrize("kind", ["upright", "tomosynthesis", "separable"])
 def test_captured_calls_as_child_graphs(kind):
-    """Captured calls are kernel nodes only, so their graph can be a child of another one; its scratch stays its own
+    """Captured calls add no allocation nodes, so their graph can be a child of another one; its scratch stays its own
     while later captures come and go."""
     import torch
     from cuda.bindings import runtime as rt
