@@ -25,6 +25,8 @@ CASES = {
     "x_class_only": (dict(nx=40, ny=70), 9, 0.6),
     "one_view": (dict(nx=33, ny=35), 1, 0.0),
     "past_the_source": (dict(nx=64, ny=64, dx=2.0, dy=2.0, dso=220.0, dsd=400.0, da=0.012), 11, ALL),
+    # the quartic's bound at 0.0495 of 0.05 cells for the diagonal views
+    "quartic_just_inside": (dict(nx=64, ny=64, dx=1.0, dy=1.0, dso=328.0, dsd=600.0, da=0.0012, nu=230), 16, ALL),
     "wide_pixels": (dict(nx=40, ny=33, dx=3.0, dy=3.0, da=0.0012, nu=140), 10, ALL),
     # table windows of 232 entries (eight views per chunk), 472 (four), 832 (two)
     "window_232": (dict(nx=70, ny=75, dx=1.2, dy=1.2, nu=300, da=0.0009), 17, ALL),
