@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(128, 3) cone_bp_tile_kernel(float* __restrict_
                                                                int accumulate) {
     extern __shared__ __align__(16) float smem[];
     __shared__ float4 s_ray[4][32];   // per warp: crossing time, patch row offset, voxel | flags
-    __shared__ int4 s_win[4];         // per slot: first u, first v (a multiple of 4), columns (a multiple of 4)
+    __shared__ int4 s_win[4];         // per slot: first u, first v (a multiple of 4), columns (a multiple of 4), cut
     if (*bad) return;   // cone_bp_tile_direct_kernel's
     const int S = min(4, smem_bytes / (4 * patch));   // >= 2
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -325,8 +325,11 @@ __global__ void __launch_bounds__(128, 3) cone_bp_tile_kernel(float* __restrict_
         const int ub = max((int)floorf(ulo - 0.01f), 0), vb = max((int)floorf(vlo - 0.01f), 0) & ~3;
         const int cols = (max(min((int)ceilf(vhi + 0.01f), cd.nv - 1) - vb, 0) + KV + 4) & ~3;
         int rows = min((int)ceilf(uhi + 0.01f), cd.nu - 1) - ub + 1;
-        if (rows * cols > patch) rows = patch / cols;   // not reached: the host's patch bounds every window
-        if (threadIdx.x == 0) s_win[slot] = make_int4(ub, vb, cols, 0);
+        // (the host's patch holds every window, see cone_tile_views; were it ever smaller,
+        // the tile would come out NaN)
+        const bool cut = rows * cols > patch;
+        if (cut) rows = patch / cols;
+        if (threadIdx.x == 0) s_win[slot] = make_int4(ub, vb, cols, cut);
         const int j = vb + 4 * lane;
         const float* row = wp + ((long long)view * cd.nu + ub + warp) * pitch + j;
         const uint32_t dst = smem_u32(smem + slot * patch) + (warp * cols + 4 * lane) * 4;
@@ -364,6 +367,13 @@ __global__ void __launch_bounds__(128, 3) cone_bp_tile_kernel(float* __restrict_
         const TileView& V = views[view];
         const int4 win = s_win[slot];
         const int ub = win.x, vb = win.y, cols = win.z;
+        if (win.w) {
+            const float nan = __int_as_float(0x7fffffff);
+#pragma unroll
+            for (int z = 0; z < kBpTz; z++)
+#pragma unroll
+                for (int k = 0; k < kBpXpw; k++) acc[z][k] = f2_pack(nan, nan);
+        }
         const float* pbase = smem + slot * patch;
 #pragma unroll
         for (int z = 0; z < kBpTz; z++) {
@@ -635,8 +645,13 @@ bool cone_tile_views(const std::vector<ConeView>& views, const ConeDims& cd, std
     if (tp.kv > 4) return false;
     tp.kv = std::max(tp.kv, 3);
     const int kv = tp.kv;
-    // backprojection window of a tile: rays between its faces, which move by
-    // at most one voxel per slab
+    // Backprojection window of a tile.  Of the detector's rays those between the
+    // lowest and the highest that meet it count; two of them that cross its faces at
+    // m0 and m1, x0 and x1 apart, lie (x1 - x0 - r (m1 - m0)) / g1 apart, r <= ru_hi the
+    // slope of one and g1 the spacing at m1: at most (kBpTx + kBpTz ru_hi) / lo_u.  The
+    // kernel adds 0.02 for its FP32 arithmetic and rounds outwards, which is under 3.1
+    // rows more (4 and a row here), along v to a multiple of 4 before and after, under
+    // 9.1 + KV (10 + kv and 3 here).
     const double rows = (kBpTx + kBpTz * ru_hi) / lo_u + 4.0, cols = (kBpTy + kBpTz * rv_hi) / lo_v + kv + 10.0;
     tp.bp_patch = ((int)rows + 1) * (((int)cols + 4) & ~3);
     if (8LL * tp.bp_patch > kBpTileSmemWide) return false;
