@@ -24,7 +24,7 @@
 //
 // Measured, 512x512x128 voxels, 736x736 cells, 25 views: forward 1.70 ms with
 // the plane-major copy (3.98 ms for cone_fp_staged_kernel, one thread per ray),
-// back 2.91 ms with the weighting (6.42 ms for cone_bp_sep_kernel, which works
+// back 3.00 ms with the weighting (6.42 ms for cone_bp_sep_kernel, which works
 // out each lane's rows once per voxel pair).  Both are bound by instruction
 // issue.
 #include <cuda_runtime.h>

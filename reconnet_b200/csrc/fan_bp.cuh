@@ -36,8 +36,13 @@ __device__ __forceinline__ float matched_t(const ViewGeo& vg, float r) {
 
 // Edge index t(r) = tA + tB atan(kappa r) as a cubic around the slope r_t at
 // the lane's middle lattice point: along one lane the lattice points differ
-// in one coordinate only, and the truncation stays below 4e-5 cells over 17
-// points (it only selects the cell; the value inside it is exact).
+// in one coordinate only.  It is off by at most 4.7 / 24 |tB| h^4 cells for slopes h
+// / kappa from the middle: 4e-5 over 17 points of a 512 x 512 image of 0.7 mm pixels
+// 595 mm from the source, but a cell and more where the image comes close to it.  The
+// Siddon and pixel-driven kernels, and the matched one for points 4 from the middle,
+// only select a cell with it and are exact inside; reference mode (fan.cu,
+// fan_group.cu) takes an interval's ends from it, where the shift cancels between the
+// two but for its change over a pixel.
 struct TCubic {
     float rt, c0, c1, c2, c3;
 };
@@ -76,9 +81,9 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
 // the edge index at its corner, a 4-lane min gives the first staged table entry
 // (edge 0 is entry `pad`; `back` entries of slack before it), and the
 // view's parameters go to slot c % 3.  kPoly 3 or 4: also whether the window holds
-// every entry that a cubic (quartic) index of the tile can select.  Kept out of line: it runs once per
-// chunk in one warp, and inlined its temporaries would raise the register
-// count of the whole accumulation loop.
+// every entry that a cubic (quartic) index of the tile can select.  Kept out of
+// line: it runs once per chunk in one warp, and inlined its temporaries would raise the
+// register count of the whole accumulation loop.
 template <int V, int kCols, int kRows, int kPoly = 0>
 __device__ __noinline__ void bp_prep(BpSharedT<V>* sh, const ViewGeo* src, int c, int nview, int X0, int Y0,
                                      int nx, int ny, int tabn, int win, int pad, int back) {

@@ -53,9 +53,9 @@ struct MtParams {
 
 // A view as a warp reads it: the quartic of the edge index t(r) = tA + tB
 // atan(kappa r) around the slope at the middle of the warp's 31 x 31 pixels
-// (ViewGeo::quartic says that it stays within 0.05 cells, usually 1e-3; it only selects the
-// cell), as pairs for
-// packed arithmetic.  Lane v works out view v of a chunk.
+// (ViewGeo::quartic says that it stays within 0.05 cells, usually 1e-3; it only
+// selects the cell), as pairs for packed arithmetic.  Lane v works out view v of a
+// chunk.
 struct alignas(16) MtView {
     f32x2 c0, c1, c2, c3, c4, nrt, npar;
     float perp;

@@ -54,11 +54,11 @@ struct ViewGeo {
     float rmin, rmax;   // slope range covered by the detector
     float sigma;        // +-1: do edge indices increase along the line?
     int xcls;           // 1 = X-class
-    int cubic;            // t_cubic is good to a quarter of a cell over every tile of the image
-    float round;          // rounds stepped coordinates (split_step)
-    int quartic;          // the same for the matched backprojection's quartic and tiles         // 64-byte records: chunks of them are bulk-copyable
+    int cubic;          // t_cubic is within a quarter of a cell over every 31 x 128-pixel tile of the image
+    float round;        // rounds stepped coordinates (split_step)
+    int quartic;        // the matched backprojection's quartic is within 0.05 cells over every tile of its
 };
-static_assert(sizeof(ViewGeo) == 64, "ViewGeo is staged by 16-byte bulk copies");
+static_assert(sizeof(ViewGeo) == 64, "records of 64 bytes: chunks of them are staged by bulk copies");
 
 // A 2D forward problem: sinogram plane at prj_off (strides su, sview)
 // projected from a mix of up to 2 image planes (z interpolation).
@@ -159,8 +159,8 @@ struct rn_fan_plan {
     long long line_slot_elems = 0;  // per FP slice: ny*lpx + nx*lpy
     long long fp_slots = 0;         // FP slices whose lines fit in the scratch
     bool matched_near = false;      // a view's quartic is not good over every tile (fan_matched.cu)
-    int table_win_t = 0;            // the same for the matched backprojection's tiles
     int table_win_m = 0;            // staged table entries per view (BP tiles of 31 x 128 pixels)
+    int table_win_t = 0;            // the same for the matched backprojection's 62 x 62
     float4* d_tab = nullptr;        // BP edge tables
     long long tab_elems = 0;
     float* d_tmp_img = nullptr;     // image-sized scratch (SQS update, autotuner)
