@@ -19,7 +19,7 @@
 // lane holds 16 or 8 rows of every slice.
 //
 // Measured: 16 slices of 512 x 512, 701 views of 888 channels, pixel driven: 5.62
-// ms with fan.cu's kernel, 2.18 ms with four slices per block, 1.80 with eight
+// ms with fan.cu's kernel, 2.18 ms with four slices per block, 1.71 with eight
 // (tables 0.11 and 0.04 ms); 12 slices of 301 x 333, 413 views of 611 channels,
 // reference mode: 0.93, 0.52 and 0.53 ms (three quads fill two blocks of two by
 // three quarters).
