@@ -819,12 +819,13 @@ public:
         Buffer* buffer = nullptr;
     };
 
-    // The size that serves every call of the plan; a buffer of it now (best effort),
-    // so that the first call need not allocate.
+    // The size that serves every call of the plan; a buffer of it now (best effort)
+    // unless there is one, so that the first call need not allocate.
     void reserve(size_t bytes) {
         std::lock_guard<std::mutex> lk(mu_);
         full_ = bytes;
-        if (bytes > 0) grow(bytes);
+        if (bytes > 0 && std::none_of(buffers_.begin(), buffers_.end(), [&](const Buffer& b) { return b.bytes >= bytes; }))
+            grow(bytes);
     }
 
     int get(size_t bytes, cudaStream_t st, Hold* out) {
@@ -837,8 +838,10 @@ public:
         for (;;) {
             Buffer* pick = nullptr;
             bool idle = false, held = false;
+            size_t fit = 0;   // (smaller ones were for other routes, or all there was room for)
             for (Buffer& b : buffers_) {
                 if (b.bytes < bytes) continue;
+                fit++;
                 held = held || b.held;
                 if (b.held) continue;
                 RelaxedCapture relaxed;
@@ -846,7 +849,7 @@ public:
                 if (idle || !pick) pick = &b;
                 if (idle) break;
             }
-            if (!idle && buffers_.size() < kBuffers && grow(bytes)) pick = &buffers_.back();
+            if (!idle && fit < kBuffers && grow(bytes)) pick = &buffers_.back();
             if (pick) {
                 RN_CUDA_TRY(cudaStreamWaitEvent(st, pick->done, 0));
                 pick->held = true;

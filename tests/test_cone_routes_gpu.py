@@ -53,6 +53,35 @@ def test_route_matches_oracle(family, name, route, rng):
     assert rel_l2(plan.backproject(yd).cpu().numpy(), ref) <= TOL
 
 
+# rays in a voxel face: the forward and back kernels of either family have to give them to the same voxel
+@pytest.mark.parametrize("routes", [("own", "own"), ("own", "general"), ("general", "own"), ("general", "general")],
+                         ids="-".join)
+@pytest.mark.parametrize("family,name", [(f, n) for f in (col, tile) for n in f.CASES if n.startswith("level") and n not in OTHER]
+                         + [(col, f"along{n}") for n in (1, 4, 8)], ids=lambda v: v if isinstance(v, str) else v.__name__)
+def test_rays_in_a_face_are_adjoint(family, name, routes, rng):
+    import torch
+    from reconnet_b200.torch_ops import ConeGeometry, ConePlan
+    if name.startswith("along"):
+        g = col._geom(nx=24, ny=20, nz=16, dy=1.0, dz=1.0, cx=0.0, cy=0.0, cz=0.0, nu=41, nv=21, off_u=0.0, off_v=0.0)
+        geo, B, C = col._orbit(int(name[5:]), start=0.0), 1, 1
+    else:
+        g, geo, B, C = _case(family, name)
+    plan = ConePlan(ConeGeometry(**g), *geo, nbatches=B, nchannels=C)
+    plan.set_route(*routes)
+    x = torch.from_numpy(rng.random(plan.img_shape).astype(np.float32)).cuda()
+    r = torch.from_numpy(rng.random(plan.prj_shape).astype(np.float32)).cuda()
+    ax = plan.project(x).double()
+    for part in ("row", "column"):
+        y = torch.zeros_like(r)   # the middle rays alone
+        if part == "row":
+            y[:, :, :, g["nv"] // 2] = r[:, :, :, g["nv"] // 2]
+        else:
+            y[:, g["nu"] // 2] = r[:, g["nu"] // 2]
+        lhs = float((ax * y.double()).sum())
+        rhs = float((x.double() * plan.backproject(y).double()).sum())
+        assert abs(lhs - rhs) <= 1e-5 * abs(lhs), part
+
+
 @pytest.mark.parametrize("name", sorted(OTHER))
 def test_route_that_is_not_there(name):
     from reconnet_b200.torch_ops import ConeGeometry, ConePlan

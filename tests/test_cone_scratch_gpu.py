@@ -26,7 +26,10 @@ def _plan(kind):
         u = np.tile(np.float32([1, 0, 0]), (n, 1))
         v = np.tile(np.float32([0, -1 if kind == "separable" else 1, 0]), (n, 1))
     g = ConeGeometry(nx=24, ny=20, nz=12, dx=1.0, dy=1.0, dz=1.0, nu=30, nv=22, du=1.2, dv=1.2)
-    return ConePlan(g, cen, u, v, src)
+    plan = ConePlan(g, cen, u, v, src)
+    if kind != "separable":
+        plan.set_route("own", "own")   # (calls as small as these would go to the general kernels)
+    return plan
 
 
 @pytest.mark.parametrize("kind", ["upright", "tomosynthesis"])
@@ -122,6 +125,38 @@ def test_captured_calls_as_child_graphs(kind):
     for parent, ex, *_ in runs:
         ok(rt.cudaGraphExecDestroy(ex))
         ok(rt.cudaGraphDestroy(parent))
+
+
+@pytest.mark.parametrize("kind", ["upright", "tomosynthesis", "separable"])
+def test_call_beside_one_that_waits(kind):
+    """A call whose plan's buffers are all in use on another stream, which is far behind."""
+    import torch
+    plan = _plan(kind)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    ys = [torch.rand(plan.prj_shape, device="cuda", generator=gen) for _ in range(6)]
+    want = [plan.backproject(y).clone() for y in ys]
+    got = [torch.empty_like(w) for w in want]
+    torch.cuda.synchronize()
+    for y, o in zip(ys, got):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            torch.cuda._sleep(20_000_000)   # some 10 ms
+            plan.backproject(y, out=o)
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, w) for o, w in zip(got, want))
+
+
+def test_routes_back_and_forth_keep_the_scratch():
+    """Choosing routes again and again allocates no more than choosing each once."""
+    import torch
+    plan = _plan("tomosynthesis")
+    ways = [("general", "general"), ("own", "own"), ("auto", "auto"), ("own", "general")]
+    for way in ways:
+        plan.set_route(*way)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    for _ in range(5000):
+        plan.set_route(*ways[_ % 4])
+    assert free - torch.cuda.mem_get_info()[0] <= 4 << 20
 
 
 @pytest.mark.parametrize("kind", ["upright", "tomosynthesis", "separable"])
