@@ -828,7 +828,40 @@ public:
             grow(bytes);
     }
 
+    // (no exception leaves it: the plan's C functions call it)
     int get(size_t bytes, cudaStream_t st, Hold* out) {
+        try {
+            return take(bytes, st, out);
+        } catch (const std::exception&) {
+            return set_error(RN_ERR_ALLOC, "cone scratch: out of host memory");
+        }
+    }
+
+    // the launches that use the buffer are on `st`
+    int put(const Hold& h, cudaStream_t st) {
+        if (!h.buffer) return RN_OK;
+        const cudaError_t e = cudaEventRecord(h.buffer->done, st);
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            h.buffer->held = false;
+        }
+        cv_.notify_one();
+        RN_CUDA_TRY(e);
+        return RN_OK;
+    }
+
+    ~ConeScratch() {
+        for (Buffer& b : buffers_) {
+            cudaFree(b.ptr);
+            cudaEventDestroy(b.done);
+        }
+        for (Captured& c : captured_) cudaFree(c.ptr);
+    }
+
+private:
+    static constexpr size_t kBuffers = 4;
+
+    int take(size_t bytes, cudaStream_t st, Hold* out) {
         cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
         unsigned long long id = 0;
         cudaGraph_t graph = nullptr;
@@ -863,29 +896,6 @@ public:
         }
     }
 
-    // the launches that use the buffer are on `st`
-    int put(const Hold& h, cudaStream_t st) {
-        if (!h.buffer) return RN_OK;
-        const cudaError_t e = cudaEventRecord(h.buffer->done, st);
-        {
-            std::lock_guard<std::mutex> lk(mu_);
-            h.buffer->held = false;
-        }
-        cv_.notify_one();
-        RN_CUDA_TRY(e);
-        return RN_OK;
-    }
-
-    ~ConeScratch() {
-        for (Buffer& b : buffers_) {
-            cudaFree(b.ptr);
-            cudaEventDestroy(b.done);
-        }
-        for (Captured& c : captured_) cudaFree(c.ptr);
-    }
-
-private:
-    static constexpr size_t kBuffers = 4;
     struct Captured {
         void* ptr;
         size_t bytes;
@@ -931,11 +941,13 @@ private:
             }
         }
         if (!free) {
+            auto live = std::make_shared<std::atomic<bool>>(false);
+            captured_.reserve(captured_.size() + 1);
             size_t size = std::max(bytes, full_);
             void* ptr = allocate(size);
             if (!ptr && bytes < size) ptr = allocate(size = bytes);
             if (!ptr) return RN_OK;
-            captured_.push_back(Captured{ptr, size, 0, nullptr, std::make_shared<std::atomic<bool>>(false)});
+            captured_.push_back(Captured{ptr, size, 0, nullptr, std::move(live)});
             free = &captured_.back();
         }
         auto* token = new std::shared_ptr<std::atomic<bool>>(free->live);
