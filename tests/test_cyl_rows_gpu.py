@@ -42,3 +42,20 @@ def test_cyl_row_groups_match_oracle(name, rng):
     aty = plan.backproject(torch.from_numpy(y).cuda()).cpu().numpy()
     assert rel_l2(ax, O.cyl_fp(x, ang, g)) <= TOL
     assert rel_l2(aty, O.cyl_bp(y, ang, g, (g.nx, g.ny, g.nz))) <= TOL
+
+
+def test_even_volume_sums_in_groups():
+    """Equal terms on every plane: a group's 32 sums, each rounded by up to half a unit of a sum that grows evenly, come
+    to 32 / 2 * 2^-25 of the result where all round the same way (4.8e-7; the 6 groups, tables and lengths add less).
+    One chain over the 190 planes may be 2.8e-6 off."""
+    import torch
+    from oracle import oracle as O
+    from reconnet_b200.torch_ops import CylGeometry, CylPlan
+    g = CylGeometry(nx=190, ny=180, nz=40, dx=1.4, dy=1.4, dz=0.8, nu=260, nv=16, da=0.0021, dv=1.0, dsd=1085.6, dso=595.0)
+    ang = (0.05 + np.arange(16) * 2 * np.pi / 16).astype(np.float32)
+    plan = CylPlan(g, ang)
+    err = []
+    for value in (0.0213, 0.0271, 0.0339):
+        x = np.full(plan.vol_shape, value, np.float32)
+        err.append(rel_l2(plan.project(torch.from_numpy(x).cuda()).cpu().numpy(), O.cyl_fp(x, ang, g)))
+    assert max(err) <= 5e-7, err
